@@ -284,7 +284,7 @@ swr_status swr_framebuffer_create(uint32_t width, uint32_t height, uint32_t num_
     fb->num_layers = num_layers;
     cudaError_t e = cudaMalloc(&fb->layers, ((size_t)fb->layer_stride * num_layers + 64) * 4);
     if (e == cudaSuccess) e = cudaMalloc(&fb->keys, (size_t)fb->layer_stride * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&fb->tileMin, (size_t)fb->layer_stride / 16 * 4);
+    if (e == cudaSuccess) e = cudaMalloc(&fb->tileMin, ((size_t)fb->layer_stride / 16 + tile_blocks(width, height)) * 4);
     if (e == cudaSuccess) e = cudaMemsetAsync(fb->layers, 0, ((size_t)fb->layer_stride * num_layers + 64) * 4, t_stream);
     if (e != cudaSuccess) {
         swr_framebuffer_destroy(fb);
@@ -323,7 +323,7 @@ swr_status swr_framebuffer_clear(swr_framebuffer fb, uint32_t color, float depth
     fb->layers_stale = kStaleNone;  // every layer word is overwritten
     uint32_t d;
     memcpy(&d, &depth, 4);
-    launch_clear(fb->layers, fb->layers + fb->layer_stride, fb->keys, fb->tileMin, fb->width * fb->height, color, d,
+    launch_clear(fb->layers, fb->layers + fb->layer_stride, fb->keys, fb->tileMin, fb->width, fb->height, color, d,
                  t_stream);
     SWR_CHECK_LAUNCH("swr_framebuffer_clear");
     fb->keys_valid = true;
@@ -529,7 +529,7 @@ swr_status draw_impl(swr_rasterizer r, swr_framebuffer fb, uint32_t count, const
     if (overdraw && !fb->counts) SWR_CUDA(cudaMalloc(&fb->counts, (size_t)fb->layer_stride * 8));
     if ((overdraw || kind == DrawKind::Hooked) && (st = swr_internal_finalize(fb)) != SWR_OK) return st;
     if (!fb->keys_valid || kind == DrawKind::Hooked) {
-        launch_init_keys(fb->layers + fb->layer_stride, fb->keys, fb->tileMin, fb->width * fb->height, t_stream);
+        launch_init_keys(fb->layers + fb->layer_stride, fb->keys, fb->tileMin, fb->width, fb->height, t_stream);
         SWR_CHECK_LAUNCH("draw: init keys");
         fb->keys_valid = true;
     }

@@ -26,6 +26,7 @@ struct BatchView {              // device table for the batched clear and cull k
     unsigned long long* keys;
     uint32_t* groupMasks;       // one word per 32 draw positions (ViewParams::groupMasks)
     uint32_t pixels;            // width * height
+    uint32_t blocks;            // tile_blocks
     uint32_t* tileMin;          // per 4x4 tile depth bound
     uint32_t frustum, cone;     // tests of the batched cull: frustum planes, backface cone
     float eye[3];               // camera centre in object space (cone_camera)
@@ -37,6 +38,8 @@ __global__ void k_clear_views(const BatchView* __restrict__ views, uint32_t colo
     const BatchView& v = views[blockIdx.y];
     const uint32_t hi = float_order(__uint_as_float(depthBits));
     const unsigned long long key = ((unsigned long long)hi << 32) | kKeyEmptyLow;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < v.blocks; i += gridDim.x * blockDim.x)
+        v.tileMin[(v.pixels >> 4) + i] = hi;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < v.pixels; i += gridDim.x * blockDim.x) {
         v.layer0[i] = color;
         v.layer1[i] = depthBits;
@@ -151,6 +154,7 @@ swr_status upload_views(swr_batch b, const swr_view_desc* views) {
         w.tileMin = fb->tileMin;
         w.groupMasks = b->dGroupMasks + (size_t)i * words;
         w.pixels = fb->width * fb->height;
+        w.blocks = tile_blocks(fb->width, fb->height);
         w.frustum = (b->cullFlags & SWR_CULL_FRUSTUM) ? 1u : 0u;
         w.cone = ((b->cullFlags & SWR_CULL_BACKFACE_CONE) && swr_hostmath::cone_camera(objToClip, w.eye)) ? 1u : 0u;
         b->depthOnly[i] = d.depth_only != 0;

@@ -127,7 +127,8 @@ struct ViewParams {
     unsigned long long* keys;
     const uint32_t* groupMasks;  // batched views: bit l of word g is the cull result of draw position
                                  // 32 g + l (nullptr: every meshlet visible)
-    uint32_t* tileMin;      // per 4x4 tile: lower bound of its keys' depth words (nullptr: no tile culling)
+    uint32_t* tileMin;      // per 4x4 tile: lower bound of its keys' depth words (nullptr: no tile culling); then
+                            // the blocks' bounds (tile_blocks)
     uint32_t orderStride;   // draw order: position p draws meshlet (p * orderStride) mod count (order_stride)
     uint32_t pad;
 };
@@ -193,9 +194,15 @@ __device__ __forceinline__ uint32_t draw_order(uint32_t p, uint32_t count, uint3
 }
 
 void launch_draw(const DrawArgs& a, cudaStream_t st, int numSMs);
-void launch_init_keys(const uint32_t* depthLayer, unsigned long long* keys, uint32_t* tileMin, uint32_t n, cudaStream_t st);
-void launch_clear(uint32_t* layer0, uint32_t* layer1, unsigned long long* keys, uint32_t* tileMin, uint32_t n,
-                  uint32_t color, uint32_t depthBits, cudaStream_t st);
+// The 32x32-pixel blocks of a framebuffer. Tile depth bounds (tileMin) are followed by one word per
+// block, a lower bound of the block's tile bounds (the chunk stage's coarse test).
+inline __host__ __device__ uint32_t tile_blocks(uint32_t width, uint32_t height) {
+    return ((width + 31) / 32) * ((height + 31) / 32);
+}
+void launch_init_keys(const uint32_t* depthLayer, unsigned long long* keys, uint32_t* tileMin, uint32_t width, uint32_t height,
+                      cudaStream_t st);
+void launch_clear(uint32_t* layer0, uint32_t* layer1, unsigned long long* keys, uint32_t* tileMin, uint32_t width,
+                  uint32_t height, uint32_t color, uint32_t depthBits, cudaStream_t st);
 void launch_fill(uint32_t* dst, uint32_t n, uint32_t value, cudaStream_t st);
 void launch_finalize(const unsigned long long* keys, uint32_t* layer0, uint32_t* layer1, uint32_t n, cudaStream_t st);
 void launch_finalize_overdraw(const unsigned long long* keys, const unsigned long long* counts, uint32_t* layer0,
@@ -233,7 +240,7 @@ struct swr_framebuffer_t {
     uint32_t width, height, tile_stride, layer_stride, num_layers;
     uint32_t* layers;              // num_layers * layer_stride words (+64 pad)
     unsigned long long* keys;      // one vis-buffer key per pixel, tiled like the layers
-    uint32_t* tileMin;             // per 4x4 tile: lower bound of its keys' depth words
+    uint32_t* tileMin;             // per 4x4 tile: lower bound of its keys' depth words, then tile_blocks block bounds
     unsigned long long* counts;    // OverdrawShader counters, allocated by its first draw
     bool keys_valid;               // keys and tileMin reflect the depth layer
     uint8_t layers_stale;          // the keys hold draws not yet written to the layers: kStale*

@@ -143,7 +143,7 @@ extern "C" swr_status swr_draw_meshlets_noalloc(const void* meshlets, uint32_t m
         LaunchScope ls("k_expand_material_flags", stream);
         k_expand_material_flags<<<(num_materials + 255) / 256, 256, 0, stream>>>(material_flags, num_materials, mats);
     }
-    launch_init_keys((const uint32_t*)depth, keys, nullptr, n, stream);
+    launch_init_keys((const uint32_t*)depth, keys, nullptr, width, height, stream);
 
     DrawArgs a = {};
     a.meshlets = (const uint8_t*)meshlets;
