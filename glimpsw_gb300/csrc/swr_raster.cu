@@ -188,9 +188,12 @@ __device__ __forceinline__ TileTest tile_test(const TriRec& r) {
 }
 
 // Raises the tile's depth bound to the minimum of the values its 16 pixels reported (the two
-// halves of the warp shade one tile each: two whole-warp reductions, each over one half's values).
+// halves of the warp shade one tile each). A bound rises only if every pixel's value is above it, which a
+// ballot tells for both halves; the two whole-warp reductions, each over one half's values, run only then.
 __device__ __forceinline__ void update_tile_min(uint32_t obs, uint32_t* tileMin, uint32_t tileIdx, uint32_t known,
                                                 bool active, int lane) {
+    const unsigned above = __ballot_sync(0xFFFFFFFFu, active && obs > known);
+    if ((above & 0xFFFFu) != 0xFFFFu && (above >> 16) != 0xFFFFu) return;
     const bool upper = lane & 16;
     const uint32_t lo = __reduce_min_sync(0xFFFFFFFFu, upper ? 0xFFFFFFFFu : obs);
     const uint32_t hi = __reduce_min_sync(0xFFFFFFFFu, upper ? obs : 0xFFFFFFFFu);
@@ -482,48 +485,49 @@ __device__ __forceinline__ unsigned long long tile_pixel_key(const TriRec& r, ui
 
 // Shades the live tiles of the warp-wide candidate set (the lanes in `mask` hold a tile origin
 // tpx/tpy, its depth bound tmin and a triangle selector rsel for rec()) and raises the tiles' depth
-// bounds (each pixel reports a lower bound of its depth word afterwards). Four tiles per step: each
-// half-warp takes two, and a lane's two key loads are issued together (the walk is bound by their
-// latency).
+// bounds (each pixel reports a lower bound of its depth word afterwards). The live tiles are first packed
+// into `list` (32 entries of shared memory): a step then reads its tiles' entries instead of searching the
+// mask and shuffling every field. Four tiles per step: each half-warp takes two, and a lane's two key loads
+// are issued together (the walk is bound by instruction issue and by their latency). With the packed list
+// and update_tile_min's ballot: 1080p mesh stage of 100k meshlets 408 -> 379 us, 60k meshlets from inside
+// 265 -> 237 us. Loading the next step's keys ahead cost spills: 443 us.
 template <class Rec, class ReadKey>
 __device__ __forceinline__ void shade_live_tiles(Rec&& rec, ReadKey&& readKey, uint32_t rsel, unsigned mask, uint32_t tpx,
                                                  uint32_t tpy, uint32_t tmin, unsigned long long* keys, uint32_t* tileMin,
-                                                 uint32_t width, int lane) {
-    const uint32_t half = lane >> 4, tw = width >> 2, l = lane & 15;
-    const uint32_t txy = tpx | (tpy << 16);  // tile origins are below 2896
-    while (mask) {
-        int s[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            s[k] = mask ? __ffs(mask) - 1 : -1;
-            if (s[k] >= 0) mask &= mask - 1;
-        }
-        const int srcA = half ? s[1] : s[0], srcB = half ? s[3] : s[2];
-        const uint32_t pa_ = __shfl_sync(0xFFFFFFFFu, txy, srcA & 31), pb_ = __shfl_sync(0xFFFFFFFFu, txy, srcB & 31);
-        const uint32_t ax = pa_ & 0xFFFF, ay = pa_ >> 16, bx = pb_ & 0xFFFF, by = pb_ >> 16;
-        const uint32_t am = __shfl_sync(0xFFFFFFFFu, tmin, srcA & 31), ar = __shfl_sync(0xFFFFFFFFu, rsel, srcA & 31);
-        const uint32_t bm = __shfl_sync(0xFFFFFFFFu, tmin, srcB & 31), br = __shfl_sync(0xFFFFFFFFu, rsel, srcB & 31);
-        unsigned long long* pa = keys + (ax << 2) + ay * width + l;
-        unsigned long long* pb = keys + (bx << 2) + by * width + l;
-        // The key read filters losing atomics and gives the tile bound each pixel's new depth. For
-        // triangles whose readKey(selector) is false (above the draw's keyReadTiles tiles) it is
-        // skipped: the atomic is unconditional and a pixel's bound is max(new depth, old tile
-        // bound), still a lower bound of its final key.
-        const bool readA = srcA >= 0 && readKey(ar);
-        const bool readB = srcB >= 0 && readKey(br);
-        const unsigned long long curA = readA ? *(volatile unsigned long long*)pa : 0ull;
-        const unsigned long long curB = readB ? *(volatile unsigned long long*)pb : 0ull;
-        const unsigned long long keyA = srcA >= 0 ? tile_pixel_key(rec(ar), ax, ay, l) : 0ull;
-        const unsigned long long keyB = srcB >= 0 ? tile_pixel_key(rec(br), bx, by, l) : 0ull;
-        if (keyA > curA) atomicMax(pa, keyA);
-        if (keyB > curB) atomicMax(pb, keyB);
+                                                 uint32_t width, int lane, uint4* list) {
+    const uint32_t half = lane >> 4, l = lane & 15, m = __popc(mask);
+    if ((mask >> lane) & 1)  // key offset of the tile, its origin (below 2896), depth bound and triangle
+        list[__popc(mask & ((1u << lane) - 1u))] = make_uint4((tpx << 2) + tpy * width, tpx | (tpy << 16), tmin, rsel);
+    __syncwarp();
+    unsigned long long* k = keys + l;
+    // The key read filters losing atomics and gives the tile bound each pixel's new depth. For
+    // triangles whose readKey(selector) is false (above the draw's keyReadTiles tiles) it is
+    // skipped: the atomic is unconditional and a pixel's bound is max(new depth, old tile
+    // bound), still a lower bound of its final key.
+    auto fetch = [&](uint32_t i, uint4& e, bool& valid, bool& read, unsigned long long& cur) {
+        e = list[i & 31];
+        valid = i < m;
+        read = valid && readKey(valid ? e.w : 0u);
+        cur = read ? *(volatile unsigned long long*)(k + e.x) : 0ull;
+    };
+    auto shade = [&](const uint4& e, bool valid, bool read, unsigned long long cur) {
+        const unsigned long long key = valid ? tile_pixel_key(rec(e.w), e.y & 0xFFFF, e.y >> 16, l) : 0ull;
+        if (key > cur) atomicMax(k + e.x, key);
         if (tileMin) {
-            const uint32_t obsA = readA ? (uint32_t)((keyA > curA ? keyA : curA) >> 32) : max((uint32_t)(keyA >> 32), am);
-            const uint32_t obsB = readB ? (uint32_t)((keyB > curB ? keyB : curB) >> 32) : max((uint32_t)(keyB >> 32), bm);
-            update_tile_min(obsA, tileMin, (ay >> 2) * tw + (ax >> 2), am, srcA >= 0, lane);
-            update_tile_min(obsB, tileMin, (by >> 2) * tw + (bx >> 2), bm, srcB >= 0, lane);
+            const uint32_t obs = read ? (uint32_t)((key > cur ? key : cur) >> 32) : max((uint32_t)(key >> 32), e.z);
+            update_tile_min(obs, tileMin, e.x >> 4, e.z, valid, lane);
         }
+    };
+    for (uint32_t i = 0; i < m; i += 4) {
+        uint4 a, b;
+        bool va, vb, ra, rb;
+        unsigned long long ca, cb;
+        fetch(i + half, a, va, ra, ca);
+        fetch(i + 2 + half, b, vb, rb, cb);
+        shade(a, va, ra, ca);
+        shade(b, vb, rb, cb);
     }
+    __syncwarp();
 }
 
 // shade_live_tiles for alpha-tested triangles of one material (texture tex, cutoff << 24): a
@@ -585,12 +589,12 @@ __device__ __forceinline__ bool raster_region_with(const TriRec& r, const TileTe
 // raster_region_with for an opaque triangle, two tiles per step.
 __device__ __forceinline__ bool raster_region(const TriRec& r, const TileTest& tt, uint32_t x0, uint32_t y0, int tilesX, int tilesY,
                                               unsigned long long* keys, uint32_t* tileMin, uint32_t width, int lane, uint32_t readTiles,
-                                              uint32_t divMagic = 0) {
+                                              uint4* list, uint32_t divMagic = 0) {
     const bool readKey = readTiles == 0 || triangle_tiles(r) <= readTiles;
     return raster_region_with(r, tt, x0, y0, tilesX, tilesY, tileMin, width, lane,
                        [&](unsigned mask, uint32_t tpx, uint32_t tpy, uint32_t tmin) {
                            shade_live_tiles([&](uint32_t) -> const TriRec& { return r; }, [&](uint32_t) { return readKey; }, 0,
-                                            mask, tpx, tpy, tmin, keys, tileMin, width, lane);
+                                            mask, tpx, tpy, tmin, keys, tileMin, width, lane, list);
                        }, divMagic);
 }
 
@@ -772,6 +776,7 @@ struct WarpSmem {
     uint8_t owner[32 * kSmallTiles];
     uint8_t code[64];    // vertex_code
     uint8_t live[128];   // the meshlet's triangles that survive the face test or need clipping
+    uint4 list[32];      // the live tiles being shaded (shade_live_tiles)
     float zmax[32];      // each small triangle's depth bound (triangle_depth_bound)
 };
 struct WarpSmemAlpha : WarpSmem {
@@ -1126,7 +1131,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                 } else {
                     shade_live_tiles([&](uint32_t q) -> const TriRec& { return tris[q].v; },
                                      [&](uint32_t q) { return (tris[q].v.pad & kPadReadKey) != 0u; }, own, liveMask, tpx, tpy,
-                                     tmin, vp.keys, vp.tileMin, vp.width, lane);
+                                     tmin, vp.keys, vp.tileMin, vp.width, lane, S.list);
                 }
             }
             // Triangles the full queue turned away are rasterized here by the whole warp.
@@ -1144,7 +1149,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                 } else if constexpr (kOver) {
                     raster_region_overdraw(r, tile_test(r), x0, y0, tx, ty, vp.keys, a.counts, vp.width, lane);
                 } else {
-                    raster_region(r, tile_test(r), x0, y0, tx, ty, vp.keys, vp.tileMin, vp.width, lane, a.keyReadTiles);
+                    raster_region(r, tile_test(r), x0, y0, tx, ty, vp.keys, vp.tileMin, vp.width, lane, a.keyReadTiles, S.list);
                 }
             }
             __syncwarp();
@@ -1255,6 +1260,7 @@ __global__ void __launch_bounds__(256, 5) k_raster_big(const TriRec* __restrict_
                                                     const ViewParams* __restrict__ views, uint32_t chunk,
                                                     const DevMaterial* __restrict__ materials, unsigned long long* counts,
                                                     uint32_t readTiles) {
+    __shared__ uint4 list[8][32];  // per warp: the live tiles being shaded
     const unsigned long long q = control[1];
     if (blockIdx.x == 0 && threadIdx.x == 0)  // the next draw's second cursor, alpha list and idle-warp counts
         control[7] = control[9] = control[10] = control[11] = control[12] = 0;
@@ -1330,7 +1336,7 @@ __global__ void __launch_bounds__(256, 5) k_raster_big(const TriRec* __restrict_
                 if (r.pad & kTriAlpha)
                     any = raster_chunk_alpha(big + s, materials, x0, y0, tilesX, tilesY, vkeys, vtiles, vw, lane);
                 else
-                    any = raster_region(r, tile_test(r), x0, y0, tilesX, tilesY, vkeys, vtiles, vw, lane, readTiles, kDiv16[tilesX]);
+                    any = raster_region(r, tile_test(r), x0, y0, tilesX, tilesY, vkeys, vtiles, vw, lane, readTiles, list[threadIdx.x >> 5], kDiv16[tilesX]);
                 if (!any && vtiles) refresh_blocks(x0, y0, x1, y1, vtiles, vw, vh, lane);
             }
         }
