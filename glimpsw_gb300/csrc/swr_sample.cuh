@@ -15,19 +15,6 @@ __device__ __forceinline__ uint32_t texel_offset(int32_t x, int32_t y, int32_t s
     return (uint32_t)((y & 7) | (x << 3) | ((y & ~7) << stride));
 }
 
-// simd::lerp16 (SIMD.h:450) on both 16-bit halves: a + mulhrs(b - a, t).
-__device__ __forceinline__ uint32_t lerp16(uint32_t a, uint32_t b, uint32_t t) {
-    uint32_t r = 0;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        int32_t ah = (int16_t)(a >> (16 * h)), bh = (int16_t)(b >> (16 * h)), th = (int16_t)(t >> (16 * h));
-        int32_t d = (int16_t)(bh - ah);
-        int32_t mm = (int16_t)((d * th + 0x4000) >> 15);
-        r |= (uint32_t)(uint16_t)(ah + mm) << (16 * h);
-    }
-    return r;
-}
-
 // vcvtph2ps of one half (exact).
 __device__ __forceinline__ float h2f(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
 
@@ -38,12 +25,21 @@ __device__ __forceinline__ int32_t ilog2_x86(float x) {
     return (int32_t)(b - (127u << 23)) >> 23;
 }
 
-// Bilinear blend of four RGBA8 texels with 1.15 fixed-point weights (the 16-bit lane lerps of
-// SampleLevel<SurfaceSampler>, Texture.h:540-556).
+// simd::lerp16 (SIMD.h:450), a + mulhrs(b - a, 128 w), of the 8-bit values in both 16-bit halves with a weight
+// w of 0..255: mulhrs is ((b - a) 128 w + 2^14) >> 15 = ((b - a) w + 128) >> 8, so the blend is
+// (a (256 - w) + b w + 128) >> 8 in each half, at most 65408: two multiplies serve both (about 4
+// operations instead of 16; equal for all 2^24 (a, b, w)).
+__device__ __forceinline__ uint32_t lerp8x2(uint32_t a, uint32_t b, uint32_t w) {
+    return ((a * (256u - w) + b * w + 0x00800080u) >> 8) & 0x00FF00FFu;
+}
+
+// Bilinear blend of four RGBA8 texels (the 16-bit lane lerps of SampleLevel<SurfaceSampler>,
+// Texture.h:540-556); fx and fy hold the 1.15 fixed-point weight (a multiple of 128) in both halves.
 __device__ __forceinline__ uint32_t filter_rgba8(uint32_t d00, uint32_t d10, uint32_t d01, uint32_t d11, uint32_t fx, uint32_t fy) {
-    uint32_t rb1 = lerp16(d00 & 0x00FF00FF, d10 & 0x00FF00FF, fx), ga1 = lerp16((d00 >> 8) & 0x00FF00FF, (d10 >> 8) & 0x00FF00FF, fx);
-    uint32_t rb2 = lerp16(d01 & 0x00FF00FF, d11 & 0x00FF00FF, fx), ga2 = lerp16((d01 >> 8) & 0x00FF00FF, (d11 >> 8) & 0x00FF00FF, fx);
-    return lerp16(rb1, rb2, fy) | (lerp16(ga1, ga2, fy) << 8);
+    const uint32_t wx = (fx >> 7) & 255u, wy = (fy >> 7) & 255u, k = 0x00FF00FFu;
+    const uint32_t rb = lerp8x2(lerp8x2(d00 & k, d10 & k, wx), lerp8x2(d01 & k, d11 & k, wx), wy);
+    const uint32_t ga = lerp8x2(lerp8x2((d00 >> 8) & k, (d10 >> 8) & k, wx), lerp8x2((d01 >> 8) & k, (d11 >> 8) & k, wx), wy);
+    return rb | (ga << 8);
 }
 
 // The texel coordinates one lane's SampleLevel<SurfaceSampler> reads (Texture.h:412-459): level m,
@@ -73,13 +69,17 @@ __device__ __forceinline__ TexelQuad texel_quad(const DevTexture& t, float u, fl
     return q;
 }
 
-// SampleLevel<SurfaceSampler> for one lane once the tile's filter is known (Texture.h:412-459).
-__device__ __forceinline__ uint32_t sample_rgba8(const DevTexture& t, float u, float v, int layer, int32_t mipIn, bool nearest) {
-    const TexelQuad q = texel_quad(t, u, v, mipIn, nearest);
+// The texel of one layer at a quad (SampleLevel<SurfaceSampler>, Texture.h:412-459).
+__device__ __forceinline__ uint32_t sample_quad(const DevTexture& t, const TexelQuad& q, int layer, bool nearest) {
     const uint32_t* base = t.data + (size_t)layer * t.layer_stride + t.mip_offsets[q.m & 15];
     if (nearest) return base[texel_offset(q.tx, q.ty, q.stride)];
-    uint32_t i00 = texel_offset(q.tx, q.ty, q.stride), i01 = texel_offset(q.tx, q.ty + (q.inY ? 1 : 0), q.stride);
+    const uint32_t i00 = texel_offset(q.tx, q.ty, q.stride), i01 = texel_offset(q.tx, q.ty + (q.inY ? 1 : 0), q.stride);
     return filter_rgba8(base[i00], base[i00 + 8], base[i01], base[i01 + 8], q.fx, q.fy);
+}
+
+// SampleLevel<SurfaceSampler> for one lane once the tile's filter is known (Texture.h:412-459).
+__device__ __forceinline__ uint32_t sample_rgba8(const DevTexture& t, float u, float v, int layer, int32_t mipIn, bool nearest) {
+    return sample_quad(t, texel_quad(t, u, v, mipIn, nearest), layer, nearest);
 }
 
 }  // namespace swr

@@ -112,8 +112,10 @@ HEADER = r"""// Exact restatement of the AVX-512 instructions VRCP14PS and VRSQR
 
 #if defined(__CUDACC__)
 #define SWR_A14_FN static __host__ __device__ __forceinline__
+#define SWR_A14_SLOW static __host__ __device__ __noinline__
 #else
 #define SWR_A14_FN static inline
+#define SWR_A14_SLOW static inline
 #endif
 
 // Segments: [0, 64) rcp14 by m[22:17]; [64, 96) rsqrt14 of even exponents by m[22:18];
@@ -147,8 +149,8 @@ SWR_A14_FN uint32_t swr_a14_clz(uint32_t v) {
 
 SWR_A14_FN float swr_a14_from_bits(uint32_t u) { float f; memcpy(&f, &u, 4); return f; }
 
-// VRCP14PS on one lane.
-SWR_A14_FN float swr_rcp14(float x) {
+// VRCP14PS on one lane, any input.
+SWR_A14_SLOW float swr_rcp14_any(float x) {
     uint32_t u;
     memcpy(&u, &x, 4);
     const uint32_t sign = u & 0x80000000u, e = (u >> 23) & 0xFF;
@@ -170,8 +172,8 @@ SWR_A14_FN float swr_rcp14(float x) {
     return swr_a14_from_bits(sign | (sig >> (1 - re)));
 }
 
-// VRSQRT14PS on one lane.
-SWR_A14_FN float swr_rsqrt14(float x) {
+// VRSQRT14PS on one lane, any input.
+SWR_A14_SLOW float swr_rsqrt14_any(float x) {
     uint32_t u;
     memcpy(&u, &x, 4);
     const uint32_t sign = u & 0x80000000u, e = (u >> 23) & 0xFF;
@@ -190,6 +192,32 @@ SWR_A14_FN float swr_rsqrt14(float x) {
     if (!odd && m == 0) return swr_a14_from_bits((uint32_t)(127 - half) << 23);
     const uint32_t sig = swr_a14_significand(64 + 32 * odd + (m >> 18), (m >> 8) & 1023);
     return swr_a14_from_bits(((uint32_t)(126 - half) << 23) | (sig & 0x7FFFFFu));
+}
+
+// The instructions with the inputs in use handled inline: about 12 operations and one test, instead of
+// the branches of every special case at every use (a resolved pixel takes about 20 of them). rcp14:
+// normal inputs with a normal result (exponent fields 1 to 252); rsqrt14: positive normal inputs. Other inputs
+// go out of line. (With the packed texel filter: 1080p resolve 106 -> 97 us, G-buffer fragment stage 189 ->
+// 149 us, alpha-tested chunk stage 459 -> 424 us, IBL irradiance 1.59 -> 1.47 ms.)
+SWR_A14_FN float swr_rcp14(float x) {
+    uint32_t u;
+    memcpy(&u, &x, 4);
+    if ((u & 0x7FFFFFFFu) - 0x00800000u >= 0x7E000000u) return swr_rcp14_any(x);
+    const uint32_t m = u & 0x7FFFFFu;
+    const uint32_t sig = swr_a14_significand(m >> 17, (m >> 7) & 1023) & 0x7FFFFFu;
+    // sign and exponent 253 - e, or 254 - e with a zero mantissa for a power of two
+    const uint32_t top = (u & 0x80000000u) | (253u * 0x800000u - (u & 0x7F800000u));
+    return swr_a14_from_bits(m ? top | sig : top + 0x800000u);
+}
+SWR_A14_FN float swr_rsqrt14(float x) {
+    uint32_t u;
+    memcpy(&u, &x, 4);
+    if (u - 0x00800000u >= 0x7F000000u) return swr_rsqrt14_any(x);
+    // bits 23-18: the exponent's lowest bit (0 for the odd unbiased exponents) and the segment
+    const uint32_t sig = swr_a14_significand(64 + (((u >> 18) & 63) ^ 32), (u >> 8) & 1023) & 0x7FFFFFu;
+    const uint32_t half = (u + 0x800000u) >> 24;  // (e + 1) / 2
+    const uint32_t top = (190u - half) << 23;
+    return swr_a14_from_bits((u & 0xFFFFFFu) == 0x800000u ? top + 0x800000u : top | sig);
 }
 
 // simd::approx_sqrt (SIMD.h:296).
