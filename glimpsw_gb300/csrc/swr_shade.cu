@@ -204,6 +204,9 @@ __global__ void __launch_bounds__(1024) k_hiz_tail(uint32_t fbW, uint32_t fbH, u
 }
 
 // =========================================================================== resolve
+// Up to this many lights travel in the kernel's parameters; more are copied to a device allocation (an
+// allocation, a copy and a free per frame cost more host and stream time than a small frame's resolve).
+constexpr uint32_t kParamLights = 16;
 struct ResolveArgs {
     const uint8_t* meshlets;
     uint32_t numMeshlets;
@@ -217,8 +220,9 @@ struct ResolveArgs {
     float invProj[16];
     float viewPos[3];
     float exposure;
-    const swr_light* lights;  // device copy
+    const swr_light* lights;  // device copy (nullptr: the lights are in `light`)
     uint32_t numLights;
+    swr_light light[kParamLights];
     DevTexture sky;
     int hasSky;
     uint32_t debugLayer;    // SWR_DEBUG_* of the debug mode
@@ -314,8 +318,10 @@ __device__ __forceinline__ uint32_t debug_pixel(uint32_t layer, uint32_t data, u
            (255u << 24);
 }
 
+// Bound by instruction issue (82 % of the slots; 1080p: 1400 instructions a warp, 90 us; 1600 and 106 us
+// with the waterfalls, a load round per surface id and a sampling round per material).
 template <int kMode>
-__global__ void __launch_bounds__(256) k_resolve(ResolveArgs a, NeuralResolve nr) {
+__global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ ResolveArgs a, const __grid_constant__ NeuralResolve nr) {
     const uint32_t lane = threadIdx.x & 31, l = lane & 15, half = lane >> 4;
     const unsigned hm = 0xFFFFu << (16 * half);
     const uint32_t tilesX = a.width >> 2, numTiles = tilesX * (a.height >> 2);
@@ -394,34 +400,32 @@ __global__ void __launch_bounds__(256) k_resolve(ResolveArgs a, NeuralResolve nr
             }
         }
         if (!fast) {
-        // ---- ResolveSurface (Shading.cpp:471-579): waterfall over the tile's surface ids
+        // ---- ResolveSurface (Shading.cpp:471-579). The reference's waterfall over the tile's surface ids loads
+        // each id's record for the lanes that hold it; here every lane loads its own (a pixel without a
+        // surface takes part only if a covered pixel holds its id). A tile of small triangles had one
+        // round of dependent loads per id.
         F3 pos[3] = {};
         uint32_t tc[3] = {}, matId = 0;
         uint32_t sflags = kSurfFast, sfx = 0, sfy = 0;  // the emit pass's record of this pixel
-        unsigned pending = (~skyBits) & 0xFFFF;
-        while (pending) {
-            const int src = __ffs(pending) - 1;
-            const uint32_t sid = __shfl_sync(hm, id, src + 16 * half);
-            const unsigned iter = (__ballot_sync(hm, id == sid) >> (16 * half)) & 0xFFFF;
-            pending &= ~iter;
-            const uint32_t mId = sid / 128, tri = sid % 128;
-            if (((iter >> l) & 1) && mId < a.numMeshlets) {
-                const uint8_t* mp = a.meshlets + (size_t)mId * kMeshletSize;
-                const float* P = (const float*)(mp + kOffPositions);
-                const uint32_t* TC = (const uint32_t*)(mp + kOffTexCoords);
-                const uint32_t* NT = (const uint32_t*)(mp + kOffNormalTangents);
-                const uint8_t* I = mp + kOffIndices;
-                const unsigned long long handBits = *(const unsigned long long*)(mp + kOffHandedness);
+        const unsigned covered = ((~skyBits) & 0xFFFF) << (16 * half);
+        const bool holds = skyBits == 0 || (__match_any_sync(hm, id) & covered) != 0;
+        const uint32_t mId = id / 128, tri = id % 128;
+        if (holds && mId < a.numMeshlets) {
+            const uint8_t* mp = a.meshlets + (size_t)mId * kMeshletSize;
+            const float* P = (const float*)(mp + kOffPositions);
+            const uint32_t* TC = (const uint32_t*)(mp + kOffTexCoords);
+            const uint32_t* NT = (const uint32_t*)(mp + kOffNormalTangents);
+            const uint8_t* I = mp + kOffIndices;
+            const unsigned long long handBits = *(const unsigned long long*)(mp + kOffHandedness);
 #pragma unroll
-                for (int vi = 0; vi < 3; vi++) {
-                    const uint32_t idx = I[vi * 128 + tri] & 63;
-                    pos[vi] = { P[idx], P[64 + idx], P[128 + idx] };
-                    tc[vi] = TC[idx];
-                    ntg[vi] = NT[idx];
-                    if (vi == 0 && ((handBits >> idx) & 1)) hand = 1u << 31;
-                }
-                matId = *(const uint32_t*)(mp + kOffMaterialId);
+            for (int vi = 0; vi < 3; vi++) {
+                const uint32_t idx = I[vi * 128 + tri] & 63;
+                pos[vi] = { P[idx], P[64 + idx], P[128 + idx] };
+                tc[vi] = TC[idx];
+                ntg[vi] = NT[idx];
+                if (vi == 0 && ((handBits >> idx) & 1)) hand = 1u << 31;
             }
+            matId = *(const uint32_t*)(mp + kOffMaterialId);
         }
         // IntersectTriangle (Shading.cpp:417-464)
         float w0, w1, w2;
@@ -458,80 +462,98 @@ __global__ void __launch_bounds__(256) k_resolve(ResolveArgs a, NeuralResolve nr
         const float g0 = t10x * dx[1] + t20x * dx[2], g1 = t10y * dx[1] + t20y * dx[2];
         const float g2 = t10x * dy[1] + t20x * dy[2], g3 = t10y * dy[1] + t20y * dy[2];
 
-        // waterfall over materials: filter chosen over the whole tile per material
-        unsigned pm = (__ballot_sync(hm, !isSky && matId != 0xFFFFFFFFu) >> (16 * half)) & 0xFFFF;
-        while (pm) {
-            const int src = __ffs(pm) - 1;
-            const uint32_t mid = __shfl_sync(hm, matId, src + 16 * half);
-            const unsigned iter = (__ballot_sync(hm, matId == mid) >> (16 * half)) & 0xFFFF;
-            pm &= ~iter;
-            if (mid >= a.numMaterials || !a.materials[mid].has_texture) continue;
-            const DevTexture& tex = a.materials[mid].tex;
-            const float ssu = tex.scale_u * tex.scale_u, ssv = tex.scale_v * tex.scale_v;
-            const float ddx2 = fmaf(g0, g0, g1 * g1) * ssu, ddy2 = fmaf(g2, g2, g3 * g3) * ssv;
-            const int32_t mip = ilog2_x86(vmax(ddx2, ddy2)) >> 1;
-            const bool nearest = __ballot_sync(hm, mip > 0) & hm;
-            if ((iter >> l) & 1) {
-                if constexpr (kMode == kResolvePlain || kMode == kResolveDebug) {
-                    albedo = sample_rgba8(tex, texU, texV, 0, mip, nearest);
-                    if (tex.num_layers >= 2) nmr = sample_rgba8(tex, texU, texV, 1, mip, nearest);
-                } else {
-                    const TexelQuad q = texel_quad(tex, texU, texV, mip, nearest);
-                    // decoded when the model covers the level and its texture has this texture's size
-                    const bool dec = mid < nr.numMaterials && q.m < (int32_t)nr.decodedLevels && nr.tex[mid].data != nullptr &&
-                                     nr.tex[mid].width == tex.width && nr.tex[mid].height == tex.height;
-                    if constexpr (kMode == kResolveEmit) {
-                        uint32_t nq = 0;
-                        sflags = dec ? kSurfFast | kSurfDecoded | (nearest ? kSurfNearest : 0u) | (q.inX ? kSurfInX : 0u) |
-                                           (q.inY ? kSurfInY : 0u) | (tex.num_layers >= 2 ? kSurfTwoLayers : 0u)
-                                     : 0u;  // sampled from the plain texture: the second pass reconstructs
-                        sfx = q.fx, sfy = q.fy;
-                        if (dec) {
-                            const unsigned long long b = ((unsigned long long)mid << 32) | ((uint32_t)q.m << 28);
-                            const uint32_t x0 = (uint32_t)q.tx, y0 = (uint32_t)q.ty;
-                            req[0] = b | (y0 << 14) | x0, nq = 1;
-                            if (!nearest) {
-                                if (q.inX) req[1] = b | (y0 << 14) | (x0 + 1), nq++;
-                                if (q.inY) req[2] = b | ((y0 + 1) << 14) | x0, nq++;
-                                if (q.inX && q.inY) req[3] = b | ((y0 + 1) << 14) | (x0 + 1), nq++;
-                            }
-                        }
-                        const unsigned grp = iter << (16 * half);
-                        nq = 0;
-#pragma unroll
-                        for (int k = 0; k < 4; k++) {  // requests equal to a lower lane's at the same position
-                            const unsigned peers = __match_any_sync(grp, req[k]);
-                            const int lead = __ffs(peers) - 1;
-                            const uint32_t leadOff = __shfl_sync(grp, off, lead);
-                            if (req[k] == ~0ull) continue;
-                            if (lead != (int)lane) req[k] = kReqRedirect | ((unsigned long long)leadOff * 4 + k);
-                            else nq++;
-                        }
-                        const uint32_t total = __reduce_add_sync(grp, nq);
-                        if (total && (int)lane == __ffs(grp) - 1) atomicAdd(&nr.counts[mid], total);
-                    } else if (dec) {
-                        // a slot's decoded texel, or the one of the slot it redirects to
-                        const ulonglong2* rq = (const ulonglong2*)(nr.pixelReq + (size_t)off * 4);
-                        const ulonglong2 r01 = rq[0], r23 = rq[1];
-                        auto at = [&](unsigned long long r, uint32_t k) {
-                            const size_t slot = (r != ~0ull && (r & kReqRedirect)) ? (size_t)(uint32_t)r : (size_t)off * 4 + k;
-                            return nr.decoded[slot];
-                        };
-                        const uint2 d00 = at(r01.x, 0);
-                        uint2 r0 = d00;
-                        if (!nearest) {
-                            const uint2 d10 = q.inX ? at(r01.y, 1) : d00, d01 = q.inY ? at(r23.x, 2) : d00;
-                            const uint2 d11 = q.inY ? (q.inX ? at(r23.y, 3) : d01) : d10;
-                            r0.x = filter_rgba8(d00.x, d10.x, d01.x, d11.x, q.fx, q.fy);
-                            r0.y = filter_rgba8(d00.y, d10.y, d01.y, d11.y, q.fx, q.fy);
-                        }
-                        albedo = r0.x;
-                        if (tex.num_layers >= 2) nmr = r0.y;
-                    } else {
-                        albedo = sample_rgba8(tex, texU, texV, 0, mip, nearest);
-                        if (tex.num_layers >= 2) nmr = sample_rgba8(tex, texU, texV, 1, mip, nearest);
+        // Materials. The reference's waterfall picks the filter over the whole tile per material: nearest if
+        // any of the 16 pixels' gradients, scaled by that material's texture, calls for a level above 0.
+        // Textures of one size (the usual case) give one answer; others are asked per material.
+        bool sampled = (skyBits == 0 || (__match_any_sync(hm, matId) & covered) != 0) && matId < a.numMaterials;
+        if (sampled) sampled = a.materials[matId].has_texture;
+        const unsigned sampledBits = __ballot_sync(hm, sampled) & hm;
+        if (sampledBits) {
+            const DevTexture& tex = a.materials[sampled ? matId : 0].tex;
+            const float d1 = fmaf(g0, g0, g1 * g1), d2 = fmaf(g2, g2, g3 * g3);
+            const float sU = sampled ? tex.scale_u : 0.0f, sV = sampled ? tex.scale_v : 0.0f;
+            const float lU = __shfl_sync(hm, sU, __ffs(sampledBits) - 1), lV = __shfl_sync(hm, sV, __ffs(sampledBits) - 1);
+            auto level = [&](float u, float v) { return ilog2_x86(vmax(d1 * (u * u), d2 * (v * v))) >> 1; };
+            int32_t mip = level(lU, lV);
+            bool nearest = __ballot_sync(hm, mip > 0) & hm;
+            if (__ballot_sync(hm, sampled && (sU != lU || sV != lV)) & hm) {
+                unsigned pm = sampledBits;
+                while (pm) {
+                    const int src = __ffs(pm) - 1;
+                    const uint32_t mid = __shfl_sync(hm, matId, src);
+                    const float u = __shfl_sync(hm, sU, src), v = __shfl_sync(hm, sV, src);
+                    const unsigned iter = __ballot_sync(hm, matId == mid) & hm;
+                    pm &= ~iter;
+                    const int32_t m = level(u, v);
+                    const bool n = __ballot_sync(hm, m > 0) & hm;
+                    if (matId == mid) mip = m, nearest = n;
+                }
+            }
+            const TexelQuad q = texel_quad(tex, texU, texV, mip, nearest);
+            const uint32_t mid = matId;
+            // decoded when the model covers the level and its texture has this texture's size
+            bool dec = false;
+            if constexpr (kMode == kResolveEmit || kMode == kResolveNeural)
+                dec = sampled && mid < nr.numMaterials && q.m < (int32_t)nr.decodedLevels && nr.tex[mid].data != nullptr &&
+                      nr.tex[mid].width == tex.width && nr.tex[mid].height == tex.height;
+            if constexpr (kMode == kResolveEmit) {
+                uint32_t nq = 0;
+                if (sampled) {
+                    sflags = dec ? kSurfFast | kSurfDecoded | (nearest ? kSurfNearest : 0u) | (q.inX ? kSurfInX : 0u) |
+                                       (q.inY ? kSurfInY : 0u) | (tex.num_layers >= 2 ? kSurfTwoLayers : 0u)
+                                 : 0u;  // sampled from the plain texture: the second pass reconstructs
+                    sfx = q.fx, sfy = q.fy;
+                }
+                if (dec) {
+                    const unsigned long long b = ((unsigned long long)mid << 32) | ((uint32_t)q.m << 28);
+                    const uint32_t x0 = (uint32_t)q.tx, y0 = (uint32_t)q.ty;
+                    req[0] = b | (y0 << 14) | x0;
+                    if (!nearest) {
+                        if (q.inX) req[1] = b | (y0 << 14) | (x0 + 1);
+                        if (q.inY) req[2] = b | ((y0 + 1) << 14) | x0;
+                        if (q.inX && q.inY) req[3] = b | ((y0 + 1) << 14) | (x0 + 1);
                     }
                 }
+#pragma unroll
+                for (int k = 0; k < 4; k++) {  // requests equal to a lower lane's at the same position
+                    const unsigned peers = __match_any_sync(hm, req[k]);
+                    const int lead = __ffs(peers) - 1;
+                    const uint32_t leadOff = __shfl_sync(hm, off, lead);
+                    if (req[k] == ~0ull) continue;
+                    if (lead != (int)lane) req[k] = kReqRedirect | ((unsigned long long)leadOff * 4 + k);
+                    else nq++;
+                }
+                unsigned pm = __ballot_sync(hm, nq != 0) & hm;
+                while (pm) {  // the requests of each of the tile's materials
+                    const uint32_t m = __shfl_sync(hm, mid, __ffs(pm) - 1);
+                    const unsigned iter = __ballot_sync(hm, nq != 0 && mid == m) & hm;
+                    pm &= ~iter;
+                    if ((iter >> lane) & 1) {
+                        const uint32_t total = __reduce_add_sync(iter, nq);
+                        if ((int)lane == __ffs(iter) - 1) atomicAdd(&nr.counts[m], total);
+                    }
+                }
+            } else if (dec) {
+                // a slot's decoded texel, or the one of the slot it redirects to
+                const ulonglong2* rq = (const ulonglong2*)(nr.pixelReq + (size_t)off * 4);
+                const ulonglong2 r01 = rq[0], r23 = rq[1];
+                auto at = [&](unsigned long long r, uint32_t k) {
+                    const size_t slot = (r != ~0ull && (r & kReqRedirect)) ? (size_t)(uint32_t)r : (size_t)off * 4 + k;
+                    return nr.decoded[slot];
+                };
+                const uint2 d00 = at(r01.x, 0);
+                uint2 r0 = d00;
+                if (!nearest) {
+                    const uint2 d10 = q.inX ? at(r01.y, 1) : d00, d01 = q.inY ? at(r23.x, 2) : d00;
+                    const uint2 d11 = q.inY ? (q.inX ? at(r23.y, 3) : d01) : d10;
+                    r0.x = filter_rgba8(d00.x, d10.x, d01.x, d11.x, q.fx, q.fy);
+                    r0.y = filter_rgba8(d00.y, d10.y, d01.y, d11.y, q.fx, q.fy);
+                }
+                albedo = r0.x;
+                if (tex.num_layers >= 2) nmr = r0.y;
+            } else if (sampled) {
+                albedo = sample_quad(tex, q, 0, nearest);
+                if (tex.num_layers >= 2) nmr = sample_quad(tex, q, 1, nearest);
             }
         }
         if constexpr (kMode == kResolveEmit) {
@@ -543,14 +565,10 @@ __global__ void __launch_bounds__(256) k_resolve(ResolveArgs a, NeuralResolve nr
             return;
         }
         }  // !fast
-        F3 nrm[3], tan[3];
+        F3 nrm[3];
+        const float s255 = 1.0f / 255;
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const uint32_t p = ntg[k];
-            const float s = 1.0f / 255;
-            nrm[k] = unmap_oct((float)(p & 255) * s, (float)((p >> 8) & 255) * s);
-            tan[k] = unmap_oct((float)((p >> 16) & 255) * s, (float)(p >> 24) * s);
-        }
+        for (int k = 0; k < 3; k++) nrm[k] = unmap_oct((float)(ntg[k] & 255) * s255, (float)((ntg[k] >> 8) & 255) * s255);
         const float* M = a.objectToWorld;
         auto bl = [&](const F3* v) {
             return F3{ fmaf(v[0].x, b[0], fmaf(v[1].x, b[1], v[2].x * b[2])), fmaf(v[0].y, b[0], fmaf(v[1].y, b[1], v[2].y * b[2])),
@@ -563,6 +581,9 @@ __global__ void __launch_bounds__(256) k_resolve(ResolveArgs a, NeuralResolve nr
         const F3 nws = normalize3(m3(bl(nrm)));
         F3 N = nws;
         if (__ballot_sync(hm, (nmr & 0xFFFF) != 0) & hm) {
+            F3 tan[3];
+#pragma unroll
+            for (int k = 0; k < 3; k++) tan[k] = unmap_oct((float)((ntg[k] >> 16) & 255) * s255, (float)(ntg[k] >> 24) * s255);
             const F3 tws = normalize3(m3(bl(tan)));
             F3 bws = { fmaf(nws.y, tws.z, -nws.z * tws.y), fmaf(nws.z, tws.x, -nws.x * tws.z), fmaf(nws.x, tws.y, -nws.y * tws.x) };
             bws = { __uint_as_float(__float_as_uint(bws.x) ^ hand), __uint_as_float(__float_as_uint(bws.y) ^ hand),
@@ -597,7 +618,7 @@ __global__ void __launch_bounds__(256) k_resolve(ResolveArgs a, NeuralResolve nr
         const float NoV = fabsf(dot3(N, viewDir)) + 1e-5f;
         const float exposure = a.exposure * 0.001f;
         for (uint32_t i = 0; i < a.numLights; i++) {
-            const swr_light& li = a.lights[i];
+            const swr_light& li = a.lights ? a.lights[i] : a.light[i];
             F3 ld = li.type == 0 ? F3{ -li.direction[0], -li.direction[1], -li.direction[2] }
                                  : normalize3({ li.position[0] - world.x, li.position[1] - world.y, li.position[2] - world.z });
             const float NoL = dot3(N, ld);
@@ -678,7 +699,9 @@ swr_status build_resolve_args(swr_framebuffer fb, const swr_shading_context* ctx
     memcpy(a.viewPos, ctx->view_pos, sizeof(a.viewPos));
     a.exposure = ctx->exposure;
     if (ctx->skybox) a.sky = ctx->skybox->d, a.hasSky = 1;
-    if (ctx->num_lights) {
+    if (ctx->num_lights && ctx->num_lights <= kParamLights) {
+        memcpy(a.light, ctx->lights, ctx->num_lights * sizeof(swr_light));
+    } else if (ctx->num_lights) {
         swr_light* dl = nullptr;
         cudaError_t e = cudaMallocAsync(&dl, ctx->num_lights * sizeof(swr_light), st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(dl, ctx->lights, ctx->num_lights * sizeof(swr_light), cudaMemcpyHostToDevice, st);
