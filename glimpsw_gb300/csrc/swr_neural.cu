@@ -13,8 +13,8 @@
 // nearest filtering, Texture.h:412-459); AO has no source channel (layer 1 holds NX, NY, M, R;
 // Scene.h:9, Scene.cpp:31-34) and is trained towards a constant 1.
 //
-// One CTA of 128 threads works on 128-sample tiles: thread t owns sample row t, which is TMEM
-// lane t of every accumulator (M = 128). Every matrix product is a tcgen05.mma issued by thread 0
+// A CTA works on 128-sample tiles: sample row t is TMEM lane t of every accumulator (M = 128); the decoder
+// runs one thread per row, the training kernel two. Every matrix product is a tcgen05.mma issued by thread 0
 // from shared-memory operands in the slab layout of swr_tc.cuh, FP32 accumulation in TMEM,
 // completion signalled through tcgen05.commit on an mbarrier that every thread waits on with a
 // one-second limit (a timeout sets a status bit, skips the remaining work and still frees TMEM).
@@ -86,9 +86,12 @@ __device__ __forceinline__ float tanh_hw(float x) {
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float gelu(float x) {
-    const float t = tanh_hw(kGeluA * x * fmaf(kGeluB, x * x, 1.0f));
+// Both from one tanh: returns gelu(x), d receives gelu'(x).
+__device__ __forceinline__ float gelu_and_grad(float x, float& d) {
+    const float x2 = x * x;
+    const float t = tanh_hw(kGeluA * x * fmaf(kGeluB, x2, 1.0f));
     const float h = 0.5f * x;
+    d = fmaf(0.5f, t, 0.5f) + h * fmaf(-t, t, 1.0f) * kGeluA * fmaf(3.0f * kGeluB, x2, 1.0f);
     return fmaf(h, t, h);
 }
 // 2 gelu(x) = x + x tanh(sqrt(2/pi) x (1 + 0.044715 x^2)): four instructions and the tanh. The
@@ -116,12 +119,6 @@ __device__ __forceinline__ void gelu_x2_16(float (&v)[16], const float* b) {
         x = gelu_x2_pair(x);
         v[j] = x.x, v[j + 1] = x.y;
     }
-}
-__device__ __forceinline__ float gelu_grad(float x) {
-    const float x2 = x * x;
-    const float t = tanh_hw(kGeluA * x * fmaf(kGeluB, x2, 1.0f));
-    const float dt = 0.5f * x * fmaf(-t, t, 1.0f) * kGeluA * fmaf(3.0f * kGeluB, x2, 1.0f);
-    return fmaf(0.5f, t, 0.5f) + dt;
 }
 __device__ __forceinline__ float half_round(float v) { return __half2float(__float2half_rn(v)); }
 __device__ __forceinline__ float h2f(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
@@ -172,16 +169,15 @@ __device__ __forceinline__ void interpolate(const float (&c)[4][8], float fx, fl
     }
 }
 
-// Point-sampled texel of both layers as 8 targets in [0, 1]; AO = 1.
-__device__ __forceinline__ void fetch_targets(const DevTexture& t, Sample s, float* out) {
+// Point-sampled texel of both layers, and its 8 targets in [0, 1]; AO = 1.
+__device__ __forceinline__ uint2 fetch_texel(const DevTexture& t, Sample s) {
     const int32_t stride = (int32_t)t.row_shift - (int32_t)s.level;
     const uint32_t off = t.mip_offsets[s.level & 15] + texel_offset((int32_t)s.tx, (int32_t)s.ty, stride);
-    const uint32_t a0 = t.data[off];
-    const uint32_t a1 = t.num_layers >= 2 ? t.data[(size_t)t.layer_stride + off] : 0u;
-    const float k = 1.0f / 255.0f;
-    out[0] = (float)(a0 & 255) * k, out[1] = (float)((a0 >> 8) & 255) * k, out[2] = (float)((a0 >> 16) & 255) * k;
-    out[3] = (float)(a1 & 255) * k, out[4] = (float)((a1 >> 8) & 255) * k, out[5] = (float)((a1 >> 16) & 255) * k;
-    out[6] = (float)(a1 >> 24) * k, out[7] = 1.0f;
+    return make_uint2(t.data[off], t.num_layers >= 2 ? t.data[(size_t)t.layer_stride + off] : 0u);
+}
+__device__ __forceinline__ float target_of(uint2 a, int c) {
+    const uint32_t v = c < 3 ? a.x >> (8 * c) : a.y >> (8 * (c - 3));
+    return c == 7 ? 1.0f : (float)(v & 255) * (1.0f / 255.0f);
 }
 
 __device__ Sample draw_sample(const NeuralTrainArgs& a, const DevTexture& t, uint32_t slot, uint32_t s) {
@@ -237,39 +233,50 @@ __device__ __forceinline__ void load_latent_f16(const uint16_t* L, const Taps& q
 }
 
 // Synchronise the CTA (publishing its shared-memory operand writes to the tensor cores), let
-// thread 0 issue `issue()` and commit, and wait for completion. Returns the CTA-uniform status.
+// thread 0 issue `issue()` and commit, and wait for completion. A thread whose wait gave up clears its
+// own `mine`; the next round's barrier tells every thread, so the returned verdict is CTA-uniform (and
+// one round late) without a second barrier per round. Once false, no thread issues or waits again.
 template <class F>
-__device__ __forceinline__ bool tc_round(bool ok, uint64_t* bar, uint32_t& phase, uint64_t limitNs, F&& issue) {
+__device__ __forceinline__ bool tc_round(bool& mine, uint64_t* bar, uint32_t& phase, uint64_t limitNs, F&& issue) {
     fence_proxy_async();
     fence_before_sync();
-    ok = __syncthreads_and(ok);
+    const bool ok = __syncthreads_and(mine);
     fence_after_sync();
-    if (!ok) return false;
+    if (!ok) {
+        mine = false;
+        return false;
+    }
     if (threadIdx.x == 0) {
         issue();
         mma_commit(bar);
     }
-    ok = mbar_wait_drained(bar, phase, limitNs);
+    mine = mbar_wait_drained(bar, phase, limitNs);
     phase ^= 1;
-    ok = __syncthreads_and(ok);  // every thread leaves with the same verdict
     fence_after_sync();
-    return ok;
+    return true;
 }
 
-__global__ void __launch_bounds__(128) k_neural_train(const __grid_constant__ NeuralTrainArgs a) {
+// 256 threads per 128-sample tile: threads t and t + 128 share sample row t (TMEM lane t, which warps w
+// and w + 4 may both read) and take half of the hidden columns each; of the row's other work, the first
+// reads the latents and scatters their gradient, the second reads the targets and forms the loss. The
+// tile's six dependent rounds are bound by latency (one CTA of 128 threads had one warp per scheduler in
+// its element-wise stages; two CTAs fit an SM): a step of 8 materials x 8192 samples 40.8 -> 30.2 us, with one
+// barrier a round instead of two and gelu and its derivative from one tanh.
+constexpr uint32_t kTrainThreads = 256;
+__global__ void __launch_bounds__(kTrainThreads, 2) k_neural_train(const __grid_constant__ NeuralTrainArgs a) {
     extern __shared__ __align__(1024) uint8_t sm[];
     uint64_t* barMma = (uint64_t*)(sm + kSBar);
     uint64_t* barLoad = barMma + 1;
     uint32_t* tmemSlot = (uint32_t*)(barMma + 2);
     float* red = (float*)(barMma + 3);
-    const uint32_t t = threadIdx.x, warp = t >> 5;
+    const uint32_t t = threadIdx.x & 127, hf = threadIdx.x >> 7, warp = threadIdx.x >> 5;
     const uint32_t slot = blockIdx.x / a.ctasPerMaterial, sub = blockIdx.x - slot * a.ctasPerMaterial;
     const uint32_t mat = a.materials[slot];
     const DevTexture& tex = a.n.tex[mat];
     const uint32_t tilesPerMat = a.samplesPerMaterial / 128;
     const uint32_t tBegin = sub * tilesPerMat / a.ctasPerMaterial, tEnd = (sub + 1) * tilesPerMat / a.ctasPerMaterial;
 
-    if (t == 0) {
+    if (threadIdx.x == 0) {
         mbar_init(barMma, 1);
         mbar_init(barLoad, 1);
         fence_mbar_init();
@@ -278,26 +285,28 @@ __global__ void __launch_bounds__(128) k_neural_train(const __grid_constant__ Ne
         tmem_alloc(tmemSlot, kTrainTmemCols);
         tmem_relinquish();
     }
-    {
-        const float one[8] = { 1.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f }, zero[8] = {};
+    if (hf == 0) {
+        const float one[8] = { 1.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
         store_row8(sm + kSR, 128, 8, t, one);   // ONES slab: feature 0 = 1
+    } else {
+        const float zero[8] = {};
         store_row8(sm + kSP, 128, 1, t, zero);  // DY columns 8-15
     }
     fence_proxy_async();
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    if (t == 0) {
+    if (threadIdx.x == 0) {
         mbar_arrive_expect_tx(barLoad, kNeuralImage);
         bulk_g2s(sm, a.n.image + (size_t)mat * kNeuralImage, kNeuralImage, barLoad);
     }
     const uint32_t tmem = *tmemSlot;
-    const uint32_t tRow = tmem + ((warp * 32) << 16);
+    const uint32_t tRow = tmem + (((warp & 3) * 32) << 16);
     const uint32_t sb = smem_u32(sm);
-    bool ok = mbar_wait_drained(barLoad, 0, a.n.waitNs);
+    bool ok = true, mine = true, loaded = false;
     uint32_t phase = 0;
     float lossAcc = 0.f;
-    const float* b2 = (const float*)(sm + kIB2);
+    const float* b2 = (const float*)(sm + kIB2) + 32 * hf;
     const float* b3 = (const float*)(sm + kIB3);
     const size_t matLatent = (size_t)mat * a.n.texelsPerMaterial;
     const float* latent = a.latent + matLatent * 8;
@@ -307,105 +316,110 @@ __global__ void __launch_bounds__(128) k_neural_train(const __grid_constant__ Ne
 
     for (uint32_t tile = tBegin; tile < tEnd && ok; tile++) {
         const Sample smp = draw_sample(a, tex, slot, tile * 128 + t);
-        float target[8];
-        fetch_targets(tex, smp, target);
-        const Taps q = latent_taps(a.n, smp);
-        float x0[8];
-        {
-            float c[4][8];
+        // What the tile's end needs of its start, in the same registers: the first half's latent taps, the
+        // second's texel.
+        uint32_t keep[6] = {};
+        if (hf == 0) {
+            const Taps q = latent_taps(a.n, smp);
+#pragma unroll
+            for (int k = 0; k < 4; k++) keep[k] = q.idx[k];
+            keep[4] = __float_as_uint(q.fx), keep[5] = __float_as_uint(q.fy);
+            float x0[8], c[4][8];
             load_latent_f32(latent, q, c);
             interpolate(c, q.fx, q.fy, x0);
-        }
-        store_row8(sm + kSQ, 128, 8, t, x0);
-        {
+            store_row8(sm + kSQ, 128, 8, t, x0);
+        } else {
+            const uint2 texel = fetch_texel(tex, smp);
+            keep[0] = texel.x, keep[1] = texel.y;
             float li[8];
             level_inputs(smp.level, li);
             store_row8(sm + kSQ, 128, 9, t, li);  // X0 columns 8-15
         }
+        if (!loaded) {  // the weights, first needed here
+            mine = mbar_wait_drained(barLoad, 0, a.n.waitNs);
+            loaded = true;
+        }
         // ---- layer 1
-        ok = tc_round(ok, barMma, phase, a.n.waitNs, [&] {
+        ok = tc_round(mine, barMma, phase, a.n.waitNs, [&] {
             mma_bf16(tmem + kT0, desc_kmajor(sb + kSQ + 8 * kSlab, 128), desc_kmajor(sb + kIW1, 64), iFwd128x64, 0);
         });
-        float z1[64];
+        float d1[32];  // gelu'(z1) of the thread's columns
 #pragma unroll
-        for (int c = 0; c < 4; c++) tmem_ld16(tRow + kT0 + 16 * c, z1 + 16 * c);
+        for (int c = 0; c < 2; c++) {
+            float v[16];
+            tmem_ld16(tRow + kT0 + 32 * hf + 16 * c, v);
 #pragma unroll
-        for (int s = 0; s < 8; s++) {
-            float h[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) h[j] = gelu(z1[8 * s + j]);
-            store_row8(sm + kSQ, 128, s, t, h);
+            for (int j = 0; j < 16; j++) v[j] = gelu_and_grad(v[j], d1[16 * c + j]);
+            store_row8(sm + kSQ, 128, 4 * hf + 2 * c, t, v);
+            store_row8(sm + kSQ, 128, 4 * hf + 2 * c + 1, t, v + 8);
         }
         // ---- layer 2
-        ok = tc_round(ok, barMma, phase, a.n.waitNs, [&] {
+        ok = tc_round(mine, barMma, phase, a.n.waitNs, [&] {
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++)
                 mma_bf16(tmem + kT0, desc_kmajor(sb + kSQ + 2 * k * kSlab, 128), desc_kmajor(sb + kIW2 + 2 * k * 1024, 64),
                          iFwd128x64, k);
         });
-        float z2[64];
+        float d2[32];
 #pragma unroll
-        for (int c = 0; c < 4; c++) tmem_ld16(tRow + kT0 + 16 * c, z2 + 16 * c);
+        for (int c = 0; c < 2; c++) {
+            float v[16];
+            tmem_ld16(tRow + kT0 + 32 * hf + 16 * c, v);
 #pragma unroll
-        for (int s = 0; s < 8; s++) {
-            float h[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                z2[8 * s + j] += b2[8 * s + j];
-                h[j] = gelu(z2[8 * s + j]);
-            }
-            store_row8(sm + kSR, 128, s, t, h);
+            for (int j = 0; j < 16; j++) v[j] = gelu_and_grad(v[j] + b2[16 * c + j], d2[16 * c + j]);
+            store_row8(sm + kSR, 128, 4 * hf + 2 * c, t, v);
+            store_row8(sm + kSR, 128, 4 * hf + 2 * c + 1, t, v + 8);
         }
         // ---- layer 3 and the loss gradient
-        ok = tc_round(ok, barMma, phase, a.n.waitNs, [&] {
+        ok = tc_round(mine, barMma, phase, a.n.waitNs, [&] {
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++)
                 mma_bf16(tmem + kT0, desc_kmajor(sb + kSR + 2 * k * kSlab, 128), desc_kmajor(sb + kIW3 + 2 * k * 256, 16),
                          iFwd128x16, k);
         });
-        {
+        if (hf == 1) {  // whole warps
             float y[16], dy[8];
             tmem_ld16(tRow + kT0, y);
 #pragma unroll
             for (int c = 0; c < 8; c++) {
-                const float e = (y[c] + b3[c]) - target[c];
+                const float e = (y[c] + b3[c]) - target_of(make_uint2(keep[0], keep[1]), c);
                 lossAcc += e * e;
                 dy[c] = e * kGradScale;
             }
             store_row8(sm + kSP, 128, 0, t, dy);
         }
         // ---- dh2 = (DY W3) * gelu'(z2)
-        ok = tc_round(ok, barMma, phase, a.n.waitNs, [&] {
+        ok = tc_round(mine, barMma, phase, a.n.waitNs, [&] {
             mma_bf16(tmem + kT0, desc_kmajor(sb + kSP, 128), desc_kmajor(sb + kIW3t, 64), iFwd128x64, 0);
         });
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
+        for (int c = 0; c < 2; c++) {
             float v[16];
-            tmem_ld16(tRow + kT0 + 16 * c, v);
+            tmem_ld16(tRow + kT0 + 32 * hf + 16 * c, v);
 #pragma unroll
-            for (int j = 0; j < 16; j++) v[j] *= gelu_grad(z2[16 * c + j]);
-            store_row8(sm + kSP, 128, 2 + 2 * c, t, v);
-            store_row8(sm + kSP, 128, 3 + 2 * c, t, v + 8);
+            for (int j = 0; j < 16; j++) v[j] *= d2[16 * c + j];
+            store_row8(sm + kSP, 128, 2 + 4 * hf + 2 * c, t, v);
+            store_row8(sm + kSP, 128, 3 + 4 * hf + 2 * c, t, v + 8);
         }
         // ---- dh1 = (DH2 W2) * gelu'(z1)
-        ok = tc_round(ok, barMma, phase, a.n.waitNs, [&] {
+        ok = tc_round(mine, barMma, phase, a.n.waitNs, [&] {
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++)
                 mma_bf16(tmem + kT0, desc_kmajor(sb + kSP + (2 + 2 * k) * kSlab, 128),
                          desc_kmajor(sb + kIW2t + 2 * k * 1024, 64), iFwd128x64, k);
         });
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
+        for (int c = 0; c < 2; c++) {
             float v[16];
-            tmem_ld16(tRow + kT0 + 16 * c, v);
+            tmem_ld16(tRow + kT0 + 32 * hf + 16 * c, v);
 #pragma unroll
-            for (int j = 0; j < 16; j++) v[j] *= gelu_grad(z1[16 * c + j]);
-            store_row8(sm + kSP, 128, 10 + 2 * c, t, v);
-            store_row8(sm + kSP, 128, 11 + 2 * c, t, v + 8);
+            for (int j = 0; j < 16; j++) v[j] *= d1[16 * c + j];
+            store_row8(sm + kSP, 128, 10 + 4 * hf + 2 * c, t, v);
+            store_row8(sm + kSP, 128, 11 + 4 * hf + 2 * c, t, v + 8);
         }
         // ---- dx0 = DH1 W1, and the weight-gradient accumulators
         const uint32_t acc = tile > tBegin ? 1u : 0u;
-        ok = tc_round(ok, barMma, phase, a.n.waitNs, [&] {
+        ok = tc_round(mine, barMma, phase, a.n.waitNs, [&] {
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++)
                 mma_bf16(tmem + kT0, desc_kmajor(sb + kSP + (10 + 2 * k) * kSlab, 128),
@@ -419,12 +433,16 @@ __global__ void __launch_bounds__(128) k_neural_train(const __grid_constant__ Ne
                 mma_bf16(tmem + kTGb, desc_mnmajor(sb + kSR + i * 256, 128), desc_mnmajor(sb + kSP + i * 256, 128), iGrad,
                          acc | (i > 0));
         });
-        {
+        if (hf == 0) {
             float d[16];
             tmem_ld16(tRow + kT0, d);
+            Taps q;
+#pragma unroll
+            for (int k = 0; k < 4; k++) q.idx[k] = keep[k];
+            q.fx = __uint_as_float(keep[4]), q.fy = __uint_as_float(keep[5]);
             const float gx = 1.0f - q.fx, gy = 1.0f - q.fy;
             const float w[4] = { gx * gy, q.fx * gy, gx * q.fy, q.fx * q.fy };
-            if (ok) {
+            if (ok && mine) {
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
                     if (!tap_used(q, k)) continue;
@@ -435,48 +453,51 @@ __global__ void __launch_bounds__(128) k_neural_train(const __grid_constant__ Ne
             }
         }
     }
-    ok = __syncthreads_and(ok);
+    if (!loaded) mine = mbar_wait_drained(barLoad, 0, a.n.waitNs);  // a CTA without tiles: its copy still lands
+    ok = __syncthreads_and(mine);
+    fence_after_sync();
 
-    // ---- this CTA's parameter gradients
+    // ---- this CTA's parameter gradients, half of the columns per thread
     float* out = a.partial + (size_t)blockIdx.x * kNeuralParams;
     if (!ok || tEnd == tBegin) {
-        for (uint32_t i = t; i < kNeuralParams; i += 128) out[i] = 0.f;
+        for (uint32_t i = threadIdx.x; i < kNeuralParams; i += kTrainThreads) out[i] = 0.f;
     } else {  // every entry is written below (W1 columns 11-15 multiply zero inputs: 0)
         float v[16];
-        if (warp < 2) {  // rows 0-63: dW2 row o = t, dW3^T row i = t
+        if ((warp & 3) < 2) {  // rows 0-63: dW2 row o = t, dW3^T row i = t
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                tmem_ld16(tRow + kTGa + 16 * c, v);
+            for (int c = 0; c < 2; c++) {
+                tmem_ld16(tRow + kTGa + 32 * hf + 16 * c, v);
 #pragma unroll
-                for (int j = 0; j < 16; j++) out[kPW2 + t * 64 + 16 * c + j] = v[j];
+                for (int j = 0; j < 16; j++) out[kPW2 + t * 64 + 32 * hf + 16 * c + j] = v[j];
             }
-            tmem_ld16(tRow + kTGb, v);
+            if (hf == 0) {
+                tmem_ld16(tRow + kTGb, v);
 #pragma unroll
-            for (int o = 0; o < 8; o++) out[kPW3 + o * 64 + t] = v[o];
-        } else {  // rows 64-127: dW1 row o = t - 64; row 64 of G_b: db3, db2
+                for (int o = 0; o < 8; o++) out[kPW3 + o * 64 + t] = v[o];
+            }
+        } else if (hf == 0) {  // rows 64-127: dW1 row o = t - 64
             tmem_ld16(tRow + kTGa + 64, v);
 #pragma unroll
             for (int j = 0; j < 16; j++) out[kPW1 + (t - 64) * 16 + j] = v[j];
-            if (warp == 2) {
-                tmem_ld16(tRow + kTGb, v);
-                if (t == 64)
-                    for (int o = 0; o < 8; o++) out[kPB3 + o] = v[o];
+        } else if ((warp & 3) == 2) {  // row 64 of G_b: db3, db2
+            tmem_ld16(tRow + kTGb, v);
+            if (t == 64)
+                for (int o = 0; o < 8; o++) out[kPB3 + o] = v[o];
 #pragma unroll
-                for (int c = 1; c < 5; c++) {
-                    tmem_ld16(tRow + kTGb + 16 * c, v);
-                    if (t == 64)
-                        for (int j = 0; j < 16; j++) out[kPB2 + 16 * (c - 1) + j] = v[j];
-                }
+            for (int c = 1; c < 5; c++) {
+                tmem_ld16(tRow + kTGb + 16 * c, v);
+                if (t == 64)
+                    for (int j = 0; j < 16; j++) out[kPB2 + 16 * (c - 1) + j] = v[j];
             }
         }
     }
     // ---- loss
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) lossAcc += __shfl_xor_sync(0xFFFFFFFFu, lossAcc, o);
-    if ((t & 31) == 0) red[warp] = lossAcc;
+    if (hf == 1 && (t & 31) == 0) red[warp & 3] = lossAcc;
     fence_before_sync();
     __syncthreads();
-    if (t == 0) {
+    if (threadIdx.x == 0) {
         atomicAdd(a.loss, red[0] + red[1] + red[2] + red[3]);
         atomicAdd(a.loss + 1, (float)(128 * (tEnd - tBegin)));
         if (!ok) atomicOr(a.status, 1u);
@@ -648,17 +669,17 @@ __global__ void __launch_bounds__(128) k_neural_decode(const __grid_constant__ N
         else hi = mid;
     }
     uint32_t mat = lo, loaded = 0xFFFFFFFFu, phase = 0, loadPhase = 0;
-    bool ok = true;
+    bool ok = true, mine = true;
     for (uint32_t tile = tb; tile < te && ok; tile++) {
         while (tile >= a.tileOffset[mat + 1]) mat++;
         if (mat != loaded) {
-            ok = __syncthreads_and(ok);  // the previous tile's readers of the image are done
+            __syncthreads();  // the previous tile's readers of the image are done
             if (t == 0) {
                 fence_proxy_async();
                 mbar_arrive_expect_tx(barLoad, kNeuralFwdImage);
                 bulk_g2s(sm, a.n.image + (size_t)mat * kNeuralImage, kNeuralFwdImage, barLoad);
             }
-            ok = mbar_wait_drained(barLoad, loadPhase, a.n.waitNs) && ok;
+            mine = mbar_wait_drained(barLoad, loadPhase, a.n.waitNs) && mine;
             loadPhase ^= 1;
             loaded = mat;
             // W2 and W3 halved in place: the activations they weigh are 2 gelu (gelu_x2)
@@ -683,7 +704,7 @@ __global__ void __launch_bounds__(128) k_neural_decode(const __grid_constant__ N
             level_inputs(smp.level, li);
             store_row8(sm + kDX, 128, 1, t, li);
         }
-        ok = tc_round(ok, barMma, phase, a.n.waitNs, [&] {
+        ok = tc_round(mine, barMma, phase, a.n.waitNs, [&] {
             mma_bf16(tmem, desc_kmajor(sb + kDX, 128), desc_kmajor(sb + kIW1, 64), i64, 0);
         });
 #pragma unroll
@@ -694,7 +715,7 @@ __global__ void __launch_bounds__(128) k_neural_decode(const __grid_constant__ N
             store_row8(sm + kDH1, 128, 2 * c, t, v);
             store_row8(sm + kDH1, 128, 2 * c + 1, t, v + 8);
         }
-        ok = tc_round(ok, barMma, phase, a.n.waitNs, [&] {
+        ok = tc_round(mine, barMma, phase, a.n.waitNs, [&] {
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++)
                 mma_bf16(tmem, desc_kmajor(sb + kDH1 + 2 * k * kSlab, 128), desc_kmajor(sb + kIW2 + 2 * k * 1024, 64), i64, k);
@@ -707,21 +728,21 @@ __global__ void __launch_bounds__(128) k_neural_decode(const __grid_constant__ N
             store_row8(sm + kDH2, 128, 2 * c, t, v);
             store_row8(sm + kDH2, 128, 2 * c + 1, t, v + 8);
         }
-        ok = tc_round(ok, barMma, phase, a.n.waitNs, [&] {
+        ok = tc_round(mine, barMma, phase, a.n.waitNs, [&] {
 #pragma unroll
             for (uint32_t k = 0; k < 4; k++)
                 mma_bf16(tmem, desc_kmajor(sb + kDH2 + 2 * k * kSlab, 128), desc_kmajor(sb + kIW3 + 2 * k * 256, 16), i16, k);
         });
         float y[16];
         tmem_ld16(tRow, y);
-        if (valid && ok) {
+        if (valid && ok && mine) {
             uint32_t u[8];
 #pragma unroll
             for (int c = 0; c < 8; c++) u[c] = unorm8(y[c] + b3[c]);
             a.out[req >> 32] = make_uint2(u[0] | (u[1] << 8) | (u[2] << 16) | (u[7] << 24), u[3] | (u[4] << 8) | (u[5] << 16) | (u[6] << 24));
         }
     }
-    ok = __syncthreads_and(ok);
+    ok = __syncthreads_and(mine);
     if (t == 0 && !ok) atomicOr(a.status, 1u);
     fence_before_sync();
     __syncthreads();
@@ -800,7 +821,7 @@ void launch_neural_train(const NeuralTrainArgs& a, uint32_t blocks, cudaStream_t
         cudaFuncSetAttribute(k_neural_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem);
         attr = true;
     }
-    k_neural_train<<<blocks, 128, kTrainSmem, st>>>(a);
+    k_neural_train<<<blocks, kTrainThreads, kTrainSmem, st>>>(a);
 }
 void launch_neural_adam(const NeuralAdamArgs& a, cudaStream_t st) {
     k_neural_adam_params<<<dim3((kNeuralParams + 127) / 128, a.numSlots), 128, 0, st>>>(a);
