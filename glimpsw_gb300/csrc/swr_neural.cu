@@ -266,6 +266,7 @@ __device__ __forceinline__ bool tc_round(bool& mine, uint64_t* bar, uint32_t& ph
 constexpr uint32_t kTrainThreads = 256;
 __global__ void __launch_bounds__(kTrainThreads, 2) k_neural_train(const __grid_constant__ NeuralTrainArgs a) {
     extern __shared__ __align__(1024) uint8_t sm[];
+    if (a.invalid && *a.invalid) return;  // before anything is allocated
     uint64_t* barMma = (uint64_t*)(sm + kSBar);
     uint64_t* barLoad = barMma + 1;
     uint32_t* tmemSlot = (uint32_t*)(barMma + 2);
@@ -554,6 +555,35 @@ __device__ __forceinline__ void adam_update(float g, float& m, float& v, float& 
     w -= __fdividef(lrm * m, fmaf(sqrt_approx(v), s2, eps));
 }
 
+// Parameter i of the CTAs' partial gradients, summed in CTA order with 8 loads in flight.
+__device__ __forceinline__ float sum_partials(const float* part, uint32_t ctas, uint32_t i) {
+    float g = 0.f;
+    uint32_t c = 0;
+    for (; c + 8 <= ctas; c += 8) {
+        float q[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) q[k] = part[(size_t)(c + k) * kNeuralParams + i];
+#pragma unroll
+        for (int k = 0; k < 8; k++) g += q[k];
+    }
+    for (; c < ctas; c++) g += part[(size_t)c * kNeuralParams + i];
+    return g;
+}
+__global__ void __launch_bounds__(64) k_neural_sum(const float* partial, uint32_t ctas, float* out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kNeuralParams) out[i] = sum_partials(partial, ctas, i);
+}
+
+__global__ void k_neural_check(const uint32_t* __restrict__ texels, uint32_t count, uint32_t decodedLevels, uint32_t width,
+                               uint32_t height, uint32_t* invalid) {
+    bool bad = false;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const Sample s = unpack_sample(texels[i]);
+        bad = bad || s.level >= decodedLevels || s.tx >= (width >> s.level) || s.ty >= (height >> s.level);
+    }
+    if (bad) *invalid = 1;
+}
+
 // Adam on the parameters of the step's materials (sum of the CTAs' partial gradients in a fixed
 // order), then the new BF16 image.
 __device__ __forceinline__ void adam_params(const NeuralAdamArgs& a, uint32_t slot, uint32_t i) {
@@ -561,18 +591,8 @@ __device__ __forceinline__ void adam_params(const NeuralAdamArgs& a, uint32_t sl
     float* p = a.params + (size_t)mat * kNeuralParams;
     float* m = a.m + (size_t)mat * kNeuralParams;
     float* v = a.v + (size_t)mat * kNeuralParams;
-    const float* part = a.partial + (size_t)slot * a.ctasPerMaterial * kNeuralParams;
     if (i < kNeuralParams) {
-        float g = 0.f;
-        uint32_t c = 0;
-        for (; c + 8 <= a.ctasPerMaterial; c += 8) {  // 8 loads in flight, summed in CTA order
-            float q[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) q[k] = part[(size_t)(c + k) * kNeuralParams + i];
-#pragma unroll
-            for (int k = 0; k < 8; k++) g += q[k];
-        }
-        for (; c < a.ctasPerMaterial; c++) g += part[(size_t)c * kNeuralParams + i];
+        const float g = sum_partials(a.partial + (size_t)slot * a.ctasPerMaterial * kNeuralParams, a.ctasPerMaterial, i);
         float mi = m[i], vi = v[i], w = p[i];
         adam_update(g, mi, vi, w, a.beta1, a.beta2, a.lrm[slot], a.s2[slot], a.eps);
         m[i] = mi, v[i] = vi, p[i] = w;
@@ -645,10 +665,12 @@ __device__ __forceinline__ uint32_t unorm8(float v) {
     return (uint32_t)__float2int_rn(fminf(fmaxf(v, 0.0f), 1.0f) * 255.0f);
 }
 
-__global__ void __launch_bounds__(128) k_neural_decode(const __grid_constant__ NeuralDecodeArgs a) {
+__global__ void __launch_bounds__(128, 7) k_neural_decode(const __grid_constant__ NeuralDecodeArgs a) {
     extern __shared__ __align__(1024) uint8_t sm[];
+    if (a.invalid && *a.invalid) return;
     const uint32_t numMat = a.n.numMaterials;
-    const uint32_t total = a.tileOffset[numMat];
+    const bool lists = a.sorted != nullptr;  // requests grouped by material, or one material's texels
+    const uint32_t total = lists ? a.tileOffset[numMat] : (a.count + 127) / 128;
     const uint32_t tb = (uint32_t)((uint64_t)blockIdx.x * total / gridDim.x);
     const uint32_t te = (uint32_t)((uint64_t)(blockIdx.x + 1) * total / gridDim.x);
     if (tb >= te) return;
@@ -675,7 +697,7 @@ __global__ void __launch_bounds__(128) k_neural_decode(const __grid_constant__ N
     const float* b3 = (const float*)(sm + kIB3);
     const uint32_t i64 = idesc_bf16(128, 64, false, false), i16 = idesc_bf16(128, 16, false, false);
     // first material with tiles at or after tb
-    uint32_t lo = 0, hi = numMat;
+    uint32_t lo = lists ? 0u : a.material, hi = lists ? numMat : a.material;
     while (lo < hi) {
         const uint32_t mid = (lo + hi) / 2;
         if (a.tileOffset[mid + 1] <= tb) lo = mid + 1;
@@ -684,7 +706,7 @@ __global__ void __launch_bounds__(128) k_neural_decode(const __grid_constant__ N
     uint32_t mat = lo, loaded = 0xFFFFFFFFu, phase = 0, loadPhase = 0;
     bool ok = true, mine = true;
     for (uint32_t tile = tb; tile < te && ok; tile++) {
-        while (tile >= a.tileOffset[mat + 1]) mat++;
+        while (lists && tile >= a.tileOffset[mat + 1]) mat++;
         if (mat != loaded) {
             __syncthreads();  // the previous tile's readers of the image are done
             if (t == 0) {
@@ -700,9 +722,17 @@ __global__ void __launch_bounds__(128) k_neural_decode(const __grid_constant__ N
             const __nv_bfloat162 half2 = __floats2bfloat162_rn(0.5f, 0.5f);
             for (uint32_t i = t; i < (kIB2 - kIW2) / 4; i += blockDim.x) w[i] = __hmul2(w[i], half2);
         }
-        const uint32_t first = a.reqOffset[mat] + (tile - a.tileOffset[mat]) * 128;
-        const bool valid = first + t < a.reqOffset[mat + 1];
-        const unsigned long long req = valid ? a.sorted[first + t] : 0ull;
+        bool valid;
+        unsigned long long req = 0;
+        if (lists) {
+            const uint32_t first = a.reqOffset[mat] + (tile - a.tileOffset[mat]) * 128;
+            valid = first + t < a.reqOffset[mat + 1];
+            if (valid) req = a.sorted[first + t];
+        } else {
+            const uint32_t i = tile * 128 + t;
+            valid = i < a.count;
+            if (valid) req = ((unsigned long long)i << 32) | a.texels[i];
+        }
         const Sample smp = unpack_sample((uint32_t)req);
         const Taps q = latent_taps(a.n, smp);
         float x0[8];
@@ -828,6 +858,13 @@ __global__ void __launch_bounds__(kScatterThreads) k_neural_scatter(const unsign
 
 }  // namespace
 
+void launch_neural_check(const uint32_t* texels, uint32_t count, uint32_t decodedLevels, uint32_t width, uint32_t height,
+                         uint32_t* invalid, cudaStream_t st) {
+    k_neural_check<<<std::min((count + 255) / 256, 1216u), 256, 0, st>>>(texels, count, decodedLevels, width, height, invalid);
+}
+void launch_neural_sum(const float* partial, uint32_t ctas, float* out, cudaStream_t st) {
+    k_neural_sum<<<(kNeuralParams + 63) / 64, 64, 0, st>>>(partial, ctas, out);
+}
 void launch_neural_train(const NeuralTrainArgs& a, uint32_t blocks, cudaStream_t st) {
     static bool attr = false;
     if (!attr) {

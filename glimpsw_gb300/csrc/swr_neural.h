@@ -49,6 +49,7 @@ struct NeuralTrainArgs {
     float* latentGrad;          // same shape, accumulated by the step
     float* partial;             // [block][kNeuralParams] parameter gradients of each block
     const uint32_t* samples;    // optional explicit samples [slot][samplesPerMaterial]: level<<28 | ty<<14 | tx
+    const uint32_t* invalid;    // with explicit samples: nonzero if one lies outside the texture (nothing runs)
     float* loss;                // [0] += squared error, [1] += samples
     uint32_t* status;           // bit 0: a tensor-core wait timed out
     uint32_t materials[kNeuralMaxStepMaterials];
@@ -82,8 +83,18 @@ struct NeuralDecodeArgs {
     const uint32_t* tileOffset;         // [numMaterials + 1] first 128-request tile of each material
     uint2* out;                         // [slot] decoded (layer 0 RGBA8 with AO in alpha, layer 1 RGBA8)
     uint32_t* status;
+    // without lists (sorted == nullptr): the count texels of one material, decoded to slots 0, 1, ...
+    const uint32_t* texels;
+    const uint32_t* invalid;            // nonzero if one of them lies outside the texture (nothing runs)
+    uint32_t material, count;
 };
 
+// Sets *invalid if one of the packed texels (level<<28 | ty<<14 | tx) is outside the decoded levels of a width x
+// height texture.
+void launch_neural_check(const uint32_t* texels, uint32_t count, uint32_t decodedLevels, uint32_t width, uint32_t height,
+                         uint32_t* invalid, cudaStream_t st);
+// out[i] = the sum of partial[c][i] over the c < ctas gradients, in that order.
+void launch_neural_sum(const float* partial, uint32_t ctas, float* out, cudaStream_t st);
 void launch_neural_train(const NeuralTrainArgs& a, uint32_t blocks, cudaStream_t st);
 void launch_neural_adam(const NeuralAdamArgs& a, cudaStream_t st);
 void launch_neural_decode(const NeuralDecodeArgs& a, uint32_t blocks, cudaStream_t st);
@@ -118,8 +129,8 @@ struct swr_neural_t {
     uint8_t* image;
     float* partial;
     size_t partialFloats;
-    float* loss;                             // device [2]
-    uint32_t* status;                        // device
+    float* loss;                             // device: squared error, samples, then the status word
+    uint32_t* status;                        // device: loss + 2
     std::vector<uint32_t> steps;             // Adam step count per material
     uint64_t seed;
     uint32_t trainCalls;

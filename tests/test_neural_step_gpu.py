@@ -66,3 +66,34 @@ def test_first_step(size, group, batch):
         assert np.array_equal(made[0].get_params(i), before[i][0].astype(np.float32))
         assert np.array_equal(made[0].get_latents(i), before[i][1].astype(np.float32))
     assert abs(loss - total / (batch * 8)) <= 1e-5 * abs(loss)
+
+
+@pytest.mark.parametrize("count", [1, 127, 128, 129, 20_001])
+def test_decode_counts_and_refused_texels(count):
+    """Any number of texels decodes as the same texels of a longer list do; one texel outside the decoded
+    levels refuses the call and leaves the caller's buffers alone, for decoding and for gradients."""
+    import torch
+    api = _setup_stream()
+    size = 128
+    tex = _device_texture([scenes.value_noise_rgba(size, 61, cells=8, layer=l) for l in range(2)], size)
+    m = api.NeuralMaterials([tex, None], latent_levels=4, seed=3)
+    packed = _samples(0, 0, 20_224, size)
+    dev = torch.from_numpy(packed.view(np.int32)).cuda()
+    whole = torch.zeros(len(packed), 2, dtype=torch.int32, device="cuda")
+    m.decode(0, dev, len(packed), whole)
+    out = torch.full((count + 1, 2), -7, dtype=torch.int32, device="cuda")
+    m.decode(0, dev, count, out)
+    assert torch.equal(out[:count], whole[:count]) and bool((out[count] == -7).all())
+    for bad in (api.pack_texel(6, 0, 0), api.pack_texel(0, size, 0), api.pack_texel(2, 0, size >> 2)):
+        wrong = packed[: (count + 127) // 128 * 128].copy()
+        wrong[count - 1] = bad
+        wdev = torch.from_numpy(wrong.view(np.int32)).cuda()
+        out.fill_(-7)
+        with pytest.raises(api.SwrError) as e:
+            m.decode(0, wdev, count, out)
+        assert e.value.code == api.SWR_EINVAL and bool((out == -7).all())
+        with pytest.raises(api.SwrError) as e:
+            m.gradients(0, wdev, len(wrong))
+        assert e.value.code == api.SWR_EINVAL
+    m.decode(0, dev, len(packed), out := torch.zeros_like(whole))
+    assert torch.equal(out, whole)
