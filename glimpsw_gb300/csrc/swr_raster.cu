@@ -23,6 +23,7 @@
 // tile is shaded, an upper bound of the triangle's depth over the tile is compared with it; a tile
 // the triangle cannot win anywhere is skipped. The vis-buffer is unchanged (only fragments that
 // would fail the depth test are skipped), while the dense scenes' overdraw mostly disappears.
+#include <algorithm>
 #include <cfloat>
 #include <mutex>
 #include <numeric>
@@ -39,7 +40,7 @@ namespace swr {
 constexpr int kWarpsPerBlock = 8;
 constexpr int kSmallTiles = 16;
 static_assert(kSmallTiles <= 16, "the small triangles' tile -> row multiply-shift is exact for at most 16 tiles");
-constexpr int kPacketTiles = 128;  // in-warp tile budget of a 32-triangle step
+constexpr int kPacketTiles = 128, kPacketTilesAlpha = 64;  // in-warp tile budget of a 32-triangle step
 constexpr int kSpreadTiles = 4;    // over budget, triangles above this many tiles are queued
 constexpr int kChunkTiles = 8;  // chunk = 8x8 tiles = 32x32 pixels
 
@@ -278,15 +279,13 @@ __device__ __forceinline__ int32_t alpha_mip(float gx, float gy, float gz, float
 }
 
 // The opaque tile shading of shade_live_tiles with the alpha test, for pixel (tx + l % 4,
-// ty + l / 4), l = lane % 16, called by all 32 lanes: each half-warp shades one tile of
-// the same triangle (valid is false on a half without a tile). The x and y differences pair
-// lanes l ^ 1 and l ^ 4 of a half.
+// ty + l / 4), l = lane % 16, called by all 32 lanes: each half-warp shades one tile
+// (valid is false on a half without one); cur is the pixel's key, read before (0: no tile). The x and y
+// differences pair lanes l ^ 1 and l ^ 4 of a half. Returns a lower bound of the pixel's depth word.
 __device__ __forceinline__ uint32_t shade_tile_pixel_alpha(const TriRec& r, const AlphaExt& x, const DevTexture& tex,
                                                            uint32_t cutoff, uint32_t tx, uint32_t ty, bool valid, int lane,
-                                                           unsigned long long* keys, uint32_t width) {
+                                                           unsigned long long* p, unsigned long long cur) {
     const uint32_t l = lane & 15;
-    unsigned long long* p = keys + (tx << 2) + ty * width + l;
-    const unsigned long long cur = valid ? *(volatile unsigned long long*)p : 0ull;
     const uint32_t px = tx + (l & 3), py = ty + (l >> 2);
     const int32_t e0 = (int32_t)((uint32_t)r.E0 + (uint32_t)r.A12 * px + (uint32_t)r.B12 * py);
     const int32_t e1 = (int32_t)((uint32_t)r.E1 + (uint32_t)r.A20 * px + (uint32_t)r.B20 * py);
@@ -300,11 +299,10 @@ __device__ __forceinline__ uint32_t shade_tile_pixel_alpha(const TriRec& r, cons
         const float su = fmul(s.u, tex.scale_lerp_u), sv = fmul(s.v, tex.scale_lerp_v);
         const float sux = __shfl_xor_sync(0xFFFFFFFFu, su, 1), svx = __shfl_xor_sync(0xFFFFFFFFu, sv, 1);
         const float suy = __shfl_xor_sync(0xFFFFFFFFu, su, 4), svy = __shfl_xor_sync(0xFFFFFFFFu, sv, 4);
-        const bool ox = l & 1, oy = l & 4;  // dFdx = p[l | 1] - p[l & ~1], dFdy = p[l | 4] - p[l & ~4]
-        const int32_t mip = alpha_mip(ox ? fsub(su, sux) : fsub(sux, su), ox ? fsub(sv, svx) : fsub(svx, sv),
-                                      oy ? fsub(su, suy) : fsub(suy, su), oy ? fsub(sv, svy) : fsub(svy, sv));
+        // dFdx = p[l | 1] - p[l & ~1], dFdy = p[l | 4] - p[l & ~4]; alpha_mip squares them, so their sign is free
+        const int32_t mip = alpha_mip(fsub(su, sux), fsub(sv, svx), fsub(su, suy), fsub(sv, svy));
         const bool nearest = (__ballot_sync(0xFFFFFFFFu, mip > 0) & (0xFFFFu << (lane & 16))) != 0;
-        if (pass) pass = sample_rgba8(tex, s.u, s.v, 0, mip, nearest) >= cutoff;
+        if (pass) pass = sample_alpha8(tex, s.u, s.v, mip, nearest) >= cutoff;
     }
     if (!pass) return (uint32_t)(cur >> 32);
     atomicMax(p, key);
@@ -316,7 +314,7 @@ __device__ __forceinline__ uint32_t shade_tile_pixel_alpha(const TriRec& r, cons
 __device__ __noinline__ void raster_serial_alpha(const TriRec& r, const AlphaExt& x, const DevMaterial* materials,
                                                  unsigned long long* keys, uint32_t width) {
     const DevMaterial& mt = materials[x.material & ~kTriAlpha];
-    const uint32_t cutoff = mt.alpha_cutoff << 24;
+    const uint32_t cutoff = mt.alpha_cutoff;
     const uint32_t minX = r.bbMin & 0xFFFF, minY = r.bbMin >> 16, maxX = r.bbMax & 0xFFFF, maxY = r.bbMax >> 16;
     for (uint32_t ty = minY; ty < maxY; ty += 4) {
         for (uint32_t tx = minX; tx < maxX; tx += 4) {
@@ -345,7 +343,7 @@ __device__ __noinline__ void raster_serial_alpha(const TriRec& r, const AlphaExt
                 nearest |= mip[l] > 0;
             }
             for (uint32_t l = 0; l < 16; l++) {
-                if (!((pass >> l) & 1) || sample_rgba8(mt.tex, tu[l], tv[l], 0, mip[l], nearest) < cutoff) continue;
+                if (!((pass >> l) & 1) || sample_alpha8(mt.tex, tu[l], tv[l], mip[l], nearest) < cutoff) continue;
                 const uint32_t px = tx + (l & 3), py = ty + (l >> 2);
                 const int32_t e1 = (int32_t)((uint32_t)r.E1 + (uint32_t)r.A20 * px + (uint32_t)r.B20 * py);
                 const int32_t e2 = (int32_t)((uint32_t)r.E2 + (uint32_t)r.A01 * px + (uint32_t)r.B01 * py);
@@ -530,29 +528,37 @@ __device__ __forceinline__ void shade_live_tiles(Rec&& rec, ReadKey&& readKey, u
     __syncwarp();
 }
 
-// shade_live_tiles for alpha-tested triangles of one material (texture tex, cutoff << 24): a
-// candidate's triangle is rec(rsel), its alpha terms ext(rsel) (the two tiles of a step may belong
-// to different triangles).
+// shade_live_tiles for alpha-tested triangles of one material (texture tex, alpha cutoff): a
+// candidate's triangle is rec(rsel), its alpha terms ext(rsel) (the tiles of a step may belong
+// to different triangles). The keys of both tiles of a half-warp are loaded first (alpha pass of a G-buffer
+// draw 431 -> 385 us).
 template <class Rec, class Ext>
 __device__ __forceinline__ void shade_live_tiles_alpha(Rec&& rec, Ext&& ext, uint32_t rsel,
                                                        const DevTexture& tex, uint32_t cutoff, unsigned mask,
                                                        uint32_t tpx, uint32_t tpy, uint32_t tmin,
                                                        unsigned long long* keys, uint32_t* tileMin, uint32_t width,
-                                                       int lane) {
-    const uint32_t half = lane >> 4, tw = width >> 2;
-    while (mask) {
-        const int s0 = __ffs(mask) - 1;
-        mask &= mask - 1;
-        const int s1 = mask ? __ffs(mask) - 1 : -1;
-        if (s1 >= 0) mask &= mask - 1;
-        const int src = half ? s1 : s0;
-        const uint32_t qx = __shfl_sync(0xFFFFFFFFu, tpx, src & 31);
-        const uint32_t qy = __shfl_sync(0xFFFFFFFFu, tpy, src & 31);
-        const uint32_t qm = __shfl_sync(0xFFFFFFFFu, tmin, src & 31);
-        const uint32_t qr = __shfl_sync(0xFFFFFFFFu, rsel, src & 31);
-        const uint32_t obs = shade_tile_pixel_alpha(rec(qr), ext(qr), tex, cutoff, qx, qy, src >= 0, lane, keys, width);
-        if (tileMin) update_tile_min(obs, tileMin, (qy >> 2) * tw + (qx >> 2), qm, src >= 0, lane);
+                                                       int lane, uint4* list) {
+    const uint32_t half = lane >> 4, l = lane & 15, m = __popc(mask);
+    if ((mask >> lane) & 1)
+        list[__popc(mask & ((1u << lane) - 1u))] = make_uint4((tpx << 2) + tpy * width, tpx | (tpy << 16), tmin, rsel);
+    __syncwarp();
+    unsigned long long* k = keys + l;
+    for (uint32_t i = half; i - half < m; i += 4) {
+        unsigned long long cur[2];
+#pragma unroll
+        for (int j = 0; j < 2; j++) cur[j] = i + 2 * j < m ? *(volatile unsigned long long*)(k + list[(i + 2 * j) & 31].x) : 0ull;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            if (i - half + 2 * j >= m) break;  // neither half has a tile
+            const uint32_t n = i + 2 * j;
+            const bool valid = n < m;
+            const uint4 e = list[valid ? n : 0];
+            const uint32_t obs = shade_tile_pixel_alpha(rec(e.w), ext(e.w), tex, cutoff, e.y & 0xFFFF, e.y >> 16, valid, lane,
+                                                        k + e.x, cur[j]);
+            if (tileMin) update_tile_min(obs, tileMin, e.x >> 4, e.z, valid, lane);
+        }
     }
+    __syncwarp();
 }
 
 // ceil(2^16 / n) for n = 1..16: t / n == (t * kDiv16[n]) >> 16 for every t < 256 (checked
@@ -602,12 +608,12 @@ __device__ __forceinline__ bool raster_region(const TriRec& r, const TileTest& t
 __device__ __forceinline__ bool raster_region_alpha(const TriRec* rp, const TileTest& tt, const AlphaExt* xp, const DevTexture& tex,
                                                     uint32_t cutoff, uint32_t x0, uint32_t y0, int tilesX, int tilesY,
                                                     unsigned long long* keys, uint32_t* tileMin, uint32_t width, int lane,
-                                                    uint32_t divMagic = 0) {
+                                                    uint4* list, uint32_t divMagic = 0) {
     return raster_region_with(*rp, tt, x0, y0, tilesX, tilesY, tileMin, width, lane,
                        [&](unsigned mask, uint32_t tpx, uint32_t tpy, uint32_t tmin) {
                            shade_live_tiles_alpha([&](uint32_t) -> const TriRec& { return *rp; },
                                                   [&](uint32_t) -> const AlphaExt& { return *xp; }, 0, tex, cutoff, mask, tpx,
-                                                  tpy, tmin, keys, tileMin, width, lane);
+                                                  tpy, tmin, keys, tileMin, width, lane, list);
                        }, divMagic);
 }
 
@@ -746,7 +752,7 @@ __device__ __forceinline__ uint32_t preload64_index4(uint32_t w) {
 // Per-warp shared memory: transformed vertices, index bytes, triangle records and the view. The alpha
 // pass also keeps each small triangle's alpha terms.
 struct WarpSmem {
-    float2 xy[64];       // projected vertices: x/w, y/w (the face test reads these alone)
+    float2 xy[64];       // projected vertices: x/w, y/w (the face test reads these alone); then 32 live tiles
     uint2 pz[64];        // snapped position (packed as TrianglePacket's) and z/w
     uint32_t idx[96];    // index bytes, mapped by preload64_index4
     Padded<TriRec> tris[32];  // the padding holds the triangle's TileTest
@@ -755,7 +761,6 @@ struct WarpSmem {
     uint8_t code[64];    // vertex_code
     uint32_t live[128];  // the meshlet's triangles that survive the face test or need clipping: mapped
                          // index bytes 0-2, then the triangle, with bit 31 set if it needs clipping
-    uint4 list[32];      // the live tiles being shaded (shade_live_tiles)
     float zmax[32];      // each small triangle's depth bound (triangle_depth_bound)
 };
 struct WarpSmemAlpha : WarpSmem {
@@ -794,6 +799,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
     Smem& S = ((Smem*)smemRaw)[warp];
     const uint8_t* idxBytes = (const uint8_t*)S.idx;
     Padded<TriRec>* tris = S.tris;
+    uint4* const list = (uint4*)S.xy;  // live tiles being shaded (shade_live_tiles): the face test is done with xy then
     const ViewParams& vp = S.view;
     const uint32_t chunk = chunk_shape(a);
     const bool multi = a.views != nullptr;
@@ -818,7 +824,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
         __syncwarp();
     }
     uint32_t nProcessed = 0, nRaster = 0, nClipped = 0;  // per warp, within 32 bits (< 2^21 meshlets x 128)
-    if (!kAlpha && blockIdx.x == 0 && threadIdx.x == 0) a.s.control[8] = 0;  // the chunk stage's cursor (runs later)
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.s.control[8] = 0;  // the cursor of the chunk stage after this pass
 
     // Work items are fetched a group at a time: one contended atomic per group. A group's cull
     // bits are tested at once (one position per lane), then the warp walks the visible ones.
@@ -838,6 +844,26 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
     // are small: a cheaper tail, and near geometry raises the tile depth bounds before the far.
     const bool twoPass = !multi && !kAlpha && !kShaded;
     uint32_t pass = twoPass ? 0u : 1u;
+    // Opaque pass of a scene with alpha-tested materials: a fetched group's alpha-tested meshlets go to the
+    // alpha pass's list with one atomic, before their records are read (a draw of alpha-tested meshlets alone:
+    // 45 -> 27 us;a shaded meshlet's FragmentShaderId is only known from its
+    // record, and is looked at later). Returns the lanes left to draw.
+    constexpr bool kSplitAlpha = kPass == kPassOpaque && !kShaded;
+    auto split_alpha = [&](unsigned mask, uint32_t meshlet, uint32_t item) -> unsigned {
+        bool alpha = false;
+        if ((mask >> lane) & 1) {
+            const uint32_t mat = *(const uint32_t*)(a.meshlets + (size_t)meshlet * kMeshletSize + kOffMaterialId);
+            if (mat != 0xFFFFFFFFu && mat < a.numMaterials)
+                alpha = a.alphaAll ? material_alpha_tested_all(a.materials[mat]) : material_alpha_tested(a.materials[mat]);
+        }
+        const unsigned am = __ballot_sync(0xFFFFFFFFu, alpha);
+        if (am == 0) return mask;
+        uint32_t at = 0;
+        if (lane == 0) at = (uint32_t)atomicAdd(&a.s.control[9], (unsigned long long)__popc(am));
+        at = __shfl_sync(0xFFFFFFFFu, at, 0);
+        if (alpha) a.s.alphaList[at + __popc(am & ((1u << lane) - 1u))] = item;
+        return mask & ~am;
+    };
     while (true) {
         uint32_t m, view = 0, item;
         if constexpr (kAlpha) {
@@ -871,6 +897,10 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                     fetchMask = (fv.groupMasks ? fv.groupMasks[g] : 0xFFFFFFFFu) & inView;
                     if (fetchMask == 0) continue;
                     laneMeshlet = q < fv.count ? draw_order(q, fv.count, fv.orderStride) : 0u;
+                    if (kSplitAlpha && a.s.alphaList) {
+                        fetchMask = split_alpha(fetchMask, fv.meshletOffset + laneMeshlet, a.viewStart[fetchView] + laneMeshlet);
+                        if (fetchMask == 0) continue;
+                    }
                 }
                 view = fetchView;
                 m = __shfl_sync(0xFFFFFFFFu, laneMeshlet, __ffs(fetchMask) - 1);
@@ -906,6 +936,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                         }
                     }
                     fetchMask = __ballot_sync(0xFFFFFFFFu, vis);
+                    if (kSplitAlpha && a.s.alphaList) fetchMask = split_alpha(fetchMask, a.meshletOffset + laneMeshlet, laneMeshlet);
                     const int got = __popc(fetchMask);
                     fetchGroup = got == 0 ? min(fetchGroup * 2, 32u) : (got > 1 ? max(fetchGroup / 2, leastGroup) : fetchGroup);
                     if (fetchMask == 0) continue;
@@ -950,7 +981,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
             if constexpr (kShaded) alphaTested = alphaTested && ((hdr >> 16) & 0xFF) == 1;
         }
         if constexpr (kShaded) cullMode = (int)((hdr >> 8) & 0xFF);
-        if (kPass == kPassOpaque && alphaTested) {  // drawn by the alpha pass
+        if (kPass == kPassOpaque && kShaded && alphaTested) {  // drawn by the alpha pass
             if (lane == 0) a.s.alphaList[atomicAdd(&a.s.control[9], 1ull)] = item;
             continue;
         }
@@ -1077,7 +1108,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
             // a second level once 90 % of the warps are idle, cost the dense frame more than they
             // gain in the sparse one.)
             bool spread = false;
-            if (__reduce_add_sync(0xFFFFFFFFu, (unsigned)myTiles) > kPacketTiles) {
+            if (__reduce_add_sync(0xFFFFFFFFu, (unsigned)myTiles) > (kAlpha ? kPacketTilesAlpha : kPacketTiles)) {
                 unsigned long long idle = 0;
                 if (lane == 0) idle = *(volatile unsigned long long*)idleWarps;
                 spread = __shfl_sync(0xFFFFFFFFu, idle, 0) * 2 >= numWarps;
@@ -1130,15 +1161,15 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                     const DevMaterial& mt = a.materials[matId];
                     shade_live_tiles_alpha([&](uint32_t q) -> const TriRec& { return tris[q].v; },
                                            [&](uint32_t q) -> const AlphaExt& { return S.exts[q].v; }, own, mt.tex,
-                                           mt.alpha_cutoff << 24, liveMask, tpx, tpy, tmin, vp.keys, vp.tileMin, vp.width,
-                                           lane);
+                                           mt.alpha_cutoff, liveMask, tpx, tpy, tmin, vp.keys, vp.tileMin, vp.width,
+                                           lane, list);
                 } else if constexpr (kOver) {
                     shade_live_tiles_overdraw([&](uint32_t q) -> const TriRec& { return tris[q].v; }, own, liveMask, tpx, tpy,
                                               vp.keys, a.counts, vp.width, lane);
                 } else {
                     shade_live_tiles([&](uint32_t q) -> const TriRec& { return tris[q].v; },
                                      [&](uint32_t q) { return (tris[q].v.pad & kPadReadKey) != 0u; }, own, liveMask, tpx, tpy,
-                                     tmin, vp.keys, vp.tileMin, vp.width, lane, S.list);
+                                     tmin, vp.keys, vp.tileMin, vp.width, lane, list);
                 }
             }
             // Triangles the full queue turned away are rasterized here by the whole warp.
@@ -1151,12 +1182,12 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                 const int tx = (int)(((r.bbMax & 0xFFFF) - x0) >> 2), ty = (int)(((r.bbMax >> 16) - y0) >> 2);
                 if constexpr (kAlpha) {
                     const DevMaterial& mt = a.materials[matId];
-                    raster_region_alpha(&tris[src].v, tile_test(r), &S.exts[src].v, mt.tex, mt.alpha_cutoff << 24, x0, y0, tx, ty, vp.keys,
-                                        vp.tileMin, vp.width, lane);
+                    raster_region_alpha(&tris[src].v, tile_test(r), &S.exts[src].v, mt.tex, mt.alpha_cutoff, x0, y0, tx, ty, vp.keys,
+                                        vp.tileMin, vp.width, lane, list);
                 } else if constexpr (kOver) {
                     raster_region_overdraw(r, tile_test(r), x0, y0, tx, ty, vp.keys, a.counts, vp.width, lane);
                 } else {
-                    raster_region(r, tile_test(r), x0, y0, tx, ty, vp.keys, vp.tileMin, vp.width, lane, a.keyReadTiles, S.list);
+                    raster_region(r, tile_test(r), x0, y0, tx, ty, vp.keys, vp.tileMin, vp.width, lane, a.keyReadTiles, list);
                 }
             }
             __syncwarp();
@@ -1187,7 +1218,9 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
 // instead of 293 M), 629 -> 466 us in an alpha-tested frame from inside the scene. Runs of 4, 16 and 32
 // chunks: 198, 184 and 193 us (the queue starts with near geometry, whose chunks survive together, so long
 // runs leave some warps with all of it; in the alpha-tested frame 385, 685 and 867 us).
-constexpr uint32_t kChunkRun = 8;
+// With alpha-tested materials runs of 4: their live chunks cost about five times more (2, 4 and 8: 405, 363 and
+// 432 us of chunk stage inside a 50k-meshlet scene).
+constexpr uint32_t kChunkRun = 8, kChunkRunAlpha = 4;
 constexpr uint32_t kRunsPerWarp = 4;  // a shorter run when the queue holds fewer chunks than this many runs a warp
 
 // Per 32x32-pixel block, a lower bound of the tile depth bounds inside it, in the words after the tile
@@ -1249,27 +1282,29 @@ __device__ __forceinline__ bool chunk_live(const TriRec& r, uint32_t x0, uint32_
     return ((uint32_t)max(__float_as_int(bound), 0) | 0x80000000u) >= known;
 }
 
-// A chunk of the alpha-tested triangle whose record (and AlphaExt after it) is at q, kept out of
-// line so that the opaque chunks keep the kernel's registers.
-__device__ __noinline__ bool raster_chunk_alpha(const TriRec* q, const DevMaterial* materials, uint32_t x0, uint32_t y0,
+// A chunk of the alpha-tested triangle whose record (and AlphaExt after it) is at q.
+__device__ __forceinline__ bool raster_chunk_alpha(const TriRec* q, const DevMaterial* materials, uint32_t x0, uint32_t y0,
                                                 int tilesX, int tilesY, unsigned long long* keys, uint32_t* tileMin,
-                                                uint32_t width, int lane) {
+                                                uint32_t width, int lane, uint4* list) {
     const AlphaExt* xp = (const AlphaExt*)&q[1];
     const DevMaterial& mt = materials[xp->material & ~kTriAlpha];
-    return raster_region_alpha(q, tile_test(*q), xp, mt.tex, mt.alpha_cutoff << 24, x0, y0, tilesX, tilesY, keys, tileMin, width,
-                               lane, kDiv16[tilesX]);
+    return raster_region_alpha(q, tile_test(*q), xp, mt.tex, mt.alpha_cutoff, x0, y0, tilesX, tilesY, keys, tileMin, width,
+                               lane, list, kDiv16[tilesX]);
 }
 
-template <bool kOver>
-__global__ void __launch_bounds__(256, 5) k_raster_big(const TriRec* __restrict__ big, const unsigned long long* __restrict__ bigBase,
+// kAlpha: the scene has alpha-tested materials (a build of its own with more registers, so that neither keeps
+// the other's; 48 and 64 registers hold 40 and 32 warps per SM: chunk stages of the alpha-tested frame 459 ->
+// 404 us).
+template <bool kOver, bool kAlpha>
+__global__ void __launch_bounds__(256, kAlpha ? 4 : 5) k_raster_big(const TriRec* __restrict__ big, const unsigned long long* __restrict__ bigBase,
                                                     unsigned long long* control, uint32_t capacity,
                                                     unsigned long long* keys, uint32_t* tileMin, uint32_t width, uint32_t height,
                                                     const ViewParams* __restrict__ views, uint32_t chunk,
                                                     const DevMaterial* __restrict__ materials, unsigned long long* counts,
-                                                    uint32_t readTiles) {
+                                                    uint32_t readTiles, uint32_t maxRun, bool lastStage) {
     __shared__ uint4 list[8][32];  // per warp: the live tiles being shaded
     const unsigned long long q = control[1];
-    if (blockIdx.x == 0 && threadIdx.x == 0)  // the next draw's second cursor, alpha list and idle-warp counts
+    if (lastStage && blockIdx.x == 0 && threadIdx.x == 0)  // the next draw's second cursor, alpha list and idle-warp counts
         control[7] = control[9] = control[10] = control[11] = control[12] = 0;
     const uint32_t n = (uint32_t)min((unsigned long long)capacity, q >> 40);
     if (n == 0) return;
@@ -1281,7 +1316,7 @@ __global__ void __launch_bounds__(256, 5) k_raster_big(const TriRec* __restrict_
     const unsigned long long total = bigBase[n - 1] + (unsigned long long)((lastTX + cw - 1) / cw) * ((lastTY + ch - 1) / ch);
     // a sparse queue (few big triangles) is spread with shorter runs so that every warp gets work
     const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-    const uint32_t run = (uint32_t)max(1ull, min((unsigned long long)kChunkRun, total / (warps * kRunsPerWarp)));
+    const uint32_t run = (uint32_t)max(1ull, min((unsigned long long)maxRun, total / (warps * kRunsPerWarp)));
     while (true) {
         unsigned long long w0 = 0;
         if (lane == 0) w0 = atomicAdd(&control[8], (unsigned long long)run);
@@ -1340,8 +1375,9 @@ __global__ void __launch_bounds__(256, 5) k_raster_big(const TriRec* __restrict_
                 raster_region_overdraw(r, tile_test(r), x0, y0, tilesX, tilesY, vkeys, counts, vw, lane, kDiv16[tilesX]);
             } else {
                 bool any;
-                if (r.pad & kTriAlpha)
-                    any = raster_chunk_alpha(big + s, materials, x0, y0, tilesX, tilesY, vkeys, vtiles, vw, lane);
+                if (kAlpha && (r.pad & kTriAlpha))
+                    any = raster_chunk_alpha(big + s, materials, x0, y0, tilesX, tilesY, vkeys, vtiles, vw, lane,
+                                             list[threadIdx.x >> 5]);
                 else
                     any = raster_region(r, tile_test(r), x0, y0, tilesX, tilesY, vkeys, vtiles, vw, lane, readTiles, list[threadIdx.x >> 5], kDiv16[tilesX]);
                 if (!any && vtiles) refresh_blocks(x0, y0, x1, y1, vtiles, vw, vh, lane);
@@ -1481,10 +1517,30 @@ void launch_draw(const DrawArgs& args, cudaStream_t st, int numSMs) {
             k_draw_meshlets<kPassOverdraw><<<grid, warps * 32, smem, st>>>(a);
         }
         LaunchScope ls("k_raster_big_overdraw", st);
-        k_raster_big<true><<<numSMs * 8, 256, 0, st>>>(a.s.big, a.s.bigBase, a.s.control, a.s.bigCapacity, a.keys, nullptr,
-                                                       a.width, a.height, a.views, chunk, a.materials, a.counts, 0u);
+        k_raster_big<true, false><<<numSMs * 8, 256, 0, st>>>(a.s.big, a.s.bigBase, a.s.control, a.s.bigCapacity, a.keys, nullptr,
+                                                       a.width, a.height, a.views, chunk, a.materials, a.counts, 0u, kChunkRun,
+                                                              true);
         return;
     }
+    auto chunks = [&](bool last) {
+        LaunchScope ls("k_raster_big", st);
+        if (a.s.alphaList && last)
+            k_raster_big<false, true><<<numSMs * 4, 256, 0, st>>>(a.s.big, a.s.bigBase, a.s.control, a.s.bigCapacity, a.keys,
+                                                                  a.tileMin, a.width, a.height, a.views, chunk, a.materials,
+                                                                  nullptr, a.keyReadTiles, kChunkRunAlpha, true);
+        else
+            k_raster_big<false, false><<<numSMs * 8, 256, 0, st>>>(a.s.big, a.s.bigBase, a.s.control, a.s.bigCapacity, a.keys,
+                                                                   a.tileMin, a.width, a.height, a.views, chunk, a.materials,
+                                                                   nullptr, a.keyReadTiles, kChunkRun, last);
+    };
+    // Before the alpha pass, which then meets the depth bounds of the opaque pass's large triangles (inside a
+    // 50k-meshlet scene, half of the materials alpha-tested: alpha pass 239 -> 109 us, chunk stages 383 -> 429 us).
+    auto opaque_chunks = [&] {
+        chunks(false);
+        cudaMemsetAsync(&a.s.control[1], 0, sizeof(unsigned long long), st);  // an empty queue
+    };
+    // The alpha pass's grid: as many blocks as its larger shared memory lets an SM hold.
+    const int gridAlpha = numSMs * (int)std::max<size_t>(1, std::min<size_t>(32 / warps, 227 * 1024 / (smemAlpha + 1024)));
     if (a.shaded) {  // meshlets shaded by a user mesh shader
         if (smem > 48 * 1024) raise_smem_limit(3, (const void*)k_draw_meshlets<kPassOpaque, true>, smem);
         if (a.s.alphaList && smemAlpha > 48 * 1024) raise_smem_limit(4, (const void*)k_draw_meshlets<kPassAlpha, true>, smemAlpha);
@@ -1493,8 +1549,9 @@ void launch_draw(const DrawArgs& args, cudaStream_t st, int numSMs) {
             k_draw_meshlets<kPassOpaque, true><<<grid, warps * 32, smem, st>>>(a);
         }
         if (a.s.alphaList) {
+            opaque_chunks();
             LaunchScope ls("k_draw_meshlets_shaded_alpha", st);
-            k_draw_meshlets<kPassAlpha, true><<<grid, warps * 32, smemAlpha, st>>>(a);
+            k_draw_meshlets<kPassAlpha, true><<<gridAlpha, warps * 32, smemAlpha, st>>>(a);
         }
     } else {
         {
@@ -1502,16 +1559,12 @@ void launch_draw(const DrawArgs& args, cudaStream_t st, int numSMs) {
             k_draw_meshlets<kPassOpaque><<<grid, warps * 32, smem, st>>>(a);
         }
         if (a.s.alphaList) {  // the scene has alpha-tested materials
+            opaque_chunks();
             LaunchScope ls("k_draw_meshlets_alpha", st);
-            k_draw_meshlets<kPassAlpha><<<grid, warps * 32, smemAlpha, st>>>(a);
+            k_draw_meshlets<kPassAlpha><<<gridAlpha, warps * 32, smemAlpha, st>>>(a);
         }
     }
-    {
-        LaunchScope ls("k_raster_big", st);
-        k_raster_big<false><<<numSMs * 8, 256, 0, st>>>(a.s.big, a.s.bigBase, a.s.control, a.s.bigCapacity, a.keys,
-                                                        a.tileMin, a.width, a.height, a.views, chunk, a.materials, nullptr,
-                                                        a.keyReadTiles);
-    }
+    chunks(true);
 }
 
 void launch_init_keys(const uint32_t* depthLayer, unsigned long long* keys, uint32_t* tileMin, uint32_t width, uint32_t height,

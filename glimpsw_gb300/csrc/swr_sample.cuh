@@ -77,6 +77,19 @@ __device__ __forceinline__ uint32_t sample_quad(const DevTexture& t, const Texel
     return filter_rgba8(base[i00], base[i00 + 8], base[i01], base[i01 + 8], q.fx, q.fy);
 }
 
+// The alpha of layer 0's SampleLevel<SurfaceSampler>: what `texel >= cutoff << 24` decides (the lower bytes can
+// only raise the word).
+__device__ __forceinline__ uint32_t sample_alpha8(const DevTexture& t, float u, float v, int32_t mipIn, bool nearest) {
+    const TexelQuad q = texel_quad(t, u, v, mipIn, nearest);
+    const uint32_t* base = t.data + t.mip_offsets[q.m & 15];
+    if (nearest) return base[texel_offset(q.tx, q.ty, q.stride)] >> 24;
+    const uint32_t i00 = texel_offset(q.tx, q.ty, q.stride), i01 = texel_offset(q.tx, q.ty + (q.inY ? 1 : 0), q.stride);
+    const uint32_t a00 = base[i00] >> 24, a10 = base[i00 + 8] >> 24, a01 = base[i01] >> 24, a11 = base[i01 + 8] >> 24;
+    const uint32_t wx = (q.fx >> 7) & 255u, wy = (q.fy >> 7) & 255u;
+    const uint32_t top = (a00 * (256u - wx) + a10 * wx + 128u) >> 8, bot = (a01 * (256u - wx) + a11 * wx + 128u) >> 8;
+    return (top * (256u - wy) + bot * wy + 128u) >> 8;
+}
+
 // SampleLevel<SurfaceSampler> for one lane once the tile's filter is known (Texture.h:412-459).
 __device__ __forceinline__ uint32_t sample_rgba8(const DevTexture& t, float u, float v, int layer, int32_t mipIn, bool nearest) {
     return sample_quad(t, texel_quad(t, u, v, mipIn, nearest), layer, nearest);
