@@ -854,7 +854,8 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
         if ((mask >> lane) & 1) {
             const uint32_t mat = *(const uint32_t*)(a.meshlets + (size_t)meshlet * kMeshletSize + kOffMaterialId);
             if (mat != 0xFFFFFFFFu && mat < a.numMaterials)
-                alpha = a.alphaAll ? material_alpha_tested_all(a.materials[mat]) : material_alpha_tested(a.materials[mat]);
+                alpha = (a.alphaAll ? material_alpha_tested_all(a.materials[mat]) : material_alpha_tested(a.materials[mat])) &&
+                        !material_alpha_passes(a.materials[mat]);
         }
         const unsigned am = __ballot_sync(0xFFFFFFFFu, alpha);
         if (am == 0) return mask;

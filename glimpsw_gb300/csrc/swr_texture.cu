@@ -44,20 +44,47 @@ __device__ __forceinline__ uint32_t pack_f10(float x) {
     return ((__float_as_uint(x) >> 18) & 0x1FFF) - 0x0E00;
 }
 
-// SetPixels for TiledY8 (Texture.h:336-354): row-major source to tiled storage.
-__global__ void k_set_pixels(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t width,
-                             uint32_t height, uint32_t rowShift) {
+// Lowers *alphaMin to the least of the block's values (all threads call it).
+__device__ __forceinline__ void block_alpha_min(uint32_t least, uint32_t* alphaMin) {
+    __shared__ uint32_t s;
+    if (threadIdx.x == 0) s = 255u;
+    __syncthreads();
+    least = __reduce_min_sync(0xFFFFFFFFu, least);
+    if ((threadIdx.x & 31) == 0) atomicMin(&s, least);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicMin(alphaMin, s);
+}
+
+// SetPixels for TiledY8 (Texture.h:336-354): row-major source to tiled storage. alphaMin: the level's least
+// alpha word (nullptr: not kept).
+__global__ void __launch_bounds__(256) k_set_pixels(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t width,
+                                                    uint32_t height, uint32_t rowShift, uint32_t* alphaMin) {
     const uint32_t n = width * height;
+    uint32_t least = 255u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t y = i / width, x = i - y * width;
-        dst[texel_offset(x, y, rowShift)] = src[i];
+        const uint32_t v = src[i];
+        dst[texel_offset(x, y, rowShift)] = v;
+        least = min(least, v >> 24);
     }
+    if (alphaMin) block_alpha_min(least, alphaMin);
+}
+
+// The least alpha of one level of a texture's storage.
+__global__ void __launch_bounds__(256) k_alpha_min(const uint32_t* __restrict__ level, uint32_t w, uint32_t h, uint32_t stride,
+                                                   uint32_t* alphaMin) {
+    uint32_t least = 255u;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < w * h; i += gridDim.x * blockDim.x)
+        least = min(least, level[texel_offset(i % w, i / w, stride)] >> 24);
+    block_alpha_min(least, alphaMin);
 }
 
 // GenerateMip (Texture.h:577-596): 2x2 box filter on unpacked texels, ((c00 + c10) + c01 + c11) * 0.25.
-__global__ void k_generate_mip(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t w, uint32_t h,
-                               uint32_t sstride, uint32_t dstride, uint32_t format) {
+__global__ void __launch_bounds__(256) k_generate_mip(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t w,
+                                                      uint32_t h, uint32_t sstride, uint32_t dstride, uint32_t format,
+                                                      uint32_t* alphaMin) {
     const uint32_t n = w * h;
+    uint32_t least = 255u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t y = i / w, x = i - y * w;
         uint32_t p00 = src[texel_offset(2 * x, 2 * y, sstride)], p10 = src[texel_offset(2 * x + 1, 2 * y, sstride)];
@@ -86,7 +113,14 @@ __global__ void k_generate_mip(const uint32_t* __restrict__ src, uint32_t* __res
                                             __uint_as_float(p11)), 0.25f));
         }
         dst[texel_offset(x, y, dstride)] = out;
+        least = min(least, out >> 24);
     }
+    if (alphaMin) block_alpha_min(least, alphaMin);
+}
+
+// Restarts the least-alpha words of levels [first, end) before they are written again.
+static cudaError_t restart_alpha_min(swr_texture t, uint32_t first, uint32_t end, cudaStream_t st) {
+    return cudaMemsetAsync((uint32_t*)t->d.alpha_min + first, 0xFF, (end - first) * sizeof(uint32_t), st);
 }
 
 static int grid_for(uint32_t n) { return (int)std::max(1u, std::min((n + 255) / 256, 152u * 16)); }
@@ -129,15 +163,24 @@ swr_status swr_texture_create(uint32_t format, uint32_t width, uint32_t height, 
     d.scale_lerp_u = (float)(d.mask_lerp_u + 1), d.scale_lerp_v = (float)(d.mask_lerp_v + 1);
     t->format = format;
     t->words = (size_t)stride * num_layers + 64;
+    // The least-alpha words follow the storage. A level 4 texels high and more than 8 wide spreads its texels
+    // past its storage (TiledY8 columns hold 8 rows): what its words hold is not kept.
+    bool shared = false;
+    for (uint32_t l = 0; l < mip; l++) shared = shared || ((height >> l) < 8 && (width >> l) > 8);
+    const bool keep = format == SWR_FORMAT_RGBA8U && !shared;
     uint32_t* p = nullptr;
-    cudaError_t e = cudaMalloc(&p, t->words * 4);
+    const size_t alphaAt = (t->words + 3) & ~(size_t)3;
+    cudaError_t e = cudaMalloc(&p, (alphaAt + 16) * 4);
     if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, t->words * 4, swr_internal_stream());
+    if (e == cudaSuccess) e = cudaMemsetAsync(p + alphaAt, 0, mip * 4, swr_internal_stream());  // texels start as 0
+    if (e == cudaSuccess && mip < 16) e = cudaMemsetAsync(p + alphaAt + mip, 0xFF, (16 - mip) * 4, swr_internal_stream());
     if (e != cudaSuccess) {
         cudaFree(p);
         delete t;
         return swr_internal_cuda_fail(e, "swr_texture_create");
     }
     d.data = p;
+    d.alpha_min = keep ? p + alphaAt : nullptr;
     *out = t;
     return SWR_OK;
 }
@@ -159,10 +202,12 @@ swr_status swr_texture_set_pixels(swr_texture t, const uint32_t* pixels, uint32_
     if (e == cudaSuccess)
         e = cudaMemcpy2DAsync(tmp, (size_t)t->d.width * 4, pixels, (size_t)stride * 4, (size_t)t->d.width * 4, t->d.height,
                               cudaMemcpyHostToDevice, st);
+    uint32_t* alphaMin = layer == 0 ? (uint32_t*)t->d.alpha_min : nullptr;
+    if (e == cudaSuccess && alphaMin) e = restart_alpha_min(t, 0, 1, st);
     if (e == cudaSuccess) {
         LaunchScope ls("k_set_pixels", st);
         k_set_pixels<<<grid_for(t->d.width * t->d.height), 256, 0, st>>>(
-            tmp, (uint32_t*)t->d.data + (size_t)layer * t->d.layer_stride, t->d.width, t->d.height, t->d.row_shift);
+            tmp, (uint32_t*)t->d.data + (size_t)layer * t->d.layer_stride, t->d.width, t->d.height, t->d.row_shift, alphaMin);
         e = cudaGetLastError();
     }
     if (tmp) cudaFreeAsync(tmp, st);
@@ -175,10 +220,15 @@ swr_status swr_texture_set_pixels_device(swr_texture t, const uint32_t* pixels_d
     if (!t || !pixels_device || layer >= t->d.num_layers || stride != t->d.width)
         return swr_internal_fail(SWR_EINVAL, "swr_texture_set_pixels_device: bad argument (stride must equal the width)");
     cudaStream_t st = swr_internal_stream();
-    LaunchScope ls("k_set_pixels", st);
-    k_set_pixels<<<grid_for(t->d.width * t->d.height), 256, 0, st>>>(
-        pixels_device, (uint32_t*)t->d.data + (size_t)layer * t->d.layer_stride, t->d.width, t->d.height, t->d.row_shift);
-    cudaError_t e = cudaGetLastError();
+    uint32_t* alphaMin = layer == 0 ? (uint32_t*)t->d.alpha_min : nullptr;
+    cudaError_t e = alphaMin ? restart_alpha_min(t, 0, 1, st) : cudaSuccess;
+    if (e == cudaSuccess) {
+        LaunchScope ls("k_set_pixels", st);
+        k_set_pixels<<<grid_for(t->d.width * t->d.height), 256, 0, st>>>(
+            pixels_device, (uint32_t*)t->d.data + (size_t)layer * t->d.layer_stride, t->d.width, t->d.height, t->d.row_shift,
+            alphaMin);
+        e = cudaGetLastError();
+    }
     if (e != cudaSuccess) return swr_internal_cuda_fail(e, "swr_texture_set_pixels_device");
     return SWR_OK;
 }
@@ -187,13 +237,18 @@ swr_status swr_texture_generate_mips(swr_texture t) {
     if (!t) return swr_internal_fail(SWR_EINVAL, "swr_texture_generate_mips: NULL texture");
     cudaStream_t st = swr_internal_stream();
     const DevTexture& d = t->d;
+    if (d.alpha_min && d.mip_levels > 1) {
+        const cudaError_t er = restart_alpha_min(t, 1, d.mip_levels, st);
+        if (er != cudaSuccess) return swr_internal_cuda_fail(er, "swr_texture_generate_mips");
+    }
     for (uint32_t layer = 0; layer < d.num_layers; layer++) {
         for (uint32_t level = 1; level < d.mip_levels; level++) {
             uint32_t w = d.width >> level, h = d.height >> level;
             uint32_t* base = (uint32_t*)d.data + (size_t)layer * d.layer_stride;
             LaunchScope ls("k_generate_mip", st);
             k_generate_mip<<<grid_for(w * h), 256, 0, st>>>(base + d.mip_offsets[level - 1], base + d.mip_offsets[level], w, h,
-                                                           d.row_shift - level + 1, d.row_shift - level, t->format);
+                                                           d.row_shift - level + 1, d.row_shift - level, t->format,
+                                                           layer == 0 && d.alpha_min ? (uint32_t*)d.alpha_min + level : nullptr);
         }
     }
     cudaError_t e = cudaGetLastError();
@@ -222,6 +277,16 @@ swr_status swr_texture_set_data(swr_texture t, const uint32_t* src, size_t words
     if (!t || !src || words > t->words) return swr_internal_fail(SWR_EINVAL, "swr_texture_set_data: bad argument");
     cudaStream_t st = swr_internal_stream();
     cudaError_t e = cudaMemcpyAsync((void*)t->d.data, src, words * 4, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && t->d.alpha_min) {
+        e = restart_alpha_min(t, 0, t->d.mip_levels, st);
+        for (uint32_t l = 0; l < t->d.mip_levels && e == cudaSuccess; l++) {
+            const uint32_t w = t->d.width >> l, h = t->d.height >> l;
+            LaunchScope ls("k_alpha_min", st);
+            k_alpha_min<<<grid_for(w * h), 256, 0, st>>>(t->d.data + t->d.mip_offsets[l], w, h, t->d.row_shift - l,
+                                                         (uint32_t*)t->d.alpha_min + l);
+            e = cudaGetLastError();
+        }
+    }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return swr_internal_cuda_fail(e, "swr_texture_set_data");
     return SWR_OK;
