@@ -283,10 +283,13 @@ struct swr_scene_t {
     uint64_t version;              // bumped when meshlets or materials move (recorded draw graphs re-capture)
 };
 
+constexpr uint32_t kSkyScratchTexels = 512 * 512;
 struct swr_texture_t {
     uint32_t format;
     swr::DevTexture d;             // d.data is the device storage
     size_t words;
+    void* skyScratch;              // R11G11B10: room for its level 2 (or last) unpacked, 8 bytes a texel, at most
+                                   // kSkyScratchTexels texels (nullptr: larger, or another format)
 };
 
 struct swr_rasterizer_t {
