@@ -429,7 +429,8 @@ __device__ __forceinline__ bool enqueue_warp(bool want, const TriRec& rec, const
 }
 
 // A small triangle's record (the mesh stage's tile walk): pad = tilesX | row_magic << 8 | kPadReadKey.
-constexpr uint32_t kPadReadKey = 1u << 24;
+// A triangle of more tiles has kPadWide instead of the first two.
+constexpr uint32_t kPadReadKey = 1u << 24, kPadWide = 1u << 25;
 // The 4x4 tiles of a triangle's render box.
 __device__ __forceinline__ uint32_t triangle_tiles(const TriRec& r) {
     return (((r.bbMax & 0xFFFF) - (r.bbMin & 0xFFFF)) >> 2) * (((r.bbMax >> 16) - (r.bbMin >> 16)) >> 2);
@@ -768,6 +769,15 @@ struct WarpSmemAlpha : WarpSmem {
     Padded<AlphaExt> exts[32];
 };
 
+// True if a meshlet of material mat goes to the alpha pass. Out of line: it is run once per 32 positions of
+// scenes with alpha-tested materials, and inline it moved the mesh stage's loop across the instruction
+// cache's reach (24 batched views without such materials: 1281 -> 1492 us).
+__device__ __noinline__ bool takes_alpha_pass(const DevMaterial* materials, uint32_t numMaterials, uint32_t mat, bool all) {
+    if (mat == 0xFFFFFFFFu || mat >= numMaterials) return false;
+    const DevMaterial& m = materials[mat];
+    return (all ? material_alpha_tested_all(m) : material_alpha_tested(m)) && !material_alpha_passes(m);
+}
+
 // Mesh stage. A work item is one meshlet of one view: a single-view draw numbers its meshlets
 // 0..count-1; a batched draw concatenates the meshlet ranges of its views (viewStart is their
 // prefix), so one launch serves views of any size.
@@ -853,9 +863,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
         bool alpha = false;
         if ((mask >> lane) & 1) {
             const uint32_t mat = *(const uint32_t*)(a.meshlets + (size_t)meshlet * kMeshletSize + kOffMaterialId);
-            if (mat != 0xFFFFFFFFu && mat < a.numMaterials)
-                alpha = (a.alphaAll ? material_alpha_tested_all(a.materials[mat]) : material_alpha_tested(a.materials[mat])) &&
-                        !material_alpha_passes(a.materials[mat]);
+            alpha = takes_alpha_pass(a.materials, a.numMaterials, mat, a.alphaAll != 0);
         }
         const unsigned am = __ballot_sync(0xFFFFFFFFu, alpha);
         if (am == 0) return mask;
@@ -1121,7 +1129,15 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
             }
             const AlphaExt* ext = nullptr;
             if constexpr (kAlpha) ext = &S.exts[lane].v;
-            const bool overflow = !enqueue_warp<kAlpha>(queue, tris[lane].v, ext, a, chunk, lane);
+            if (!enqueue_warp<kAlpha>(queue, tris[lane].v, ext, a, chunk, lane)) {
+                // The full queue turned it away: its tiles join the warp's list, however many they are. (A second
+                // copy of the tile loop for it cost the loop's place in the instruction cache.)
+                TriRec& r = tris[lane].v;
+                myTiles = (int)triangle_tiles(r);
+                r.pad = kPadWide | kPadReadKey;
+                *(TileTest*)&tris[lane].pad = tile_test(r);
+                S.zmax[lane] = __int_as_float(0x7F800000);
+            }
 
             // Small triangles: the warp walks the concatenated tile lists of all of them, two
             // tiles (32 pixels) per step, so tiny triangles share steps.
@@ -1152,8 +1168,12 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                 if (t < total) {
                     const TriRec& r = tris[own].v;
                     const int tile = t - ownerExcl;
-                    const int tilesX = r.pad & 0xFF, magic = (r.pad >> 8) & 0x1FF;
-                    const int ty = (tile * magic) >> 8, tx = tile - ty * tilesX;
+                    int tilesX = r.pad & 0xFF, ty = (tile * (int)((r.pad >> 8) & 0x1FF)) >> 8;
+                    if (r.pad & kPadWide) {
+                        tilesX = (int)(((r.bbMax & 0xFFFF) - (r.bbMin & 0xFFFF)) >> 2);
+                        ty = tile / tilesX;
+                    }
+                    const int tx = tile - ty * tilesX;
                     tpx = (r.bbMin & 0xFFFF) + tx * 4, tpy = (r.bbMin >> 16) + ty * 4;
                     live = tile_live(r, *(const TileTest*)&tris[own].pad, tpx, tpy, vp.tileMin, tw, &tmin, S.zmax[own]);
                 }
@@ -1171,24 +1191,6 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                     shade_live_tiles([&](uint32_t q) -> const TriRec& { return tris[q].v; },
                                      [&](uint32_t q) { return (tris[q].v.pad & kPadReadKey) != 0u; }, own, liveMask, tpx, tpy,
                                      tmin, vp.keys, vp.tileMin, vp.width, lane, list);
-                }
-            }
-            // Triangles the full queue turned away are rasterized here by the whole warp.
-            unsigned ovMask = __ballot_sync(0xFFFFFFFFu, overflow);
-            while (ovMask) {
-                const int src = __ffs(ovMask) - 1;
-                ovMask &= ovMask - 1;
-                const TriRec r = tris[src].v;
-                const uint32_t x0 = r.bbMin & 0xFFFF, y0 = r.bbMin >> 16;
-                const int tx = (int)(((r.bbMax & 0xFFFF) - x0) >> 2), ty = (int)(((r.bbMax >> 16) - y0) >> 2);
-                if constexpr (kAlpha) {
-                    const DevMaterial& mt = a.materials[matId];
-                    raster_region_alpha(&tris[src].v, tile_test(r), &S.exts[src].v, mt.tex, mt.alpha_cutoff, x0, y0, tx, ty, vp.keys,
-                                        vp.tileMin, vp.width, lane, list);
-                } else if constexpr (kOver) {
-                    raster_region_overdraw(r, tile_test(r), x0, y0, tx, ty, vp.keys, a.counts, vp.width, lane);
-                } else {
-                    raster_region(r, tile_test(r), x0, y0, tx, ty, vp.keys, vp.tileMin, vp.width, lane, a.keyReadTiles, list);
                 }
             }
             __syncwarp();
@@ -1264,9 +1266,12 @@ __device__ __forceinline__ bool chunk_live(const TriRec& r, uint32_t x0, uint32_
     if (!tileMin) return true;
     const uint32_t bw = (width + 31) >> 5;
     const uint32_t* blockMin = tileMin + (width >> 2) * (height >> 2);
-    uint32_t known = 0xFFFFFFFFu;
-    for (uint32_t by = y0 >> 5; by <= (y1 - 1) >> 5; by++)
-        for (uint32_t bx = x0 >> 5; bx <= (x1 - 1) >> 5; bx++) known = min(known, blockMin[by * bw + bx]);
+    // a chunk of at most 32 pixels a side touches at most 2 x 2 blocks, one of 64 at most 3 x 3
+    const uint32_t bx0 = x0 >> 5, by0 = y0 >> 5, bx1 = (x1 - 1) >> 5, by1 = (y1 - 1) >> 5;
+    uint32_t known = min(min(blockMin[by0 * bw + bx0], blockMin[by0 * bw + bx1]), min(blockMin[by1 * bw + bx0], blockMin[by1 * bw + bx1]));
+    if (bx1 - bx0 > 1 || by1 - by0 > 1)
+        for (uint32_t by = by0; by <= by1; by++)
+            for (uint32_t bx = bx0; bx <= bx1; bx++) known = min(known, blockMin[by * bw + bx]);
     const float u = __int2float_rn((int32_t)e1), v = __int2float_rn((int32_t)e2);
     const float a20 = (float)r.A20, b20 = (float)r.B20, a01 = (float)r.A01, b01 = (float)r.B01;
     const float W = (float)(w + 2), H = (float)(h + 2);
@@ -1313,7 +1318,7 @@ __global__ void __launch_bounds__(256, kAlpha ? 4 : 5) k_raster_big(const TriRec
     const TriRec& last = big[n - 1];
     const int lastTX = (int)(((last.bbMax & 0xFFFF) - (last.bbMin & 0xFFFF)) >> 2);
     const int lastTY = (int)(((last.bbMax >> 16) - (last.bbMin >> 16)) >> 2);
-    const uint32_t cw = chunk & 0xFF, ch = chunk >> 8;
+    const uint32_t cw = chunk & 0xFF, ch = chunk >> 8, cwShift = 31 - __clz(cw);  // powers of two
     const unsigned long long total = bigBase[n - 1] + (unsigned long long)((lastTX + cw - 1) / cw) * ((lastTY + ch - 1) / ch);
     // a sparse queue (few big triangles) is spread with shorter runs so that every warp gets work
     const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
@@ -1331,20 +1336,32 @@ __global__ void __launch_bounds__(256, kAlpha ? 4 : 5) k_raster_big(const TriRec
             slot += below * step;
             hi = min(hi, slot + step - 1);
         }
-        // the lane's chunk: its triangle is at most 64 slots on (32 chunks, each of another triangle and its AlphaExt)
         const unsigned long long w = w0 + lane;
         bool live = lane < run && w < total;
-        uint32_t xy0 = 0, xy1 = 0;
-        if (live) {
+        uint32_t xy0 = 0, xy1 = 0, k = (uint32_t)(w - bigBase[slot]);  // the lane's chunk of its triangle
+        if constexpr (!kAlpha) {
+            // Every slot owns chunks: the triangles that start within the run set a bit each, and a lane's
+            // triangle is as many slots on as bits are set up to it.
+            const uint32_t next = slot + 1 + lane;
+            const unsigned long long start = next < n ? bigBase[next] - w0 : 32ull;
+            const unsigned starts = __reduce_or_sync(0xFFFFFFFFu, start < 32 ? 1u << start : 0u) & (0xFFFFFFFFu >> (31 - lane));
+            slot += __popc(starts);
+            if (starts) k = lane - (31 - __clz(starts));
+        } else if (live) {  // at most 64 slots on (32 chunks, each of another triangle and its AlphaExt)
             uint32_t end = min(n - 1, slot + 2 * (uint32_t)lane);
             while (slot < end) {
                 const uint32_t mid = (slot + end + 1) >> 1;
                 if (bigBase[mid] <= w) slot = mid; else end = mid - 1;
             }
+            k = (uint32_t)(w - bigBase[slot]);
+        }
+        if (live) {
             const TriRec r = big[slot];
             const uint32_t minX = r.bbMin & 0xFFFF, minY = r.bbMin >> 16, maxX = r.bbMax & 0xFFFF, maxY = r.bbMax >> 16;
-            const uint32_t k = (uint32_t)(w - bigBase[slot]), chunksX = (((maxX - minX) >> 2) + cw - 1) / cw;
-            const uint32_t cy = k / chunksX, cx = k - cy * chunksX;
+            // k / chunksX by a reciprocal: (k + 1/2) / chunksX is at least 1 / 724 from an integer (chunksX <= 362,
+            // k < 2^17), the rounding errors below 2^-12
+            const uint32_t chunksX = (((maxX - minX) >> 2) + cw - 1) >> cwShift;
+            const uint32_t cy = (uint32_t)__fdividef((float)k + 0.5f, (float)chunksX), cx = k - cy * chunksX;
             const uint32_t x0 = minX + cx * (cw * 4), y0 = minY + cy * (ch * 4);
             const uint32_t x1 = min(x0 + cw * 4, maxX), y1 = min(y0 + ch * 4, maxY);
             const uint32_t* vtiles = tileMin;
