@@ -778,6 +778,35 @@ __device__ __noinline__ bool takes_alpha_pass(const DevMaterial* materials, uint
     return (all ? material_alpha_tested_all(m) : material_alpha_tested(m)) && !material_alpha_passes(m);
 }
 
+// True if no triangle of a meshlet can change a pixel: its vertices (slots below `slots` of pz, all of them inside
+// the view) lie in a box of tiles whose depth bounds are all above the nearest vertex (triangle_depth_bound of
+// the meshlet). The alpha pass finds 41 to 46 % of its meshlets hidden by the opaque pass and by each other: 94 ->
+// 77 us of a 1916x1036 frame from inside, 175 -> 144 us of a 1600x900 G-buffer.
+constexpr uint32_t kHiddenTiles = 512;  // larger boxes are not tested (16 loads a lane)
+__device__ __forceinline__ bool meshlet_hidden(const uint2* pz, uint32_t slots, const ViewParams& vp, int lane) {
+    uint32_t lo = 0x7FFF7FFFu, hi = 0x80008000u, z = 0;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        if (32 * j + lane < slots) {
+            const uint2 q = pz[32 * j + lane];
+            lo = __vmins2(lo, q.x), hi = __vmaxs2(hi, q.x), z = max(z, q.y);
+        }
+    }
+    z = __reduce_max_sync(0xFFFFFFFFu, z);
+    const int32_t x0 = __reduce_min_sync(0xFFFFFFFFu, (int32_t)(int16_t)(lo & 0xFFFF)), y0 = __reduce_min_sync(0xFFFFFFFFu, (int32_t)lo >> 16);
+    const int32_t x1 = __reduce_max_sync(0xFFFFFFFFu, (int32_t)(int16_t)(hi & 0xFFFF)), y1 = __reduce_max_sync(0xFFFFFFFFu, (int32_t)hi >> 16);
+    // render_bbox of the whole; a triangle's 32-bit add may carry 1 into y, which the 8 covers
+    const int32_t tx0 = max(((x0 + 7) >> 4) + vp.halfW, 0) >> 2, ty0 = max(((y0 + 7) >> 4) + vp.halfH, 0) >> 2;
+    const int32_t tx1 = (min(((x1 + 7) >> 4) + vp.halfW, 2 * vp.halfW) + 3) >> 2, ty1 = (min(((y1 + 8) >> 4) + vp.halfH, 2 * vp.halfH) + 3) >> 2;
+    if (tx1 <= tx0 || ty1 <= ty0 || (uint32_t)((tx1 - tx0) * (ty1 - ty0)) > kHiddenTiles) return false;
+    const int32_t tw = vp.width >> 2;
+    uint32_t known = 0xFFFFFFFFu;
+    for (int32_t y = ty0 + (lane >> 3); y < ty1; y += 4)
+        for (int32_t x = tx0 + (lane & 7); x < tx1; x += 8) known = min(known, vp.tileMin[y * tw + x]);
+    const float zf = __uint_as_float(z), bound = fadd(zf, fmul(zf, 0x1p-16f));
+    return (int32_t)z >= 0 && __all_sync(0xFFFFFFFFu, (__float_as_uint(bound) | 0x80000000u) < known);
+}
+
 // Mesh stage. A work item is one meshlet of one view: a single-view draw numbers its meshlets
 // 0..count-1; a batched draw concatenates the meshlet ranges of its views (viewStart is their
 // prefix), so one launch serves views of any size.
@@ -1018,14 +1047,26 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
             return code == kCodeInBand;
         };
         const bool in0 = xform(lane, px0, py0, pz0, pw0), in1 = xform(32 + lane, px1, py1, pz1, pw1);
-        // every vertex slot inside the viewport and the depth range: every triangle is trivially accepted
-        const bool allInside = __all_sync(0xFFFFFFFFu, in0 && in1);
-        S.idx[lane] = preload64_index4(ix0), S.idx[32 + lane] = preload64_index4(ix1), S.idx[64 + lane] = preload64_index4(ix2);
+        const uint32_t mx0 = preload64_index4(ix0), mx1 = preload64_index4(ix1), mx2 = preload64_index4(ix2);
+        S.idx[lane] = mx0, S.idx[32 + lane] = mx1, S.idx[64 + lane] = mx2;
+        // vertex slots that count: all, or (alpha pass) the meshlet's vertices if its triangles use no others
+        uint32_t slots = 64;
+        if (kAlpha && nv < 64) {
+            const uint32_t first = 4 * lane, used = first >= nt ? 0u : 0xFFFFFFFFu >> (8 * (4 - min(nt - first, 4u)));
+            const uint32_t past = (__vcmpgeu4(mx0, nv * 0x01010101u) | __vcmpgeu4(mx1, nv * 0x01010101u) | __vcmpgeu4(mx2, nv * 0x01010101u)) & used;
+            if (!__any_sync(0xFFFFFFFFu, past != 0)) slots = nv;
+        }
+        // every such vertex inside the viewport and the depth range: every triangle is trivially accepted
+        const bool allInside = __all_sync(0xFFFFFFFFu, (in0 || (kAlpha && lane >= slots)) && (in1 || (kAlpha && 32 + lane >= slots)));
         __syncwarp();
 
         // About half of a closed meshlet's triangles face away. The face test runs first for all of
         // them and compacts the rest into S.live, so the setup and binning below run on full
         // 32-triangle steps. Each triangle keeps its index p (its rank), so the keys do not change.
+        // Alpha pass: a meshlet behind what is drawn is only counted (its box of tiles takes fewer instructions than
+        // its triangles). The opaque pass, where a smaller part is hidden, loses by the test: 354 -> 364 us at
+        // 1080p, 1.27 -> 1.38 ms for 24 batched views.
+        const bool hidden = kAlpha && allInside && vp.tileMin && meshlet_hidden(S.pz, slots, vp, lane);
         uint32_t nLive = 0;
         for (uint32_t base = 0; base < nt; base += 32) {
             const uint32_t p = base + lane;
@@ -1043,6 +1084,16 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
             const float2 q0 = S.xy[i0], q1 = S.xy[i1], q2 = S.xy[i2];
             const bool live = clip || (accepted && front_facing({ q0.x, q0.y, 0.0f, 0.0f }, { q1.x, q1.y, 0.0f, 0.0f },
                                                                 { q2.x, q2.y, 0.0f, 0.0f }, cullMode));
+            if (kAlpha && hidden) {  // counted alone
+                if (live) {
+                    Setup t;
+                    t.Pos0 = S.pz[i0].x, t.Pos1 = S.pz[i1].x, t.Pos2 = S.pz[i2].x;
+                    uint32_t bbMin, bbMax;
+                    render_bbox(t, vp.halfW, vp.halfH, bbMin, bbMax);
+                    nRaster += lo16(bbMin) < lo16(bbMax) && hi16(bbMin) < hi16(bbMax);
+                }
+                continue;
+            }
             const unsigned liveMask = __ballot_sync(0xFFFFFFFFu, live);
             if (live) S.live[nLive + __popc(liveMask & ((1u << lane) - 1u))] = i0 | (i1 << 8) | (i2 << 16) | (p << 24) | (clip ? 0x80000000u : 0u);
             nLive += __popc(liveMask);
