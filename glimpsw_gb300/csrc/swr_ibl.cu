@@ -103,35 +103,58 @@ __device__ __forceinline__ F3 sample_env_level(const DevTexture& t, const EnvLev
     return { r.x, r.y, rz.x + (rz.y - rz.x) * fy };
 }
 
-// A texel's channels have at most 6 mantissa bits, so the top half of each float holds it: x and y in one word,
-// z as a float, row by row.
-__global__ void k_unpack_env(const __grid_constant__ DevTexture env, uint2* __restrict__ texels) {
+// A level unpacked for the irradiance integral: rows of width + 1 texels, the last one repeated, so that a sample's
+// right neighbour is always the next texel. A texel holds its x and y and those of the row below (the last row's:
+// its own) as the top halves of floats, which channels of at most 6 mantissa bits fit, and both z: a sample's
+// operands are two loads. (Whole floats in four loads took the caches' bandwidth: 1.12 ms.)
+__global__ void k_unpack_env(const __grid_constant__ DevTexture env, uint4* __restrict__ texels) {
     const EnvLevel e = env_level(env, 2);
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (uint32_t)(e.width * e.height)) return;
-    const F3 c = unpack_r11g11b10(e.base[texel_offset((int32_t)(i % e.width), (int32_t)(i / e.width), e.stride)]);
-    texels[i] = make_uint2((__float_as_uint(c.x) >> 16) | __float_as_uint(c.y), __float_as_uint(c.z));
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, pitch = (uint32_t)e.width + 1;
+    if (i >= pitch * (uint32_t)e.height) return;
+    const int32_t x = min((int32_t)(i % pitch), e.width - 1), y = (int32_t)(i / pitch);
+    const F3 c = unpack_r11g11b10(e.base[texel_offset(x, y, e.stride)]);
+    const F3 d = unpack_r11g11b10(e.base[texel_offset(x, min(y + 1, e.height - 1), e.stride)]);
+    texels[i] = make_uint4((__float_as_uint(c.x) >> 16) | __float_as_uint(c.y), (__float_as_uint(d.x) >> 16) | __float_as_uint(d.y),
+                           __float_as_uint(c.z), __float_as_uint(d.z));
 }
-__device__ __forceinline__ float2 unpacked_xy(uint2 p) { return make_float2(__uint_as_float(p.x << 16), __uint_as_float(p.x & 0xFFFF0000u)); }
-// sample_env_level from them: 8 operations unpack the four texels instead of 36, and the sample is bound by
-// integer and logic operations (half rate).
-__device__ __forceinline__ F3 sample_env_unpacked(const DevTexture& t, const EnvLevel& e, const uint2* __restrict__ texels, float u, float v) {
-    const int32_t ix = min(max(__float2int_rn(u * t.scale_lerp_u), 0), t.mask_lerp_u) >> e.m;
-    const int32_t iy = min(max(__float2int_rn(v * t.scale_lerp_v), 0), t.mask_lerp_v) >> e.m;
-    const int32_t xf = max(ix - 127, 0), yf = max(iy - 127, 0);
-    const int32_t tx = xf >> 8, ty = yf >> 8;
-    const bool inX = tx + 1 < e.width, inY = ty + 1 < e.height;
-    const uint2* p = texels + ty * e.width + tx;
-    const uint2* q = p + (inY ? e.width : 0);
-    const int32_t right = inX ? 1 : 0;
-    const uint2 c00 = p[0], c10 = p[right], c01 = q[0], c11 = q[right];
-    const float fs = 1.0f / 256;
-    const float fx = inX ? (float)(xf & 255) * fs : 0.0f, fy = (float)(yf & 255) * fs;
-    const float2 ra = lerp2(unpacked_xy(c00), unpacked_xy(c10), fx), rb = lerp2(unpacked_xy(c01), unpacked_xy(c11), fx);
-    const float2 rz = lerp2(make_float2(__uint_as_float(c00.y), __uint_as_float(c01.y)),
-                            make_float2(__uint_as_float(c10.y), __uint_as_float(c11.y)), fx);
-    const float2 r = lerp2(ra, rb, fy);
-    return { r.x, r.y, rz.x + (rz.y - rz.x) * fy };
+__device__ __forceinline__ float2 unpacked_xy(uint32_t p) { return make_float2(__uint_as_float(p << 16), __uint_as_float(p & 0xFFFF0000u)); }
+__device__ __forceinline__ float2 unpacked_z(uint4 p) { return make_float2(__uint_as_float(p.z), __uint_as_float(p.w)); }
+// A coordinate's texel and fraction: the float path's round2i by adding 2^23 (the product is below 2^22 and not
+// below -1/2, level sizes are at most 8192 << m), whose bits then take the clamp and the shift.
+__device__ __forceinline__ int32_t env_coordinate(float s, int32_t mask, int32_t m, float& frac) {
+    constexpr int32_t kTwo23 = 0x4B000000;
+    const int32_t i = min(__float_as_int(s + 8388608.0f), kTwo23 + mask) >> m;
+    const int32_t f = max(i - ((kTwo23 >> m) + 127), 0);
+    frac = __int_as_float(0x3F800000 | ((f << 15) & 0x7F8000)) - 1.0f;  // (f & 255) / 256
+    return f >> 8;
+}
+// sample_env_level from them.
+__device__ __forceinline__ void sample_env_unpacked(const DevTexture& t, const EnvLevel& e, const uint4* __restrict__ texels, float u, float v,
+                                                    float2& xy, float& z) {
+    float fx, fy;
+    const int32_t tx = env_coordinate(u * t.scale_lerp_u, t.mask_lerp_u, e.m, fx);
+    const int32_t ty = env_coordinate(v * t.scale_lerp_v, t.mask_lerp_v, e.m, fy);
+    const uint4* p = texels + (uint32_t)(ty * (e.width + 1) + tx);
+    const uint4 l = p[0], r = p[1];
+    xy = lerp2(lerp2(unpacked_xy(l.x), unpacked_xy(r.x), fx), lerp2(unpacked_xy(l.y), unpacked_xy(r.y), fx), fy);
+    const float2 rz = lerp2(unpacked_z(l), unpacked_z(r), fx);
+    z = rz.x + (rz.y - rz.x) * fy;
+}
+
+// swr_rcp14 of a positive number with a normal reciprocal, its segments in shared memory.
+__device__ __forceinline__ float rcp14_normal(float x, const uint2* segments) {
+    const uint32_t u = __float_as_uint(x);
+    const uint2 ab = *(const uint2*)((const char*)segments + ((u >> 14) & 0x1F8));
+    const uint32_t sig = ((ab.x - ab.y * ((u >> 7) & 1023)) >> 9) << 7;  // bit 23 set
+    return __uint_as_float((252u * 0x800000u - (u & 0x7F800000u)) + ((u & 0x7FFFFFu) ? sig : 0x1000000u));
+}
+// map_oct of a direction within a percent of unit length (the sum of its absolute coordinates is normal). Halving
+// is exact, so its fma is the product and the sum.
+__device__ __forceinline__ void map_oct_unit(F3 n, float& u, float& v, const uint2* segments) {
+    const float w = rcp14_normal(fabsf(n.x) + fabsf(n.y) + fabsf(n.z), segments);
+    const float t = fmaxf(-n.z * w, 0.0f);
+    u = fmaf(fmaf(n.x, w, mulsign(t, n.x)), 0.5f, 0.5f);
+    v = fmaf(fmaf(n.y, w, mulsign(t, n.y)), 0.5f, 0.5f);
 }
 
 // SampleOctLevel<EnvSampler> (Texture.h:467-480): between mips trunc(level) and trunc(level) + 1.
@@ -193,30 +216,53 @@ __device__ __forceinline__ float approx_log2(float x) {
 // receives the adding lane's sums: channel lane / T of texel lane % T, or all channels of texel lane.
 template <int T, int C>
 constexpr int lane_sums() { return T * C <= 32 ? 1 : C; }
+// A lane with one sum reads four samples at a time: the buffer then holds a row of samples (padded to the
+// banks) per channel and texel; else a sample's channels and texels are together.
+template <int T, int C, int K>
+struct SumBuffer {
+    static constexpr bool kRows = lane_sums<T, C>() == 1;
+    static constexpr int kPitch = kRows ? (K + 31) / 32 * 32 + 8 : 0;
+    static constexpr int kSize = 2 * (kRows ? T * C * kPitch : K * C * T);
+    static_assert(!kRows || T == 4, "8 words of a row step over the banks of 4 rows");
+};
 template <int W, int T, int C, int K, class ChunkFn, class TermFn>
 __device__ __forceinline__ void ordered_sum(float* buf, float (&sum)[lane_sums<T, C>()], ChunkFn chunk, TermFn term) {
     constexpr uint32_t kStep = 32 / T;
     constexpr int kSums = lane_sums<T, C>();
+    using B = SumBuffer<T, C, K>;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, texel = lane % T;
 #pragma unroll
     for (int j = 0; j < kSums; j++) sum[j] = 0.0f;
     uint32_t before = 0;
     for (uint32_t c = 0;; c++) {
         const uint32_t n = chunk(c);
-        float* b = buf + (c & 1) * (K * C * T) + texel;
+        float* b = buf + (c & 1) * (B::kSize / 2) + (B::kRows ? texel * B::kPitch : texel);
         if (warp > 0) {
             for (uint32_t k = (warp - 1) * kStep + lane / T; k < n; k += W * kStep) {
                 float t[C];
                 term(k, t);
 #pragma unroll
-                for (int j = 0; j < C; j++) b[(k * C + j) * T] = t[j];
+                for (int j = 0; j < C; j++) b[B::kRows ? j * T * B::kPitch + k : (k * C + j) * T] = t[j];
             }
         } else if (before && lane < (kSums == 1 ? T * C : T)) {  // the chunk of the last barrier
-            const float* q = buf + ((c + 1) & 1) * (K * C * T) + (kSums == 1 ? lane / T : 0) * T + texel;
+            const float* q = buf + ((c + 1) & 1) * (B::kSize / 2) + (B::kRows ? lane * B::kPitch : texel);
+            if constexpr (B::kRows) {
+                uint32_t k = 0;
+#pragma unroll 4
+                for (; k + 4 <= before; k += 4) {
+                    const float4 v = *(const float4*)(q + k);
+                    sum[0] = sum[0] + v.x;
+                    sum[0] = sum[0] + v.y;
+                    sum[0] = sum[0] + v.z;
+                    sum[0] = sum[0] + v.w;
+                }
+                for (; k < before; k++) sum[0] = sum[0] + q[k];
+            } else {
 #pragma unroll 8
-            for (uint32_t k = 0; k < before; k++)
+                for (uint32_t k = 0; k < before; k++)
 #pragma unroll
-                for (int j = 0; j < kSums; j++) sum[j] = sum[j] + q[(k * C + j) * T];
+                    for (int j = 0; j < kSums; j++) sum[j] = sum[j] + q[(k * C + j) * T];
+            }
         }
         if (n == 0) break;
         before = n;
@@ -232,9 +278,11 @@ __device__ __forceinline__ void gather_sums(float acc, uint32_t t, float (&sum)[
 }
 
 // 4 texels a block: 1024 blocks for a 64x64 map, about 7 per SM (blocks of 32 texels were 128, fewer than the
-// SMs, each with a barrier every two samples of a warp). Bound by instruction issue (about 200 operations a
-// sample, 133 M samples): 1.47 -> 1.01 ms. 3 to 6 compute warps 1.34 to 1.12 ms, 12 1.06; 8 texels a block
-// 1.07 or more; packed texels (a larger map) 1.09.
+// SMs, each with a barrier every two samples of a warp): 1.47 -> 1.01 ms for 133 M samples. Bound by instruction
+// issue (67 % of the slots, about 160 operations a sample) and by the texel loads' lines (75 % of the load
+// unit): the texels with both rows in 16 bytes, the phi steps' rows made by one warp, four sums a read
+// and reciprocals without their special cases, 1.01 -> 0.83 ms. 6 compute warps 0.94 ms, 10 0.84; a warp over two phi steps at once
+// 0.85; 8 texels a block was slower (1.07 against 1.01); with the level read as it is packed (a larger map) 0.94.
 constexpr int kIrrWarps = 8, kIrrTexels = 4;
 constexpr int kIrrRows = 2;  // phi steps a chunk
 // The other two have texels enough for 32 a block, a lane each: a warp's lanes then share the sample, and its
@@ -247,12 +295,15 @@ constexpr int kBrdfWarps = 7, kBrdfChunk = 28;
 // texel's sum in that order, as the reference's nested loops do.
 // kUnpacked: the level's texels come unpacked (k_unpack_env).
 template <bool kUnpacked>
-__global__ void __launch_bounds__((kIrrWarps + 1) * 32) k_ibl_irradiance(const __grid_constant__ DevTexture env, const uint2* __restrict__ texels, const __grid_constant__ DevTexture out,
+__global__ void __launch_bounds__((kIrrWarps + 1) * 32) k_ibl_irradiance(const __grid_constant__ DevTexture env, const uint4* __restrict__ texels, const __grid_constant__ DevTexture out,
                                                                           uint32_t* outData, const __grid_constant__ IrradianceTables tb) {
-    __shared__ float buf[2 * kIrrRows * kMaxTheta * 3 * kIrrTexels];
+    __shared__ __align__(16) float buf[SumBuffer<kIrrTexels, 3, kIrrRows * (int)kMaxTheta>::kSize];
+    __shared__ uint2 segments[64];
+    __shared__ float4 rows[2][kIrrRows][kIrrTexels];  // cos(phi) right + sin(phi) up of a chunk's phi steps
     __shared__ float2 theta[kMaxTheta], phi[kMaxPhi];  // cos, sin
     for (uint32_t i = threadIdx.x; i < tb.numTheta; i += blockDim.x) theta[i] = make_float2(tb.cosTheta[i], tb.sinTheta[i]);
     for (uint32_t i = threadIdx.x; i < tb.numPhi; i += blockDim.x) phi[i] = make_float2(tb.cosPhi[i], tb.sinPhi[i]);
+    for (uint32_t i = threadIdx.x; i < 64; i += blockDim.x) segments[i] = swr_a14_device_segments[i];
     __syncthreads();
     const uint32_t n = out.width * out.height;
     const uint32_t i = min(blockIdx.x * kIrrTexels + (threadIdx.x & 31) % kIrrTexels, n - 1);  // lanes past the end repeat the last texel
@@ -262,32 +313,46 @@ __global__ void __launch_bounds__((kIrrWarps + 1) * 32) k_ibl_irradiance(const _
     F3 right, up;
     tangent_frame(N, right, up);
     const EnvLevel level = env_level(env, 2);  // SampleOctLevel at level 2: no second mip
-    F3 tmp[kIrrRows] = {};
+    const float4(*row)[kIrrTexels] = rows[0];
     float acc[1];
+    // the adding warp prepares the next chunk's rows, a lane per row and texel
+    auto prepare = [&](uint32_t c) {
+        const uint32_t r = threadIdx.x / kIrrTexels, step = c * kIrrRows + r;
+        if (r < (uint32_t)kIrrRows && step < tb.numPhi) {
+            const float cp = phi[step].x, sp = phi[step].y;
+            rows[c & 1][r][threadIdx.x % kIrrTexels] =
+                make_float4(cp * right.x + sp * up.x, cp * right.y + sp * up.y, cp * right.z + sp * up.z, 0.0f);
+        }
+    };
+    prepare(0);
+    __syncthreads();
     ordered_sum<kIrrWarps, kIrrTexels, 3, kIrrRows * (int)kMaxTheta>(buf, acc,
         [&](uint32_t c) -> uint32_t {
-            uint32_t rows = 0;
-#pragma unroll
-            for (int r = 0; r < kIrrRows; r++) {
-                if (c * kIrrRows + r >= tb.numPhi) break;
-                const float cp = phi[c * kIrrRows + r].x, sp = phi[c * kIrrRows + r].y;
-                tmp[r] = { cp * right.x + sp * up.x, cp * right.y + sp * up.y, cp * right.z + sp * up.z };
-                rows++;
-            }
-            return rows * tb.numTheta;
+            if (threadIdx.x < 32) prepare(c + 1);
+            row = rows[c & 1];
+            return c * kIrrRows < tb.numPhi ? min((uint32_t)kIrrRows, tb.numPhi - c * kIrrRows) * tb.numTheta : 0u;
         },
         [&](uint32_t k, float (&t)[3]) {
             const bool second = k >= tb.numTheta;
-            const F3 a = second ? tmp[1] : tmp[0];
+            const float4 a = row[second ? 1 : 0][threadIdx.x % kIrrTexels];
             const float2 cs = theta[second ? k - tb.numTheta : k];
             const float ct = cs.x, st = cs.y;
             const float2 d = __fadd2_rn(__fmul2_rn(make_float2(ct, ct), make_float2(N.x, N.y)),
                                         __fmul2_rn(make_float2(st, st), make_float2(a.x, a.y)));
             const F3 dir = { d.x, d.y, ct * N.z + st * a.z };
-            float su, sv;
-            map_oct(dir, su, sv);
-            const F3 s = tonemap_sample(kUnpacked ? sample_env_unpacked(env, level, texels, su, sv) : sample_env_level(env, level, su, sv), 1.0f);
-            t[0] = s.x * ct * st, t[1] = s.y * ct * st, t[2] = s.z * ct * st;
+            float su, sv, z;
+            float2 xy;
+            map_oct_unit(dir, su, sv, segments);
+            if constexpr (kUnpacked) {
+                sample_env_unpacked(env, level, texels, su, sv, xy, z);
+            } else {
+                const F3 s = sample_env_level(env, level, su, sv);
+                xy = make_float2(s.x, s.y), z = s.z;
+            }
+            // tonemap_sample, then times cos(theta) sin(theta)
+            const float r = rcp14_normal(1.0f + dot3({ xy.x, xy.y, z }, { 0.299f, 0.587f, 0.114f }), segments);
+            xy = __fmul2_rn(__fmul2_rn(__fmul2_rn(xy, make_float2(r, r)), make_float2(ct, ct)), make_float2(st, st));
+            t[0] = xy.x, t[1] = xy.y, t[2] = z * r * ct * st;
         });
     if (threadIdx.x >= 32) return;
     float color[3];
@@ -306,7 +371,7 @@ __global__ void __launch_bounds__((kRadWarps + 1) * 32) k_ibl_radiance(const __g
                                                                         uint32_t* outData, const __grid_constant__ HammersleyTable<128> ham,
                                                                         uint32_t totalTexels) {
     constexpr uint32_t numSamples = 128;
-    __shared__ float buf[2 * kRadChunk * 4 * 32];
+    __shared__ float buf[SumBuffer<32, 4, kRadChunk>::kSize];
     const uint32_t i = min(blockIdx.x * 32 + (threadIdx.x & 31), totalTexels - 1);  // lanes past the end repeat the last texel
     uint32_t level = 0, j = i;
     while (j >= (out.width >> level) * (out.height >> level)) j -= (out.width >> level) * (out.height >> level), level++;
@@ -353,7 +418,7 @@ __global__ void __launch_bounds__((kRadWarps + 1) * 32) k_ibl_radiance(const __g
 __global__ void __launch_bounds__((kBrdfWarps + 1) * 32) k_ibl_env_brdf(const __grid_constant__ DevTexture out, uint32_t* outData,
                                                                         const __grid_constant__ HammersleyTable<1024> ham) {
     constexpr uint32_t sampleCount = 1024;
-    __shared__ float buf[2 * kBrdfChunk * 2 * 32];
+    __shared__ float buf[SumBuffer<32, 2, kBrdfChunk>::kSize];
     const uint32_t n = out.width * out.height;
     const uint32_t i = min(blockIdx.x * 32 + (threadIdx.x & 31), n - 1);
     const uint32_t x = i % out.width, y = i / out.width;
@@ -466,11 +531,11 @@ swr_status swr_ibl_irradiance_map(swr_texture env, swr_texture out) {
     static const IrradianceTables tb = irradiance_tables();
     cudaStream_t st = swr_internal_stream();
     const uint32_t n = out->d.width * out->d.height, blocks = (n + kIrrTexels - 1) / kIrrTexels;
-    // Every sample reads one level. Up to kSkyScratchTexels texels (2 MB unpacked, which the caches hold) it is
+    // Every sample reads one level. Up to kSkyScratchTexels texels (4 MB unpacked, which the caches hold) it is
     // unpacked first; a larger one is read as it is.
     if (env->skyScratch) {
-        uint2* texels = (uint2*)env->skyScratch;
-        const uint32_t level = std::min(2u, env->d.mip_levels - 1), count = (env->d.width >> level) * (env->d.height >> level);
+        uint4* texels = (uint4*)env->skyScratch;
+        const uint32_t level = std::min(2u, env->d.mip_levels - 1), count = ((env->d.width >> level) + 1) * (env->d.height >> level);
         {
             LaunchScope ls("k_unpack_env", st);
             k_unpack_env<<<(count + 255) / 256, 256, 0, st>>>(env->d, texels);

@@ -283,13 +283,13 @@ struct swr_scene_t {
     uint64_t version;              // bumped when meshlets or materials move (recorded draw graphs re-capture)
 };
 
-constexpr uint32_t kSkyScratchTexels = 512 * 512;
+constexpr uint32_t kSkyScratchTexels = 512 * 512, kSkyScratchSide = 8192;
 struct swr_texture_t {
     uint32_t format;
     swr::DevTexture d;             // d.data is the device storage
     size_t words;
-    void* skyScratch;              // R11G11B10: room for its level 2 (or last) unpacked, 8 bytes a texel, at most
-                                   // kSkyScratchTexels texels (nullptr: larger, or another format)
+    void* skyScratch;              // R11G11B10: room for its level 2 (or last) unpacked and padded, 16 bytes a texel, up
+                                   // to kSkyScratchTexels texels of a map of at most kSkyScratchSide a side (else nullptr)
 };
 
 struct swr_rasterizer_t {
