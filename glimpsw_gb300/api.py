@@ -611,15 +611,15 @@ class NeuralMaterials:
 
     def gradients(self, material: int, samples_device, count: int, want_latent: bool = True):
         """(param_grad[5704], latent_grad[texels, 8] or None, summed squared error) for explicit samples."""
-        pg = np.zeros(NEURAL_PARAMS, dtype=np.float32)
-        lg = np.zeros((self.texels_per_material, 8), dtype=np.float32) if want_latent else None
+        pg = np.empty(NEURAL_PARAMS, dtype=np.float32)
+        lg = np.empty((self.texels_per_material, 8), dtype=np.float32) if want_latent else None
         loss = C.c_float(0.0)
         _check(_lib.swr_neural_gradients(self.h, material, _ptr(samples_device), count, pg.ctypes.data,
                                          lg.ctypes.data if lg is not None else None, C.byref(loss)))
         return pg, lg, loss.value
 
     def get_params(self, material: int) -> np.ndarray:
-        p = np.zeros(NEURAL_PARAMS, dtype=np.float32)
+        p = np.empty(NEURAL_PARAMS, dtype=np.float32)
         _check(_lib.swr_neural_get_params(self.h, material, p.ctypes.data))
         return p
 
@@ -629,7 +629,7 @@ class NeuralMaterials:
         _check(_lib.swr_neural_set_params(self.h, material, p.ctypes.data))
 
     def get_latents(self, material: int) -> np.ndarray:
-        p = np.zeros((self.texels_per_material, 8), dtype=np.float32)
+        p = np.empty((self.texels_per_material, 8), dtype=np.float32)
         _check(_lib.swr_neural_get_latents(self.h, material, p.ctypes.data))
         return p
 

@@ -4,6 +4,7 @@
 // (SampleLevel<SurfaceSampler>, Texture.h:412-459) produces its training targets and stays the
 // fallback for texture levels the latents do not cover.
 #pragma once
+#include <atomic>
 #include <cstdint>
 
 #include "swr_internal.h"
@@ -129,8 +130,9 @@ struct swr_neural_t {
     uint8_t* image;
     float* partial;
     size_t partialFloats;
-    float* loss;                             // device: squared error, samples, then the status word
+    float* loss;                             // device: squared error, samples, the status word, then the check flags
     uint32_t* status;                        // device: loss + 2
+    std::atomic<uint64_t> flagsInUse{0};     // check flags (kCheckFlags words after loss[3]; 0 when free) held by calls
     std::vector<uint32_t> steps;             // Adam step count per material
     uint64_t seed;
     uint32_t trainCalls;

@@ -79,41 +79,65 @@ swr_status check_status(swr_neural_t* n, cudaStream_t st, const char* what) {
 }
 
 // The check of caller-supplied texels against a material's decoded levels, on the device before the kernels
-// that read them (which do nothing once the flag is set), with words of the call's own: the flag, then
-// copies of the model's loss and status, read back together. The lists used to come to the host to be
-// looked at, and the partial gradients to be summed: 262,000 texels and 32,768 samples with their results
-// took 1.79 ms, now 0.18 ms.
+// that read them (which do nothing once the flag is set). The call holds one of the model's flags, or an
+// allocation when all are held by other threads' calls; they lie after the model's loss and status, and one copy reads
+// all. The lists used to come to the host to be looked at, and the partial gradients to be summed: 262,000
+// texels and 32,768 samples with their results took 1.79 ms; 0.18 ms with an allocation and two copies a
+// call, 0.14 ms now.
+constexpr uint32_t kCheckFlags = 64, kOutcomeWords = 4 + kCheckFlags;
 struct TexelCheck {
-    uint32_t* words = nullptr;  // flag, loss, samples, status
+    swr_neural_t* const n;
+    uint32_t* flag = nullptr;
+    int slot = -1;  // of flag among the model's, -1: allocated
     cudaStream_t st = nullptr;
-    bool refused = false, timedOut = false;
+    bool refused = false, timedOut = false, done = false;
     float loss = 0.0f;
+    explicit TexelCheck(swr_neural_t* model) : n(model) {}
+    TexelCheck(const TexelCheck&) = delete;
     ~TexelCheck() {
-        if (words) cudaFreeAsync(words, st);
-    }
-    cudaError_t launch(const swr_neural_t* n, uint32_t material, const uint32_t* texels, uint32_t count, cudaStream_t stream) {
-        st = stream;
-        cudaError_t e = cudaMallocAsync((void**)&words, 4 * sizeof(uint32_t), st);
-        if (e != cudaSuccess) {
-            words = nullptr;
-            return e;
+        if (!flag) return;
+        if (slot < 0) {
+            cudaFreeAsync(flag, st);
+            return;
         }
-        e = cudaMemsetAsync(words, 0, sizeof(uint32_t), st);
-        if (e != cudaSuccess) return e;
+        if (refused || !done) cudaMemsetAsync(flag, 0, sizeof(uint32_t), st);
+        if (refused || !done) cudaStreamSynchronize(st);  // before another call takes the flag
+        n->flagsInUse.fetch_and(~(1ull << slot));
+    }
+    cudaError_t launch(uint32_t material, const uint32_t* texels, uint32_t count, cudaStream_t stream) {
+        st = stream;
+        uint64_t held = n->flagsInUse.load();
+        while (~held && slot < 0) {
+            const int free = __builtin_ctzll(~held);
+            if (n->flagsInUse.compare_exchange_weak(held, held | (1ull << free))) slot = free;
+        }
+        if (slot >= 0) {
+            flag = (uint32_t*)n->loss + 4 + slot;
+        } else {
+            cudaError_t e = cudaMallocAsync((void**)&flag, sizeof(uint32_t), st);
+            if (e != cudaSuccess) {
+                flag = nullptr;
+                return e;
+            }
+            e = cudaMemsetAsync(flag, 0, sizeof(uint32_t), st);
+            if (e != cudaSuccess) return e;
+        }
         const DevTexture& t = n->texHost[material];
         LaunchScope ls("k_neural_check", st);
-        launch_neural_check(texels, count, n->d.levels + 2, t.width, t.height, words, st);
+        launch_neural_check(texels, count, n->d.levels + 2, t.width, t.height, flag, st);
         return cudaGetLastError();
     }
     // Waits for the call's kernels and reads their outcome.
-    cudaError_t wait(swr_neural_t* n) {
-        uint32_t w[4] = {};
-        cudaError_t e = cudaMemcpyAsync(words + 1, n->loss, 3 * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(w, words, sizeof(w), cudaMemcpyDeviceToHost, st);
+    cudaError_t wait() {
+        uint32_t w[kOutcomeWords] = {}, set = 0;
+        cudaError_t e = cudaMemcpyAsync(w, n->loss, sizeof(w), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess && slot < 0) e = cudaMemcpyAsync(&set, flag, sizeof(set), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return e;
-        refused = w[0] != 0, timedOut = !refused && w[3] != 0;
-        memcpy(&loss, &w[1], sizeof(float));
+        done = true;
+        if (slot >= 0) set = w[4 + slot];
+        refused = set != 0, timedOut = !refused && w[2] != 0;
+        memcpy(&loss, &w[0], sizeof(float));
         if (timedOut) cudaMemsetAsync(n->status, 0, sizeof(uint32_t), st);
         return cudaSuccess;
     }
@@ -207,7 +231,7 @@ swr_status swr_neural_create(const swr_texture* textures, uint32_t num_materials
     chk(dev_alloc(&n->paramM, (size_t)num_materials * kNeuralParams));
     chk(dev_alloc(&n->paramV, (size_t)num_materials * kNeuralParams));
     chk(dev_alloc(&n->image, (size_t)num_materials * kNeuralImage));
-    chk(dev_alloc(&n->loss, 4));
+    chk(dev_alloc(&n->loss, kOutcomeWords));
     n->status = (uint32_t*)(n->loss + 2);
     chk(dev_alloc(&n->counters, 4 * (size_t)(num_materials + 1) + kNeuralMaxDecoded));
     if (e != cudaSuccess) {
@@ -226,7 +250,7 @@ swr_status swr_neural_create(const swr_texture* textures, uint32_t num_materials
     chk(cudaMemsetAsync(n->latentV, 0, latentFloats * sizeof(float), st));
     chk(cudaMemsetAsync(n->latentGrad, 0, latentFloats * sizeof(float), st));
     chk(cudaMemsetAsync(n->image, 0, (size_t)num_materials * kNeuralImage, st));
-    chk(cudaMemsetAsync(n->status, 0, 4, st));
+    chk(cudaMemsetAsync(n->loss, 0, kOutcomeWords * sizeof(uint32_t), st));
     n->d.tex = n->tex;
     n->d.latentHalf = n->latentHalf;
     n->d.image = n->image;
@@ -387,8 +411,8 @@ swr_status swr_neural_gradients(swr_neural n, uint32_t material, const uint32_t*
     const size_t T8 = (size_t)n->d.texelsPerMaterial * 8;
     float* g = n->latentGrad + (size_t)material * T8;
     float* sum = n->partial + (size_t)cpm * kNeuralParams;
-    TexelCheck check;
-    cudaError_t e = check.launch(n, material, samples_device, count, st);
+    TexelCheck check(n);
+    cudaError_t e = check.launch(material, samples_device, count, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(g, 0, T8 * sizeof(float), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(n->loss, 0, 8, st);
     NeuralTrainArgs a = train_args(n);
@@ -396,7 +420,7 @@ swr_status swr_neural_gradients(swr_neural n, uint32_t material, const uint32_t*
     a.materials[0] = material;
     a.numSlots = 1, a.samplesPerMaterial = count, a.ctasPerMaterial = cpm;
     a.samples = samples_device;
-    a.invalid = check.words;
+    a.invalid = check.flag;
     if (e == cudaSuccess) {
         LaunchScope ls("k_neural_train", st);
         launch_neural_train(a, cpm, st);
@@ -408,7 +432,7 @@ swr_status swr_neural_gradients(swr_neural n, uint32_t material, const uint32_t*
         e = cudaGetLastError();
     }
     // the outcome first: a refused call leaves the caller's arrays as they were
-    if (e == cudaSuccess) e = check.wait(n);
+    if (e == cudaSuccess) e = check.wait();
     if (e == cudaSuccess && check.refused) return swr_internal_fail(SWR_EINVAL, "swr_neural_gradients: sample outside the decoded levels");
     if (e == cudaSuccess) e = cudaMemcpyAsync(param_grad, sum, kNeuralParams * sizeof(float), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess && latent_grad) e = cudaMemcpyAsync(latent_grad, g, T8 * sizeof(float), cudaMemcpyDeviceToHost, st);
@@ -549,12 +573,12 @@ swr_status swr_neural_decode(swr_neural n, uint32_t material, const uint32_t* te
     cudaStream_t st = swr_internal_stream();
     neural_sync_half(n, st);
     // one material: the request list is the texel list itself, slot i = texel i
-    TexelCheck check;
-    cudaError_t e = check.launch(n, material, texels_device, count, st);
+    TexelCheck check(n);
+    cudaError_t e = check.launch(material, texels_device, count, st);
     if (e == cudaSuccess) {
         NeuralDecodeArgs a = {};
         a.n = n->d;
-        a.texels = texels_device, a.invalid = check.words;
+        a.texels = texels_device, a.invalid = check.flag;
         a.material = material, a.count = count;
         a.out = (uint2*)out_device;
         a.status = n->status;
@@ -562,7 +586,7 @@ swr_status swr_neural_decode(swr_neural n, uint32_t material, const uint32_t* te
         launch_neural_decode(a, std::min<uint32_t>((count + 127) / 128, neural_decode_blocks_per_sm() * num_sms()), st);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = check.wait(n);
+    if (e == cudaSuccess) e = check.wait();
     if (e != cudaSuccess) return swr_internal_cuda_fail(e, "swr_neural_decode");
     if (check.refused) return swr_internal_fail(SWR_EINVAL, "swr_neural_decode: texel outside the decoded levels");
     return check.timedOut ? swr_internal_fail(SWR_ETIMEOUT, "swr_neural: a tensor-core wait timed out") : SWR_OK;
