@@ -316,6 +316,12 @@ swr_status swr_internal_finalize(swr_framebuffer fb) {
     return SWR_OK;
 }
 
+// The keys a layer's pixels are read from if draws pend for it (nullptr: the layer's words are up to date).
+static const unsigned long long* pending_keys(swr_framebuffer fb, uint32_t layer) {
+    const bool pending = fb->layers_stale == kStaleAll ? layer <= 1 : fb->layers_stale == kStaleDepth && layer == 1;
+    return pending ? fb->keys : nullptr;
+}
+
 extern "C" {
 
 swr_status swr_framebuffer_clear(swr_framebuffer fb, uint32_t color, float depth) {
@@ -343,9 +349,8 @@ swr_status swr_framebuffer_clear_layer(swr_framebuffer fb, uint32_t layer, uint3
 swr_status swr_framebuffer_get_pixels_device(swr_framebuffer fb, uint32_t layer, uint32_t* dest_device) {
     if (!fb || layer >= fb->num_layers || !dest_device)
         return fail(SWR_EINVAL, "swr_framebuffer_get_pixels_device: bad argument");
-    swr_status st = swr_internal_finalize(fb);
-    if (st != SWR_OK) return st;
-    launch_detile(fb->layers + (size_t)layer * fb->layer_stride, dest_device, fb->width, fb->height, fb->width, t_stream);
+    launch_detile(fb->layers + (size_t)layer * fb->layer_stride, pending_keys(fb, layer), dest_device, fb->width, fb->height,
+                  fb->width, layer, t_stream);
     SWR_CHECK_LAUNCH("swr_framebuffer_get_pixels_device");
     return SWR_OK;
 }
@@ -353,14 +358,13 @@ swr_status swr_framebuffer_get_pixels_device(swr_framebuffer fb, uint32_t layer,
 swr_status swr_framebuffer_get_pixels(swr_framebuffer fb, uint32_t layer, uint32_t* dest, uint32_t stride) {
     if (!fb || layer >= fb->num_layers || !dest || stride < fb->width)
         return fail(SWR_EINVAL, "swr_framebuffer_get_pixels: bad argument");
-    swr_status st = swr_internal_finalize(fb);
-    if (st != SWR_OK) return st;
     const uint32_t* src = fb->layers + (size_t)layer * fb->layer_stride;
+    const unsigned long long* keys = pending_keys(fb, layer);
     // Pinned host memory the device can address is written by the detiling kernel itself, over the
     // host link, with no staging copy; other memory goes through a device buffer and a copy.
     cudaPointerAttributes pa = {};
     if (cudaPointerGetAttributes(&pa, dest) == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer) {
-        launch_detile(src, (uint32_t*)pa.devicePointer, fb->width, fb->height, stride, t_stream);
+        launch_detile(src, keys, (uint32_t*)pa.devicePointer, fb->width, fb->height, stride, layer, t_stream);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(t_stream);
         if (e != cudaSuccess) return cuda_fail(e, "swr_framebuffer_get_pixels");
@@ -369,7 +373,7 @@ swr_status swr_framebuffer_get_pixels(swr_framebuffer fb, uint32_t layer, uint32
     cudaGetLastError();  // an unregistered pointer is not an error
     uint32_t* tmp = nullptr;
     SWR_CUDA(cudaMallocAsync(&tmp, (size_t)fb->width * fb->height * 4, t_stream));
-    launch_detile(src, tmp, fb->width, fb->height, fb->width, t_stream);
+    launch_detile(src, keys, tmp, fb->width, fb->height, fb->width, layer, t_stream);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
         e = cudaMemcpy2DAsync(dest, (size_t)stride * 4, tmp, (size_t)fb->width * 4, (size_t)fb->width * 4, fb->height,

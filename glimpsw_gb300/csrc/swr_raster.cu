@@ -1526,13 +1526,38 @@ __global__ void k_finalize_overdraw(const unsigned long long* __restrict__ keys,
     }
 }
 
-// Framebuffer::GetPixels de-tiling (ImageHelpers.cpp:109-147) into a row-major device buffer.
-__global__ void k_detile(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t width, uint32_t height,
-                         uint32_t stride) {
-    const uint32_t n = width * height;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t y = i / width, x = i - y * width;
-        dst[(size_t)y * stride + x] = src[pixel_offset(x, y, width)];
+// Framebuffer::GetPixels de-tiling (ImageHelpers.cpp:109-147) into a row-major buffer, a thread per row of
+// a 4x4 tile: a 16-byte load, and a 16-byte store where the rows of dst are aligned (vec). kKeys: pending draws are
+// read from the keys, which the layer's words (layer 0: surface ids, 1: depths) only fill in for, instead of
+// being written to the layers first: 12 bytes a pixel instead of 24. Bound by bandwidth: two 2560x1440 layers
+// 14.9 -> 9.2 us (a thread per pixel before); the ids of 24 views of 256x256 to 2560x1440 from their keys
+// 164 -> 90 us, the pass over their layers included (a thread per tile: 157).
+template <bool kKeys>
+__global__ void __launch_bounds__(256) k_detile(const uint32_t* __restrict__ src, const unsigned long long* __restrict__ keys, uint32_t* dst,
+                                                uint32_t width, uint32_t height, uint32_t stride, uint32_t layer, uint32_t vec) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, t = i >> 2, tw = width >> 2;
+    if (t >= tw * (height >> 2)) return;
+    const uint32_t ty = t / tw, tx = t - ty * tw;
+    uint32_t v[4];
+    if constexpr (kKeys) {
+        const ulonglong2 p = ((const ulonglong2*)keys)[2 * i], q = ((const ulonglong2*)keys)[2 * i + 1];
+        const unsigned long long k[4] = { p.x, p.y, q.x, q.y };
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t low = (uint32_t)k[j];
+            if (low == kKeyEmptyLow) v[j] = src[4 * i + j];
+            else v[j] = layer == 0 ? rank_surface_id(0xFFFFFFFEu - low) : __float_as_uint(float_unorder((uint32_t)(k[j] >> 32)));
+        }
+    } else {
+        const uint4 p = ((const uint4*)src)[i];
+        v[0] = p.x, v[1] = p.y, v[2] = p.z, v[3] = p.w;
+    }
+    uint32_t* row = dst + (size_t)(ty * 4 + (i & 3)) * stride + tx * 4;
+    if (vec) {
+        *(uint4*)row = make_uint4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) row[j] = v[j];
     }
 }
 
@@ -1666,9 +1691,12 @@ void launch_finalize_overdraw(const unsigned long long* keys, const unsigned lon
     k_finalize_overdraw<<<grid_for(n, 1, 256), 256, 0, st>>>(keys, counts, l0, l1, n);
 }
 
-void launch_detile(const uint32_t* src, uint32_t* dst, uint32_t width, uint32_t height, uint32_t stride, cudaStream_t st) {
+void launch_detile(const uint32_t* src, const unsigned long long* keys, uint32_t* dst, uint32_t width, uint32_t height,
+                   uint32_t stride, uint32_t layer, cudaStream_t st) {
     LaunchScope ls("k_detile", st);
-    k_detile<<<grid_for(width * height, 1, 256), 256, 0, st>>>(src, dst, width, height, stride);
+    const uint32_t blocks = (width * (height >> 2) + 255) / 256, vec = ((uintptr_t)dst & 15) == 0 && stride % 4 == 0;
+    if (keys) k_detile<true><<<blocks, 256, 0, st>>>(src, keys, dst, width, height, stride, layer, vec);
+    else k_detile<false><<<blocks, 256, 0, st>>>(src, nullptr, dst, width, height, stride, layer, vec);
 }
 
 }  // namespace swr

@@ -213,7 +213,8 @@ struct ResolveArgs {
     const DevMaterial* materials;
     uint32_t numMaterials;
     uint32_t* color;        // layer 0 (surface ids in, RGBA8 out)
-    const float* depth;     // layer 1
+    float* depth;           // layer 1
+    const unsigned long long* keys;  // draws not yet in the layers (nullptr: the layers are up to date)
     uint32_t width, height;
     float objectToClip[16];
     float objectToWorld[9];
@@ -332,8 +333,20 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
     const uint32_t px = x0 + (l & 3), py = y0 + (l >> 2);
     const uint32_t off = pixel_offset(x0, y0, a.width) + l;
 
-    const uint32_t id = a.color[off];
-    const float d = a.depth[off];
+    // Pending draws are taken from the keys, and their depths (for the second neural pass also their ids) reach
+    // the layers here: a pass over keys and layers of its own took 3 to 11 us.
+    uint32_t id;
+    float d;
+    const unsigned long long key = (kMode == kResolvePlain || kMode == kResolveEmit) && a.keys ? a.keys[off] : kKeyEmptyLow;
+    if ((uint32_t)key != kKeyEmptyLow) {
+        id = rank_surface_id(0xFFFFFFFEu - (uint32_t)key);
+        d = float_unorder((uint32_t)(key >> 32));
+        a.depth[off] = d;
+        if constexpr (kMode == kResolveEmit) a.color[off] = id;
+    } else {
+        id = a.color[off];
+        d = a.depth[off];
+    }
     const bool isSky = d <= 0.0f;
     const float fpx = (float)(int32_t)px, fpy = (float)(int32_t)py;
     float qw;
@@ -676,21 +689,25 @@ using namespace swr;
 namespace {
 // ShadingContext::Resolve's per-frame constants (Shading.cpp:658-690); the lights are copied to a
 // stream-ordered device allocation that the caller frees after the launch.
-swr_status build_resolve_args(swr_framebuffer fb, const swr_shading_context* ctx, ResolveArgs& a, const char* fn) {
+// takesKeys: the kernel reads pending draws of both layers from the keys (it sets a.keys then); else they
+// are written to the layers first.
+swr_status build_resolve_args(swr_framebuffer fb, const swr_shading_context* ctx, ResolveArgs& a, const char* fn, bool takesKeys) {
     if (!fb || !ctx || !ctx->scene) return swr_internal_fail(SWR_EINVAL, (std::string(fn) + ": NULL argument").c_str());
     if (ctx->num_lights && !ctx->lights) return swr_internal_fail(SWR_EINVAL, (std::string(fn) + ": lights is NULL").c_str());
     if (ctx->skybox && ctx->skybox->format != SWR_FORMAT_R11G11B10F)
         return swr_internal_fail(SWR_EINVAL, (std::string(fn) + ": the skybox must be R11G11B10f").c_str());
-    swr_status fst = swr_internal_finalize(fb);  // pending draws reach layers 0 and 1 first
+    takesKeys = takesKeys && fb->layers_stale == kStaleAll;
+    swr_status fst = takesKeys ? SWR_OK : swr_internal_finalize(fb);
     if (fst != SWR_OK) return fst;
     cudaStream_t st = swr_internal_stream();
     a = {};
+    a.keys = takesKeys ? fb->keys : nullptr;
     a.meshlets = ctx->scene->meshlets;
     a.numMeshlets = ctx->scene->count;
     a.materials = ctx->scene->materials;
     a.numMaterials = ctx->scene->num_materials;
     a.color = fb->layers;
-    a.depth = (const float*)(fb->layers + fb->layer_stride);
+    a.depth = (float*)(fb->layers + fb->layer_stride);
     a.width = fb->width, a.height = fb->height;
     memcpy(a.objectToClip, ctx->object_to_clip, sizeof(a.objectToClip));
     memcpy(a.objectToWorld, ctx->object_to_world, sizeof(a.objectToWorld));
@@ -844,7 +861,7 @@ swr_status swr_downsample_depth(swr_framebuffer fb, swr_texture dest) {
 swr_status swr_resolve(swr_rasterizer r, swr_framebuffer fb, const swr_shading_context* ctx) {
     (void)r;
     ResolveArgs a = {};
-    swr_status s = build_resolve_args(fb, ctx, a, "swr_resolve");
+    swr_status s = build_resolve_args(fb, ctx, a, "swr_resolve", true);
     if (s != SWR_OK) return s;
     cudaStream_t st = swr_internal_stream();
     const uint32_t tiles = (fb->width / 4) * (fb->height / 4);
@@ -856,6 +873,7 @@ swr_status swr_resolve(swr_rasterizer r, swr_framebuffer fb, const swr_shading_c
     }
     if (a.lights) cudaFreeAsync((void*)a.lights, st);
     if (e != cudaSuccess) return swr_internal_cuda_fail(e, "swr_resolve");
+    fb->layers_stale = kStaleNone;
     fb->keys_valid = false;  // layer 0 now holds colour; a later draw rebuilds its keys from depth
     return SWR_OK;
 }
@@ -864,7 +882,7 @@ swr_status swr_resolve_debug(swr_rasterizer r, swr_framebuffer fb, const swr_sha
     (void)r;
     if (layer > SWR_DEBUG_OVERDRAW_QUAD) return swr_internal_fail(SWR_EINVAL, "swr_resolve_debug: unknown debug layer");
     ResolveArgs a = {};
-    swr_status s = build_resolve_args(fb, ctx, a, "swr_resolve_debug");
+    swr_status s = build_resolve_args(fb, ctx, a, "swr_resolve_debug", false);
     if (s != SWR_OK) return s;
     a.debugLayer = layer;
     cudaStream_t st = swr_internal_stream();
@@ -886,7 +904,7 @@ swr_status swr_resolve_neural(swr_rasterizer r, swr_framebuffer fb, const swr_sh
     (void)r;
     if (!n) return swr_internal_fail(SWR_EINVAL, "swr_resolve_neural: NULL model");
     ResolveArgs a = {};
-    swr_status s = build_resolve_args(fb, ctx, a, "swr_resolve_neural");
+    swr_status s = build_resolve_args(fb, ctx, a, "swr_resolve_neural", true);
     if (s != SWR_OK) return s;
     cudaStream_t st = swr_internal_stream();
     const uint32_t M = n->d.numMaterials;
@@ -924,6 +942,7 @@ swr_status swr_resolve_neural(swr_rasterizer r, swr_framebuffer fb, const swr_sh
         LaunchScope ls("k_resolve_emit", st);
         k_resolve<kResolveEmit><<<blocks, 256, 0, st>>>(a, nr);
         e = cudaGetLastError();
+        if (e == cudaSuccess) fb->layers_stale = kStaleNone;
     }
     if (e == cudaSuccess) {
         LaunchScope ls("k_neural_offsets", st);
