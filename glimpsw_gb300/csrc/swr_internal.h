@@ -184,6 +184,7 @@ struct DrawArgs {
     unsigned long long* counts;
     // single view: order_stride(count), set by launch_draw
     uint32_t orderStride;
+    uint32_t partShift;  // small draws: 2^partShift warps take a meshlet
     // the shading steps read a pixel's key before its atomicMax only for triangles of at most this
     // many tiles (0: for all); set by launch_draw
     uint32_t keyReadTiles;

@@ -829,7 +829,12 @@ enum : int { kPassOpaque = 0, kPassAlpha = 1, kPassOverdraw = 2 };
 // clip positions, indices, PrimCount, CullMode and FragmentShaderId are read from the record
 // instead of ShadeMeshlet's transform of the Meshlet (whose texcoords and material the alpha test
 // still reads).
-template <int kPass, bool kShaded = false>
+// kSmall: a single-view draw of at most as many meshlets as the grid has warps. 2^a.partShift warps take a meshlet
+// each, chosen by their index: all of them transform it and test its faces, and each draws its share of the
+// triangles that are left. A warp alone is a serial chain (a step of four tiles takes 1,300 cycles): 60 meshlets at
+// 252x140 56 -> 8.7 us (at most 8 warps a meshlet 13.8, 16 10.9), 1024 at 1280x720 66 -> 31 us, and with the
+// tail gone fewer triangles are queued: chunk stage 39 -> 18 us. Two items a warp: 33 us.
+template <int kPass, bool kShaded = false, bool kSmall = false>
 __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
     constexpr bool kAlpha = kPass == kPassAlpha, kOver = kPass == kPassOverdraw;
     using Smem = typename std::conditional<kAlpha, WarpSmemAlpha, WarpSmem>::type;
@@ -873,8 +878,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
     uint32_t fetchView = 0;                // batched draws: the view of the fetched group
     unsigned fetchMask = 0;                // lanes of the fetched group whose meshlet is visible
     // Single view: positions per fetch. A draw of fewer meshlets than groups for every warp starts with
-    // smaller groups, so that no warp draws several meshlets in a row while others have none (60 meshlets at
-    // 252x140: mesh stage 110 -> 55 us; 1024 at 1280x720: 106 -> 68 us).
+    // smaller groups, so that no warp draws several meshlets in a row while others have none.
     const uint32_t leastGroup = totalItems < 2 * numWarps ? 1u : 2u;
     const uint32_t firstGroup = min(kDrawGroup, max(totalItems / numWarps, leastGroup));
     uint32_t fetchGroup = firstGroup;
@@ -902,9 +906,22 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
         if (alpha) a.s.alphaList[at + __popc(am & ((1u << lane) - 1u))] = item;
         return mask & ~am;
     };
+    uint32_t nextItem = warp * gridDim.x + blockIdx.x;  // kSmall: blocks first, so that all SMs get some
     while (true) {
-        uint32_t m, view = 0, item;
-        if constexpr (kAlpha) {
+        uint32_t m, view = 0, item, part = 0;
+        if constexpr (kSmall) {
+            if (nextItem >= totalItems << a.partShift) break;
+            m = item = nextItem >> a.partShift, part = nextItem & ((1u << a.partShift) - 1u);
+            nextItem += numWarps;
+            if (a.cullBitmap && !((a.cullBitmap[m >> 4] >> (m & 15)) & 1)) continue;
+            if (a.s.alphaList) {
+                const uint32_t mat = *(const uint32_t*)(a.meshlets + (size_t)(a.meshletOffset + m) * kMeshletSize + kOffMaterialId);
+                if (takes_alpha_pass(a.materials, a.numMaterials, mat, a.alphaAll != 0)) {
+                    if (part == 0 && lane == 0) a.s.alphaList[atomicAdd(&a.s.control[9], 1ull)] = item;
+                    continue;
+                }
+            }
+        } else if constexpr (kAlpha) {
             // one item per atomic: alpha-tested meshlets are few and costly (taken four at a time, 12,600 of them
             // left most warps with none: 525 -> 306 us)
             uint32_t idx = 0;
@@ -1024,7 +1041,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
             continue;
         }
         if (nt == 0) continue;
-        nProcessed += nt;
+        if (!kSmall || part == 0) nProcessed += nt;
 
         // ShadeMeshlet vertex loop (Shading.cpp:295-298): 16-vertex chunks up to NumVertices; the
         // slots past them are zero. What the triangles need of a vertex alone is computed here, once
@@ -1077,7 +1094,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                 const uint32_t partial = (c0 | c1 | c2) & 0x3Fu, combined = c0 & c1 & c2 & 0x3Fu;
                 const bool trivial = (c0 & c1 & c2 & kCodeInBand) != 0 && !(partial & 0x30u);
                 const bool accept = accepted && combined == 0, nontriv = accept && !trivial;
-                if (a.countClipped) nClipped += __popc(__ballot_sync(0xFFFFFFFFu, nontriv)) * (lane == 0);
+                if (a.countClipped && (!kSmall || part == 0)) nClipped += __popc(__ballot_sync(0xFFFFFFFFu, nontriv)) * (lane == 0);
                 clip = nontriv && a.clipMode;
                 accepted = accept && trivial;
             }
@@ -1100,9 +1117,10 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
         }
         __syncwarp();
 
-        for (uint32_t base = 0; base < nLive; base += 32) {
-            const bool valid = base + lane < nLive;
-            const uint32_t e = valid ? S.live[base + lane] : 0u;
+        const uint32_t nMine = kSmall ? (nLive + (1u << a.partShift) - 1u - part) >> a.partShift : nLive;
+        for (uint32_t base = 0; base < nMine; base += 32) {
+            const bool valid = base + lane < nMine;
+            const uint32_t e = valid ? S.live[kSmall ? ((base + lane) << a.partShift) + part : base + lane] : 0u;
             const uint32_t i0 = e & 0xFF, i1 = (e >> 8) & 0xFF, i2 = (e >> 16) & 0xFF, p = (e >> 24) & 127u;
             const bool accepted = valid && !(e & 0x80000000u), clipped = valid && (e & 0x80000000u);
 
@@ -1578,7 +1596,7 @@ uint32_t order_stride(uint32_t count) {
 // because draws may come from several host threads.
 static void raise_smem_limit(int pass, const void* kernel, size_t bytes) {
     static std::mutex mu;
-    static size_t setSize[64][5] = {};
+    static size_t setSize[64][6] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
     std::lock_guard<std::mutex> lock(mu);
@@ -1587,6 +1605,7 @@ static void raise_smem_limit(int pass, const void* kernel, size_t bytes) {
         setSize[dev][pass] = bytes;
 }
 
+constexpr uint32_t kMaxPartShift = 5;  // a share of two to four triangles
 void launch_draw(const DrawArgs& args, cudaStream_t st, int numSMs) {
     DrawArgs a = args;
     if (!a.views) {
@@ -1650,7 +1669,13 @@ void launch_draw(const DrawArgs& args, cudaStream_t st, int numSMs) {
     } else {
         {
             LaunchScope ls("k_draw_meshlets", st);
-            k_draw_meshlets<kPassOpaque><<<grid, warps * 32, smem, st>>>(a);
+            if (a.views == nullptr && a.count <= (uint32_t)grid * warps) {
+                if (smem > 48 * 1024) raise_smem_limit(5, (const void*)k_draw_meshlets<kPassOpaque, false, true>, smem);
+                while (a.partShift < kMaxPartShift && (uint64_t)a.count << (a.partShift + 1) <= (uint64_t)grid * warps) a.partShift++;
+                k_draw_meshlets<kPassOpaque, false, true><<<grid, warps * 32, smem, st>>>(a);
+            } else {
+                k_draw_meshlets<kPassOpaque><<<grid, warps * 32, smem, st>>>(a);
+            }
         }
         if (a.s.alphaList) {  // the scene has alpha-tested materials
             opaque_chunks();
