@@ -880,13 +880,27 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
     // Single view: positions per fetch. A draw of fewer meshlets than groups for every warp starts with
     // smaller groups, so that no warp draws several meshlets in a row while others have none.
     const uint32_t leastGroup = totalItems < 2 * numWarps ? 1u : 2u;
-    const uint32_t firstGroup = min(kDrawGroup, max(totalItems / numWarps, leastGroup));
+    // Sparse: of 1024 positions sampled from the cull bitmap fewer than 32 are visible. Groups start at 32 then,
+    // which with the warps' own first groups takes 150,000 positions without a cursor (its contended atomics kept
+    // the warps from their first meshlet for 25,000 cycles and more), and every triangle above kSpreadTiles tiles is
+    // queued, as no other meshlets hide the few visible ones' serial steps: 213 of 150,000 visible, 67.6 -> 42.7 us
+    // (own first groups alone 62, with groups of 32 49); 100,000 mostly visible: no change.
+    uint32_t firstGroup = min(kDrawGroup, max(totalItems / numWarps, leastGroup));
+    bool sparse = false;
+    if (!kSmall && !kAlpha && !multi && a.cullBitmap && totalItems >= 1024) {
+        const unsigned long long words = totalItems >> 4;
+        unsigned seen = 0;
+        for (uint32_t k = 2 * lane; k < 2u * lane + 2; k++) seen += __popc(a.cullBitmap[(uint32_t)((words * k) >> 6)]);
+        sparse = __reduce_add_sync(0xFFFFFFFFu, seen) < 32;
+        if (sparse) firstGroup = 32;
+    }
     uint32_t fetchGroup = firstGroup;
     // Single-view draws walk their positions twice: meshlets large on screen first, then the rest
     // (a second cursor, control[7]), so the costliest work items start early and the last ones
     // are small: a cheaper tail, and near geometry raises the tile depth bounds before the far.
     const bool twoPass = !multi && !kAlpha && !kShaded;
     uint32_t pass = twoPass ? 0u : 1u;
+    bool ownTaken = false;  // a pass's first group is the warp's own, later ones come from the cursor
     // Opaque pass of a scene with alpha-tested materials: a fetched group's alpha-tested meshlets go to the
     // alpha pass's list with one atomic, before their records are read (a draw of alpha-tested meshlets alone:
     // 45 -> 27 us;a shaded meshlet's FragmentShaderId is only known from its
@@ -969,12 +983,17 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                 // the last work items spread evenly over the warps).
                 if (fetchMask == 0) {
                     uint32_t b = 0;
-                    if (lane == 0) b = (uint32_t)atomicAdd(twoPass && pass == 1 ? &a.s.control[7] : cursor,
-                                                           (unsigned long long)fetchGroup);
+                    if (!ownTaken) {
+                        b = (warp * gridDim.x + blockIdx.x) * firstGroup;
+                        ownTaken = true;
+                    } else if (lane == 0) {
+                        b = numWarps * firstGroup + (uint32_t)atomicAdd(twoPass && pass == 1 ? &a.s.control[7] : cursor,
+                                                                        (unsigned long long)fetchGroup);
+                    }
                     const uint32_t base = __shfl_sync(0xFFFFFFFFu, b, 0);
                     if (base >= totalItems) {
                         if (pass == 0) {  // the large meshlets are all taken: the rest from position 0
-                            pass = 1, fetchGroup = firstGroup;
+                            pass = 1, fetchGroup = firstGroup, ownTaken = false;
                             continue;
                         }
                         break;
@@ -1185,8 +1204,8 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
             // the queue, whose chunks spread over all warps of the chunk stage. (Sparser budgets, or
             // a second level once 90 % of the warps are idle, cost the dense frame more than they
             // gain in the sparse one.)
-            bool spread = false;
-            if (__reduce_add_sync(0xFFFFFFFFu, (unsigned)myTiles) > (kAlpha ? kPacketTilesAlpha : kPacketTiles)) {
+            bool spread = sparse;
+            if (!spread && __reduce_add_sync(0xFFFFFFFFu, (unsigned)myTiles) > (kAlpha ? kPacketTilesAlpha : kPacketTiles)) {
                 unsigned long long idle = 0;
                 if (lane == 0) idle = *(volatile unsigned long long*)idleWarps;
                 spread = __shfl_sync(0xFFFFFFFFu, idle, 0) * 2 >= numWarps;

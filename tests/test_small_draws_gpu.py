@@ -50,7 +50,7 @@ def test_counts(scene, part, clipping):
     _check(scene, min(count, 5000), clipping=clipping)
 
 
-@pytest.mark.parametrize("count,offset", [(40, 3000), (700, 100), (4000, 1000)])
+@pytest.mark.parametrize("count,offset", [(40, 3000), (700, 100), (4000, 1000), (5000, 0)])
 @pytest.mark.parametrize("every", [1, 3, 50])
 def test_bitmaps_and_offsets(scene, count, offset, every):
     _check(scene, count, _bitmap(count, every), meshlet_offset=offset)
