@@ -424,6 +424,7 @@ swr_status swr_scene_destroy(swr_scene s) {
     cudaFree(s->meshlets);
     cudaFree(s->materials);
     cudaFree(s->fsIds);
+    cudaFree(s->octTable);
     delete s;
     return SWR_OK;
 }
@@ -436,6 +437,16 @@ swr_status swr_scene_upload_meshlets(swr_scene s, const void* meshlets, uint32_t
                     SWR_MAX_MESHLETS);
     // Records are not inspected on the host (that would cost a cache miss per meshlet); kernels
     // clamp NumVertices to 64 and NumTriangles to 128, the sizes of the record's arrays.
+    // Room is not needed for it (the shading kernels compute what it holds without it).
+    if (!s->octTable && end) {
+        if (cudaMalloc(&s->octTable, kOctTable * sizeof(float4)) == cudaSuccess) {
+            launch_oct_table(s->octTable, t_stream);
+            SWR_CHECK_LAUNCH("swr_scene_upload_meshlets");
+        } else {
+            cudaGetLastError();
+            s->octTable = nullptr;
+        }
+    }
     if (end > s->capacity) {
         uint32_t cap = (uint32_t)std::max<uint64_t>(end, (uint64_t)s->capacity * 3 / 2);
         cap = std::min(cap, SWR_MAX_MESHLETS);

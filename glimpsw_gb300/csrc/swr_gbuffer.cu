@@ -18,6 +18,7 @@ struct GBufferCtx {
     const uint8_t* meshlets;
     const DevMaterial* materials;
     uint32_t numMaterials;
+    const float4* octTable;
     float objectToWorld[9];  // ShadingContext::ObjectToWorldMat (glm::mat3)
 };
 
@@ -60,8 +61,11 @@ struct EncodeGBuffer {
                 const float ty = (float)((nmr >> 8) & 255) * (1.0f / 127.5f) - 1.0f;
                 const float tz = approx_sqrt(1.0f - (tx * tx + ty * ty));
                 F3 n[3], g[3];
+                uint32_t nw[3], gw[3];
 #pragma unroll
-                for (int k = 0; k < 3; k++) unpack_normal_tangent(record_word(rec, kOffNormalTangents, v.VertexId[k]), n[k], g[k]);
+                for (int k = 0; k < 3; k++) nw[k] = record_word(rec, kOffNormalTangents, v.VertexId[k]), gw[k] = nw[k] >> 16;
+                unpack_units(c.octTable, nw, n);
+                unpack_units(c.octTable, gw, g);
                 auto lerp3 = [&](const F3* a) {
                     return F3{ v.Interpolate(a[0].x, a[1].x, a[2].x), v.Interpolate(a[0].y, a[1].y, a[2].y),
                                v.Interpolate(a[0].z, a[1].z, a[2].z) };
@@ -107,6 +111,7 @@ swr_status swr_internal_draw_deferred(swr_rasterizer r, swr_framebuffer fb, uint
     g.meshlets = ctx->scene->meshlets;
     g.materials = ctx->scene->materials;
     g.numMaterials = ctx->scene->num_materials;
+    g.octTable = ctx->scene->octTable;
     memcpy(g.objectToWorld, ctx->object_to_world, sizeof(g.objectToWorld));
     cudaStream_t st = swr_internal_stream();
     {

@@ -228,6 +228,8 @@ void launch_fill(uint32_t* dst, uint32_t n, uint32_t value, cudaStream_t st);
 void launch_finalize(const unsigned long long* keys, uint32_t* layer0, uint32_t* layer1, uint32_t n, cudaStream_t st);
 void launch_finalize_overdraw(const unsigned long long* keys, const unsigned long long* counts, uint32_t* layer0,
                               uint32_t* layer1, uint32_t n, cudaStream_t st);
+constexpr uint32_t kOctTable = 65536;
+void launch_oct_table(float4* table, cudaStream_t st);  // swr_shade.cu
 void launch_detile(const uint32_t* src, const unsigned long long* keys, uint32_t* dst, uint32_t width, uint32_t height,
                    uint32_t stride, uint32_t layer, cudaStream_t st);
 
@@ -282,6 +284,7 @@ struct swr_scene_t {
     bool hasAlpha;                 // some material selects FS_EncodeSurfaceId<true> (swr::material_alpha_tested)
     bool hasAlphaAll;              // some material is alpha-tested under FS_EncodeGBuffer (material_alpha_tested_all)
     uint8_t* fsIds;                // device: FragmentShaderId of each material under ShadeMeshlet
+    float4* octTable;              // device: unmap_oct of every 16-bit normal (with the first meshlets; nullptr: none)
     uint64_t version;              // bumped when meshlets or materials move (recorded draw graphs re-capture)
 };
 

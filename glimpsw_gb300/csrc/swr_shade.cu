@@ -240,6 +240,7 @@ struct ResolveArgs {
     uint32_t numMeshlets;
     const DevMaterial* materials;
     uint32_t numMaterials;
+    const float4* octTable;
     uint32_t* color;        // layer 0 (surface ids in, RGBA8 out)
     float* depth;           // layer 1
     const unsigned long long* keys;  // draws not yet in the layers (nullptr: the layers are up to date)
@@ -345,6 +346,12 @@ __device__ __forceinline__ uint32_t debug_pixel(uint32_t layer, uint32_t data, u
     else if (layer == SWR_DEBUG_OVERDRAW_QUAD) c = colormap_turbo(((float)(data >> 16) + (float)(data & 0xFFFF) * 0.5f) / 30.0f);
     return sat_u8(round2i(c.x * 255.0f)) | (sat_u8(round2i(c.y * 255.0f)) << 8) | (sat_u8(round2i(c.z * 255.0f)) << 16) |
            (255u << 24);
+}
+
+__global__ void k_oct_table(float4* table) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const F3 v = unpack_unit(i);
+    table[i] = make_float4(v.x, v.y, v.z, 0.0f);
 }
 
 // Bound by instruction issue (82 % of the slots; 1080p: 1400 instructions a warp, 90 us; 1600 and 106 us
@@ -607,9 +614,7 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
         }
         }  // !fast
         F3 nrm[3];
-        const float s255 = 1.0f / 255;
-#pragma unroll
-        for (int k = 0; k < 3; k++) nrm[k] = unmap_oct((float)(ntg[k] & 255) * s255, (float)((ntg[k] >> 8) & 255) * s255);
+        unpack_units(a.octTable, ntg, nrm);
         const float* M = a.objectToWorld;
         auto bl = [&](const F3* v) {
             return F3{ fmaf(v[0].x, b[0], fmaf(v[1].x, b[1], v[2].x * b[2])), fmaf(v[0].y, b[0], fmaf(v[1].y, b[1], v[2].y * b[2])),
@@ -623,8 +628,8 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
         F3 N = nws;
         if (__ballot_sync(hm, (nmr & 0xFFFF) != 0) & hm) {
             F3 tan[3];
-#pragma unroll
-            for (int k = 0; k < 3; k++) tan[k] = unmap_oct((float)((ntg[k] >> 16) & 255) * s255, (float)(ntg[k] >> 24) * s255);
+            const uint32_t tw[3] = { ntg[0] >> 16, ntg[1] >> 16, ntg[2] >> 16 };
+            unpack_units(a.octTable, tw, tan);
             const F3 tws = normalize3(m3(bl(tan)));
             F3 bws = { fmaf(nws.y, tws.z, -nws.z * tws.y), fmaf(nws.z, tws.x, -nws.x * tws.z), fmaf(nws.x, tws.y, -nws.y * tws.x) };
             bws = { __uint_as_float(__float_as_uint(bws.x) ^ hand), __uint_as_float(__float_as_uint(bws.y) ^ hand),
@@ -710,6 +715,11 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
 }
 
 }  // namespace
+
+void launch_oct_table(float4* table, cudaStream_t st) {
+    LaunchScope ls("k_oct_table", st);
+    k_oct_table<<<kOctTable / 256, 256, 0, st>>>(table);
+}
 }  // namespace swr
 
 using namespace swr;
@@ -734,6 +744,7 @@ swr_status build_resolve_args(swr_framebuffer fb, const swr_shading_context* ctx
     a.numMeshlets = ctx->scene->count;
     a.materials = ctx->scene->materials;
     a.numMaterials = ctx->scene->num_materials;
+    a.octTable = ctx->scene->octTable;
     a.color = fb->layers;
     a.depth = (float*)(fb->layers + fb->layer_stride);
     a.width = fb->width, a.height = fb->height;
