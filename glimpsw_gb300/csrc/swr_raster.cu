@@ -619,55 +619,57 @@ __device__ __forceinline__ bool raster_region_alpha(const TriRec* rp, const Tile
 }
 
 // ------------------------------------------------------------------ overdraw shader
-// FS_Overdraw (Shading.cpp:333-342) for pixel l of the 4x4 tile at (tx, ty), called by all 32
-// lanes (a half-warp per tile; valid is false on a half without one). DrawTriangle visits the tile
-// only if a sample is covered; then every sample counts, covered ones in the high word of the
-// pixel's counter and the others in the low word, and the tile's 16 depths feed a maximum kept in
-// the key's high word (NaN never replaces: vmaxps keeps the old value).
-__device__ __forceinline__ void shade_tile_pixel_overdraw(const TriRec& r, uint32_t tx, uint32_t ty, bool valid, int lane,
-                                                          unsigned long long* keys, unsigned long long* counts,
-                                                          uint32_t width) {
-    const uint32_t l = lane & 15;
-    const uint32_t px = tx + (l & 3), py = ty + (l >> 2);
-    const int32_t e0 = (int32_t)((uint32_t)r.E0 + (uint32_t)r.A12 * px + (uint32_t)r.B12 * py);
-    const int32_t e1 = (int32_t)((uint32_t)r.E1 + (uint32_t)r.A20 * px + (uint32_t)r.B20 * py);
-    const int32_t e2 = (int32_t)((uint32_t)r.E2 + (uint32_t)r.A01 * px + (uint32_t)r.B01 * py);
-    const bool covered = valid && (e0 | e1 | e2) >= 0;
-    if (!((__ballot_sync(0xFFFFFFFFu, covered) >> (lane & 16)) & 0xFFFFu) || !valid) return;
-    const uint32_t off = (tx << 2) + ty * width + l;
-    atomicAdd(&counts[off], covered ? (1ull << 32) : 1ull);
-    const float depth = ffma(__int2float_rn(e1), r.Z10, ffma(__int2float_rn(e2), r.Z20, r.Z0));
-    if (depth != depth) return;
-    const unsigned long long key = (unsigned long long)float_order(depth) << 32;
-    if (key > *(volatile unsigned long long*)&keys[off]) atomicMax(&keys[off], key);
-}
-
-// shade_live_tiles for the overdraw shader (no depth bounds: every tile a triangle covers counts).
+// FS_Overdraw (Shading.cpp:333-342) over the live tiles of the warp-wide candidate set, packed and stepped as
+// shade_live_tiles does (no depth bounds: every tile a triangle covers counts). DrawTriangle visits a tile
+// only if a sample is covered; then every sample counts, covered ones in the high word of the pixel's counter and
+// the others in the low word, and the tile's 16 depths feed a maximum kept in the key's high word (NaN never
+// replaces: vmaxps keeps the old value). The keys of both tiles of a half-warp are loaded ahead: mesh stage of 20,000
+// meshlets at 1280x720 209 -> 160 us (one tile a half-warp and step 196, a mask walked with shuffles 209), chunk stage
+// 164 -> 146 us with 64 registers (171 with 48, which spill).
 template <class Rec>
 __device__ __forceinline__ void shade_live_tiles_overdraw(Rec&& rec, uint32_t rsel, unsigned mask, uint32_t tpx, uint32_t tpy,
                                                           unsigned long long* keys, unsigned long long* counts,
-                                                          uint32_t width, int lane) {
-    const uint32_t half = lane >> 4;
-    while (mask) {
-        const int s0 = __ffs(mask) - 1;
-        mask &= mask - 1;
-        const int s1 = mask ? __ffs(mask) - 1 : -1;
-        if (s1 >= 0) mask &= mask - 1;
-        const int src = half ? s1 : s0;
-        const uint32_t qx = __shfl_sync(0xFFFFFFFFu, tpx, src & 31);
-        const uint32_t qy = __shfl_sync(0xFFFFFFFFu, tpy, src & 31);
-        const uint32_t qr = __shfl_sync(0xFFFFFFFFu, rsel, src & 31);
-        shade_tile_pixel_overdraw(rec(qr), qx, qy, src >= 0, lane, keys, counts, width);
+                                                          uint32_t width, int lane, uint4* list) {
+    const uint32_t half = lane >> 4, l = lane & 15, m = __popc(mask);
+    if ((mask >> lane) & 1) list[__popc(mask & ((1u << lane) - 1u))] = make_uint4((tpx << 2) + tpy * width, tpx | (tpy << 16), rsel, 0);
+    __syncwarp();
+    auto fetch = [&](uint32_t i, uint4& e, unsigned long long& cur) {
+        e = list[i & 31];
+        cur = i < m ? *(volatile unsigned long long*)&keys[e.x + l] : 0ull;
+    };
+    auto shade = [&](uint32_t i, const uint4& e, unsigned long long cur) {
+        const bool valid = i < m;
+        const TriRec& r = rec(valid ? e.z : 0u);
+        const uint32_t px = (e.y & 0xFFFF) + (l & 3), py = (e.y >> 16) + (l >> 2);
+        const int32_t e0 = (int32_t)((uint32_t)r.E0 + (uint32_t)r.A12 * px + (uint32_t)r.B12 * py);
+        const int32_t e1 = (int32_t)((uint32_t)r.E1 + (uint32_t)r.A20 * px + (uint32_t)r.B20 * py);
+        const int32_t e2 = (int32_t)((uint32_t)r.E2 + (uint32_t)r.A01 * px + (uint32_t)r.B01 * py);
+        const bool covered = valid && (e0 | e1 | e2) >= 0;
+        if (!((__ballot_sync(0xFFFFFFFFu, covered) >> (lane & 16)) & 0xFFFFu)) return;
+        atomicAdd(&counts[e.x + l], covered ? (1ull << 32) : 1ull);
+        const float depth = ffma(__int2float_rn(e1), r.Z10, ffma(__int2float_rn(e2), r.Z20, r.Z0));
+        const unsigned long long key = (unsigned long long)float_order(depth) << 32;
+        if (depth == depth && key > cur) atomicMax(&keys[e.x + l], key);
+    };
+    for (uint32_t i = half; i - half < m; i += 4) {
+        uint4 a, b;
+        unsigned long long ca, cb;
+        fetch(i, a, ca);
+        fetch(i + 2, b, cb);
+        shade(i, a, ca);
+        __syncwarp();
+        shade(i + 2, b, cb);
+        __syncwarp();
     }
 }
 
 __device__ __forceinline__ bool raster_region_overdraw(const TriRec& r, const TileTest& tt, uint32_t x0, uint32_t y0, int tilesX, int tilesY,
                                                        unsigned long long* keys, unsigned long long* counts,
-                                                       uint32_t width, int lane, uint32_t divMagic = 0) {
+                                                       uint32_t width, int lane, uint4* list, uint32_t divMagic = 0) {
     return raster_region_with(r, tt, x0, y0, tilesX, tilesY, nullptr, width, lane,
                        [&](unsigned mask, uint32_t tpx, uint32_t tpy, uint32_t) {
                            shade_live_tiles_overdraw([&](uint32_t) -> const TriRec& { return r; }, 0, mask, tpx, tpy, keys,
-                                                     counts, width, lane);
+                                                     counts, width, lane, list);
                        }, divMagic);
 }
 
@@ -1274,7 +1276,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                                            lane, list);
                 } else if constexpr (kOver) {
                     shade_live_tiles_overdraw([&](uint32_t q) -> const TriRec& { return tris[q].v; }, own, liveMask, tpx, tpy,
-                                              vp.keys, a.counts, vp.width, lane);
+                                              vp.keys, a.counts, vp.width, lane, list);
                 } else {
                     shade_live_tiles([&](uint32_t q) -> const TriRec& { return tris[q].v; },
                                      [&](uint32_t q) { return (tris[q].v.pad & kPadReadKey) != 0u; }, own, liveMask, tpx, tpy,
@@ -1390,7 +1392,7 @@ __device__ __forceinline__ bool raster_chunk_alpha(const TriRec* q, const DevMat
 // the other's; 48 and 64 registers hold 40 and 32 warps per SM: chunk stages of the alpha-tested frame 459 ->
 // 404 us).
 template <bool kOver, bool kAlpha>
-__global__ void __launch_bounds__(256, kAlpha ? 4 : 5) k_raster_big(const TriRec* __restrict__ big, const unsigned long long* __restrict__ bigBase,
+__global__ void __launch_bounds__(256, kAlpha || kOver ? 4 : 5) k_raster_big(const TriRec* __restrict__ big, const unsigned long long* __restrict__ bigBase,
                                                     unsigned long long* control, uint32_t capacity,
                                                     unsigned long long* keys, uint32_t* tileMin, uint32_t width, uint32_t height,
                                                     const ViewParams* __restrict__ views, uint32_t chunk,
@@ -1478,7 +1480,7 @@ __global__ void __launch_bounds__(256, kAlpha ? 4 : 5) k_raster_big(const TriRec
                 vkeys = v.keys, vtiles = v.tileMin, vw = v.width, vh = v.height;
             }
             if constexpr (kOver) {
-                raster_region_overdraw(r, tile_test(r), x0, y0, tilesX, tilesY, vkeys, counts, vw, lane, kDiv16[tilesX]);
+                raster_region_overdraw(r, tile_test(r), x0, y0, tilesX, tilesY, vkeys, counts, vw, lane, list[threadIdx.x >> 5], kDiv16[tilesX]);
             } else {
                 bool any;
                 if (kAlpha && (r.pad & kTriAlpha))
