@@ -940,9 +940,12 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
         } else if constexpr (kAlpha) {
             // one item per atomic: alpha-tested meshlets are few and costly (taken four at a time, 12,600 of them
             // left most warps with none: 525 -> 306 us)
-            uint32_t idx = 0;
-            if (lane == 0) idx = (uint32_t)atomicAdd(cursor, 1ull);
-            idx = __shfl_sync(0xFFFFFFFFu, idx, 0);
+            uint32_t idx = warp * gridDim.x + blockIdx.x;  // the first by the warp's index
+            if (ownTaken) {
+                if (lane == 0) idx = numWarps + (uint32_t)atomicAdd(cursor, 1ull);
+                idx = __shfl_sync(0xFFFFFFFFu, idx, 0);
+            }
+            ownTaken = true;
             if (idx >= totalItems) break;
             item = a.s.alphaList[idx];
             m = item;
@@ -1314,7 +1317,11 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
 // With alpha-tested materials runs of 4: their live chunks cost about five times more (2, 4 and 8: 405, 363 and
 // 432 us of chunk stage inside a 50k-meshlet scene).
 constexpr uint32_t kChunkRun = 8, kChunkRunAlpha = 4;
-constexpr uint32_t kRunsPerWarp = 4;  // a shorter run when the queue holds fewer chunks than this many runs a warp
+// A shorter run when the queue holds fewer chunks than this many runs a warp, but two chunks while it holds one run a
+// warp of them: the queue's first chunks, those of the nearest triangles, cost the most (runs by 4 / 6 / 8 a warp:
+// 142 / 137 / 123 us of opaque chunk stage inside a 50k-meshlet scene; one chunk a run instead of two 93 against
+// 80 us in a sparse 2560x1440 draw, by the cursor's atomics).
+constexpr uint32_t kRunsPerWarp = 8;
 
 // Per 32x32-pixel block, a lower bound of the tile depth bounds inside it, in the words after the tile
 // bounds (tile_bounds_words): one load tells a chunk's lane that the whole block is nearer. The bounds are
@@ -1412,11 +1419,17 @@ __global__ void __launch_bounds__(256, kAlpha || kOver ? 4 : 5) k_raster_big(con
     const unsigned long long total = bigBase[n - 1] + (unsigned long long)((lastTX + cw - 1) / cw) * ((lastTY + ch - 1) / ch);
     // a sparse queue (few big triangles) is spread with shorter runs so that every warp gets work
     const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-    const uint32_t run = (uint32_t)max(1ull, min((unsigned long long)maxRun, total / (warps * kRunsPerWarp)));
-    while (true) {
-        unsigned long long w0 = 0;
-        if (lane == 0) w0 = atomicAdd(&control[8], (unsigned long long)run);
-        w0 = __shfl_sync(0xFFFFFFFFu, w0, 0);
+    const unsigned long long share = total / (warps * kRunsPerWarp);
+    const uint32_t run = (uint32_t)max(share ? 2ull : 1ull, min((unsigned long long)maxRun, share));
+    // The warp's first run is its own by its index (blocks first: the queue starts with near geometry), later ones
+    // come from the cursor; every warp of the grid is resident. (All warps at the cursor at once: 17.5 -> 15.2 us at
+    // 1280x720, 93 -> 80 us in the sparse draw, with the run rule 233 -> 223 us for 24 batched views.)
+    unsigned long long w0 = ((unsigned long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * run;
+    for (bool own = true;; own = false) {
+        if (!own) {
+            if (lane == 0) w0 = warps * run + atomicAdd(&control[8], (unsigned long long)run);
+            w0 = __shfl_sync(0xFFFFFFFFu, w0, 0);
+        }
         if (w0 >= total) break;
         // the largest slot with bigBase[slot] <= w0: 32 probes a step
         uint32_t slot = 0, hi = n - 1;
@@ -1651,7 +1664,7 @@ void launch_draw(const DrawArgs& args, cudaStream_t st, int numSMs) {
             k_draw_meshlets<kPassOverdraw><<<grid, warps * 32, smem, st>>>(a);
         }
         LaunchScope ls("k_raster_big_overdraw", st);
-        k_raster_big<true, false><<<numSMs * 8, 256, 0, st>>>(a.s.big, a.s.bigBase, a.s.control, a.s.bigCapacity, a.keys, nullptr,
+        k_raster_big<true, false><<<numSMs * 4, 256, 0, st>>>(a.s.big, a.s.bigBase, a.s.control, a.s.bigCapacity, a.keys, nullptr,
                                                        a.width, a.height, a.views, chunk, a.materials, a.counts, 0u, kChunkRun,
                                                               true);
         return;
@@ -1663,7 +1676,7 @@ void launch_draw(const DrawArgs& args, cudaStream_t st, int numSMs) {
                                                                   a.tileMin, a.width, a.height, a.views, chunk, a.materials,
                                                                   nullptr, a.keyReadTiles, kChunkRunAlpha, true);
         else
-            k_raster_big<false, false><<<numSMs * 8, 256, 0, st>>>(a.s.big, a.s.bigBase, a.s.control, a.s.bigCapacity, a.keys,
+            k_raster_big<false, false><<<numSMs * 5, 256, 0, st>>>(a.s.big, a.s.bigBase, a.s.control, a.s.bigCapacity, a.keys,
                                                                    a.tileMin, a.width, a.height, a.views, chunk, a.materials,
                                                                    nullptr, a.keyReadTiles, kChunkRun, last);
     };
