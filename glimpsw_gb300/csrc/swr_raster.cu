@@ -826,6 +826,35 @@ __device__ __forceinline__ uint32_t view_of(const uint32_t* viewStart, uint32_t 
     return lo;
 }
 
+// A block's pool of meshlets that a fetched group held beyond the one its warp draws next: any warp of the block
+// takes them before it fetches another group, and a warp that gives takes until the pool is empty before it ends, so
+// none is left. Where groups hold several visible meshlets some warps used to draw three or four in a row, 20,000 to
+// 100,000 cycles each, while the median warp was done (at 0.27 of the kernel's time inside a 50k-meshlet scene, 0.35
+// in a G-buffer draw of 30k): mesh stage 160 -> 124 us and 184 -> 142 us there, 234 -> 185 in a draw of 60k meshlets
+// at 2560x1440, 357 -> 342 of 100k at 1920x1080, 1281 -> 1244 for 24 batched views (all but the first meshlet of a
+// group given; all but three 1250, all but eight 1290).
+constexpr uint32_t kPoolSlots = 64, kPoolFree = 0xFFFFFFFFu;
+static_assert(SWR_MAX_MESHLETS <= 1u << 21, "a pool's word");
+__device__ __forceinline__ uint32_t pool_take(uint32_t* pool, int lane) {
+    const uint32_t s0 = ((volatile uint32_t*)pool)[lane], s1 = ((volatile uint32_t*)pool)[32 + lane];
+    uint32_t taken = kPoolFree;
+    for (unsigned any = __ballot_sync(0xFFFFFFFFu, s0 != kPoolFree || s1 != kPoolFree); any && taken == kPoolFree; any &= any - 1) {
+        const int src = __ffs(any) - 1;
+        if (lane == src) taken = atomicExch(&pool[s0 != kPoolFree ? lane : 32 + lane], kPoolFree);
+        taken = __shfl_sync(0xFFFFFFFFu, taken, src);
+    }
+    return taken;
+}
+// Gives the lanes of mask but the first, as far as their slots are free; returns the lanes kept.
+__device__ __forceinline__ unsigned pool_give(uint32_t* pool, unsigned mask, uint32_t item, int lane, int warp) {
+    bool given = false;
+    if (((mask & (mask - 1)) >> lane) & 1) {
+        const uint32_t slot = (lane + 8 * warp) & (kPoolSlots - 1);
+        given = atomicCAS(&pool[slot], kPoolFree, item) == kPoolFree || atomicCAS(&pool[slot ^ 32], kPoolFree, item) == kPoolFree;
+    }
+    return mask & ~__ballot_sync(0xFFFFFFFFu, given);
+}
+
 enum : int { kPassOpaque = 0, kPassAlpha = 1, kPassOverdraw = 2 };
 // kShaded: the meshlets come shaded by a user mesh shader (a.shaded, swr_shaded_meshlet records):
 // clip positions, indices, PrimCount, CullMode and FragmentShaderId are read from the record
@@ -902,6 +931,10 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
     // are small: a cheaper tail, and near geometry raises the tile depth bounds before the far.
     const bool twoPass = !multi && !kAlpha && !kShaded;
     uint32_t pass = twoPass ? 0u : 1u;
+    // 2^partShift warps share a meshlet: small draws, and an alpha pass of few meshlets for its warps (a G-buffer draw's
+    // 10,000 by two: 143 -> 128 us; by four 128, and 7,200 of another 84 instead of 72 us).
+    constexpr bool kParts = kSmall || kAlpha;
+    const uint32_t partShift = kSmall ? a.partShift : kAlpha ? (totalItems < numWarps ? 2u : totalItems < 4 * numWarps ? 1u : 0u) : 0u;
     bool ownTaken = false;  // a pass's first group is the warp's own, later ones come from the cursor
     // Opaque pass of a scene with alpha-tested materials: a fetched group's alpha-tested meshlets go to the
     // alpha pass's list with one atomic, before their records are read (a draw of alpha-tested meshlets alone:
@@ -922,12 +955,18 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
         if (alpha) a.s.alphaList[at + __popc(am & ((1u << lane) - 1u))] = item;
         return mask & ~am;
     };
+    constexpr bool kPool = !kAlpha && !kSmall && !kOver;  // (the overdraw shader's pass loses by it, 159 -> 169 us)
+    __shared__ uint32_t pool[kPool ? kPoolSlots : 1];
+    if constexpr (kPool) {
+        if (threadIdx.x < kPoolSlots) pool[threadIdx.x] = kPoolFree;
+        __syncthreads();
+    }
     uint32_t nextItem = warp * gridDim.x + blockIdx.x;  // kSmall: blocks first, so that all SMs get some
     while (true) {
         uint32_t m, view = 0, item, part = 0;
         if constexpr (kSmall) {
-            if (nextItem >= totalItems << a.partShift) break;
-            m = item = nextItem >> a.partShift, part = nextItem & ((1u << a.partShift) - 1u);
+            if (nextItem >= totalItems << partShift) break;
+            m = item = nextItem >> partShift, part = nextItem & ((1u << partShift) - 1u);
             nextItem += numWarps;
             if (a.cullBitmap && !((a.cullBitmap[m >> 4] >> (m & 15)) & 1)) continue;
             if (a.s.alphaList) {
@@ -946,8 +985,9 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                 idx = __shfl_sync(0xFFFFFFFFu, idx, 0);
             }
             ownTaken = true;
-            if (idx >= totalItems) break;
-            item = a.s.alphaList[idx];
+            if (idx >= totalItems << partShift) break;
+            part = idx & ((1u << partShift) - 1u);
+            item = a.s.alphaList[idx >> partShift];
             m = item;
             if (multi) {
                 view = view_of(a.viewStart, a.numViews, item);
@@ -955,7 +995,11 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
             }
         } else {
             if (multi) {
-                if (fetchMask == 0) {
+                uint32_t taken = kPoolFree;
+                if (kPool && fetchMask == 0) {
+                    taken = pool_take(pool, lane);
+                }
+                if (taken == kPoolFree && fetchMask == 0) {
                     uint32_t b = 0;
                     if (lane == 0) b = (uint32_t)atomicAdd(cursor, (unsigned long long)kBatchGroup);
                     const uint32_t base = __shfl_sync(0xFFFFFFFFu, b, 0);
@@ -975,10 +1019,16 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                         fetchMask = split_alpha(fetchMask, fv.meshletOffset + laneMeshlet, a.viewStart[fetchView] + laneMeshlet);
                         if (fetchMask == 0) continue;
                     }
+                    // as a pool's word holds a view of up to 2046 and a meshlet
+                    if (kPool && a.numViews < 2047) fetchMask = pool_give(pool, fetchMask, fetchView << 21 | laneMeshlet, lane, warp);
                 }
-                view = fetchView;
-                m = __shfl_sync(0xFFFFFFFFu, laneMeshlet, __ffs(fetchMask) - 1);
-                fetchMask &= fetchMask - 1;
+                if (taken != kPoolFree) {
+                    view = taken >> 21, m = taken & 0x1FFFFFu;
+                } else {
+                    view = fetchView;
+                    m = __shfl_sync(0xFFFFFFFFu, laneMeshlet, __ffs(fetchMask) - 1);
+                    fetchMask &= fetchMask - 1;
+                }
                 item = a.viewStart[view] + m;
             } else {
                 // Single view: groups of fetchGroup positions (2 to 32), their cull bits tested at
@@ -986,7 +1036,11 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                 // sparse view fetches 32 positions per atomic) and shrinks while they hold more than
                 // one visible meshlet (a dense view fetches about one visible meshlet at a time, so
                 // the last work items spread evenly over the warps).
-                if (fetchMask == 0) {
+                uint32_t taken = kPoolFree;
+                if (kPool && fetchMask == 0) {
+                    taken = pool_take(pool, lane);
+                }
+                if (taken == kPoolFree && fetchMask == 0) {
                     uint32_t b = 0;
                     if (!ownTaken) {
                         b = (warp * gridDim.x + blockIdx.x) * firstGroup;
@@ -1019,9 +1073,14 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                     const int got = __popc(fetchMask);
                     fetchGroup = got == 0 ? min(fetchGroup * 2, 32u) : (got > 1 ? max(fetchGroup / 2, leastGroup) : fetchGroup);
                     if (fetchMask == 0) continue;
+                    if constexpr (kPool) fetchMask = pool_give(pool, fetchMask, laneMeshlet, lane, warp);
                 }
-                m = __shfl_sync(0xFFFFFFFFu, laneMeshlet, __ffs(fetchMask) - 1);
-                fetchMask &= fetchMask - 1;
+                if (taken != kPoolFree) {
+                    m = taken;
+                } else {
+                    m = __shfl_sync(0xFFFFFFFFu, laneMeshlet, __ffs(fetchMask) - 1);
+                    fetchMask &= fetchMask - 1;
+                }
                 item = m;
             }
         }
@@ -1065,7 +1124,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
             continue;
         }
         if (nt == 0) continue;
-        if (!kSmall || part == 0) nProcessed += nt;
+        if (!kParts || part == 0) nProcessed += nt;
 
         // ShadeMeshlet vertex loop (Shading.cpp:295-298): 16-vertex chunks up to NumVertices; the
         // slots past them are zero. What the triangles need of a vertex alone is computed here, once
@@ -1118,15 +1177,18 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                 const uint32_t partial = (c0 | c1 | c2) & 0x3Fu, combined = c0 & c1 & c2 & 0x3Fu;
                 const bool trivial = (c0 & c1 & c2 & kCodeInBand) != 0 && !(partial & 0x30u);
                 const bool accept = accepted && combined == 0, nontriv = accept && !trivial;
-                if (a.countClipped && (!kSmall || part == 0)) nClipped += __popc(__ballot_sync(0xFFFFFFFFu, nontriv)) * (lane == 0);
+                if (a.countClipped && (!kParts || part == 0)) nClipped += __popc(__ballot_sync(0xFFFFFFFFu, nontriv)) * (lane == 0);
                 clip = nontriv && a.clipMode;
                 accepted = accept && trivial;
             }
             const float2 q0 = S.xy[i0], q1 = S.xy[i1], q2 = S.xy[i2];
             const bool live = clip || (accepted && front_facing({ q0.x, q0.y, 0.0f, 0.0f }, { q1.x, q1.y, 0.0f, 0.0f },
                                                                 { q2.x, q2.y, 0.0f, 0.0f }, cullMode));
-            if (kAlpha && hidden) {  // counted alone
-                if (live) {
+            const unsigned liveMask = __ballot_sync(0xFFFFFFFFu, live);
+            if (kAlpha && hidden) {  // counted alone: the warp's share, as another warp of the meshlet may not find it hidden
+                const uint32_t at = nLive + __popc(liveMask & ((1u << lane) - 1u));
+                nLive += __popc(liveMask);
+                if (live && (at & ((1u << partShift) - 1u)) == part) {
                     Setup t;
                     t.Pos0 = S.pz[i0].x, t.Pos1 = S.pz[i1].x, t.Pos2 = S.pz[i2].x;
                     uint32_t bbMin, bbMax;
@@ -1135,16 +1197,16 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                 }
                 continue;
             }
-            const unsigned liveMask = __ballot_sync(0xFFFFFFFFu, live);
             if (live) S.live[nLive + __popc(liveMask & ((1u << lane) - 1u))] = i0 | (i1 << 8) | (i2 << 16) | (p << 24) | (clip ? 0x80000000u : 0u);
             nLive += __popc(liveMask);
         }
         __syncwarp();
 
-        const uint32_t nMine = kSmall ? (nLive + (1u << a.partShift) - 1u - part) >> a.partShift : nLive;
+        if (kAlpha && hidden) continue;
+        const uint32_t nMine = kParts ? (nLive + (1u << partShift) - 1u - part) >> partShift : nLive;
         for (uint32_t base = 0; base < nMine; base += 32) {
             const bool valid = base + lane < nMine;
-            const uint32_t e = valid ? S.live[kSmall ? ((base + lane) << a.partShift) + part : base + lane] : 0u;
+            const uint32_t e = valid ? S.live[kParts ? ((base + lane) << partShift) + part : base + lane] : 0u;
             const uint32_t i0 = e & 0xFF, i1 = (e >> 8) & 0xFF, i2 = (e >> 16) & 0xFF, p = (e >> 24) & 127u;
             const bool accepted = valid && !(e & 0x80000000u), clipped = valid && (e & 0x80000000u);
 
