@@ -38,3 +38,18 @@ def test_irradiance_and_radiance(w, h):
         n = 8 >> level
         got = [data[rad.mip_offsets[level] + ((y & 7) | (x << 3))] for y in range(n) for x in range(n)]
         assert got == [O.ibl_radiance_texel(o, level, rad.mip_levels, x, y, 8, 8) for y in range(n) for x in range(n)]
+
+
+@pytest.mark.parametrize("w,h", [(8, 4), (16, 8), (32, 16), (64, 32)])
+def test_brdf_table_sizes(w, h):
+    """Blocks of 32 texels over several rows (a narrow table) and over one."""
+    from glimpsw_gb300 import api
+    from oracle import oracle as O
+    api.load_library()
+    out = api.Texture2D(api.FORMAT_RG16F, w, h, 1, 1)
+    api._check(api._lib.swr_ibl_env_brdf_lut(out.h))
+    data = out.get_data()
+    stride = max(w, 8).bit_length() - 1
+    got = np.array([[data[(y & 7) | (x << 3) | ((y & ~7) << stride)] for x in range(w)] for y in range(h)], np.uint32)
+    exp = np.array([[O.ibl_env_brdf_texel(x, y, w, h) for x in range(w)] for y in range(h)], np.uint32)
+    assert np.array_equal(got, exp)
