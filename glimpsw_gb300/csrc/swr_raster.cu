@@ -958,7 +958,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
     constexpr bool kPool = !kAlpha && !kSmall && !kOver;  // (the overdraw shader's pass loses by it, 159 -> 169 us)
     __shared__ uint32_t pool[kPool ? kPoolSlots : 1];
     if constexpr (kPool) {
-        if (threadIdx.x < kPoolSlots) pool[threadIdx.x] = kPoolFree;
+        for (uint32_t k = threadIdx.x; k < kPoolSlots; k += blockDim.x) pool[k] = kPoolFree;
         __syncthreads();
     }
     uint32_t nextItem = warp * gridDim.x + blockIdx.x;  // kSmall: blocks first, so that all SMs get some
