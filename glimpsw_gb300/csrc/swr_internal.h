@@ -206,7 +206,7 @@ constexpr uint32_t kShadedSize = 1472, kShadedIndices = 64, kShadedPositions = 4
 // contend for the same pixels' keys. Keys are order-independent, so the image is the same for
 // every order. Work is fetched kBatchGroup positions at a time in batches (whose views' position
 // ranges are padded to multiples of it); single-view draws start at kDrawGroup positions and adapt
-// the group to the share of visible meshlets, and the alpha pass takes kDrawGroup list entries.
+// the group to the share of visible meshlets, and the alpha pass takes list entries one by one.
 constexpr uint32_t kDrawGroup = 4, kBatchGroup = 32;
 uint32_t order_stride(uint32_t count);
 // Meshlet drawn at position p of a view of count meshlets (order_stride).

@@ -3,16 +3,18 @@
 // FS_EncodeSurfaceId<true>) for sm_103a.
 //
 // Work decomposition:
-//   k_draw_meshlets  one warp per meshlet (dynamic fetch). Lanes transform the 64 vertices into
-//                    shared memory, then own one triangle each: clip codes, setup and edge
-//                    equations in registers. Triangles whose 4-aligned box covers at most
-//                    kSmallTiles 4x4 tiles are rasterized by the whole warp, two tiles (32 pixels)
-//                    per step; larger and clipped triangles, and every triangle of an
-//                    alpha-tested material, go to a device queue.
-//   k_raster_big     warps take 32x32-pixel chunks of queued triangles (flattened by a prefix of
-//                    chunk counts kept in the queue), reject empty chunks by their corners and
-//                    rasterize the rest two tiles per step.
-//   k_finalize       converts per-pixel keys to the reference's depth and surfaceId layers.
+//   k_draw_meshlets  one warp per meshlet (dynamic fetch, a block's warps sharing fetched groups), or several
+//                    in small draws. Lanes transform the 64 vertices into shared memory and test the
+//                    faces, then own one of the remaining triangles each: setup and edge equations
+//                    in registers. Triangles whose 4-aligned box covers at most kSmallTiles 4x4
+//                    tiles are rasterized by the whole warp, four tiles (64 pixels) per step, those
+//                    of at most two samples by their lane; larger and clipped triangles go to a device
+//                    queue. Alpha-tested meshlets are drawn by a pass of their own.
+//   k_raster_big     warps take runs of 32x32-pixel chunks of queued triangles (flattened by a prefix of
+//                    chunk counts kept in the queue), reject empty and hidden chunks one per lane
+//                    and rasterize the rest four tiles per step.
+//   k_finalize       converts per-pixel keys to the reference's depth and surfaceId layers, for readers of
+//                    the layers that do not take the keys themselves.
 // The depth test is a 64-bit atomicMax on (ordered depth, 0xFFFFFFFE - rank); the result is
 // independent of execution order and equals the single-threaded reference. The alpha test is a
 // function of the triangle and the fragment alone, so it only removes fragments and keeps that
