@@ -810,12 +810,12 @@ __global__ void __launch_bounds__(1024) k_neural_offsets(const uint32_t* counts,
     if (t == n - 1) reqOffset[n] = sr[t], tileOffset[n] = st[t];
 }
 
-// Groups the per-pixel requests (material<<32 | level<<28 | ty<<14 | tx, or ~0) by material. A
-// block takes kScatterSlots consecutive slots: shared-memory counters rank each request among the
-// block's requests of its material, then one global atomic per (block, material) reserves the
+// Groups the requests of the pixels' records (the second plane of the emit pass's, swr_shade.cu) by material. A
+// thread takes a pixel, whose four slots it decodes itself where it leads them; shared-memory counters rank each
+// request among the block's requests of its material, then one global atomic per (block, material) reserves the
 // block's run in that material's list (the per-material cursors see few, uncontended atomics).
-constexpr uint32_t kScatterThreads = 256, kScatterPerThread = 4, kScatterSlots = kScatterThreads * kScatterPerThread;
-__global__ void __launch_bounds__(kScatterThreads) k_neural_scatter(const unsigned long long* pixelReq, uint32_t slots,
+constexpr uint32_t kScatterThreads = 256;
+__global__ void __launch_bounds__(kScatterThreads) k_neural_scatter(const uint4* __restrict__ records, uint32_t pixels,
                                                                     const uint32_t* reqOffset, uint32_t* cursor,
                                                                     unsigned long long* sorted, uint32_t* levelCount,
                                                                     uint32_t numMaterials) {
@@ -826,18 +826,18 @@ __global__ void __launch_bounds__(kScatterThreads) k_neural_scatter(const unsign
     for (uint32_t m = threadIdx.x; m < numMaterials; m += kScatterThreads) sCount[m] = 0;
     if (threadIdx.x < kNeuralMaxDecoded) sLevel[threadIdx.x] = 0;
     __syncthreads();
-    const uint32_t first = blockIdx.x * kScatterSlots + threadIdx.x;
-    unsigned long long r[kScatterPerThread];
-    uint32_t rank[kScatterPerThread];
+    const uint32_t p = blockIdx.x * kScatterThreads + threadIdx.x;
+    const uint4 rec = p < pixels ? records[p] : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t mat = rec.w & 0xFFFFu;
+    uint32_t own = 0, rank[4];
+    if (rec.y & kSurfDecoded) {
 #pragma unroll
-    for (uint32_t k = 0; k < kScatterPerThread; k++) {  // slot first + k * 256: coalesced loads
-        const uint32_t i = first + k * kScatterThreads;
-        r[k] = i < slots ? pixelReq[i] : ~0ull;
-        if (r[k] >> 63) r[k] = ~0ull;  // none, or a redirect to another slot's request
-        if (r[k] != ~0ull) {
-            rank[k] = atomicAdd(&sCount[(uint32_t)(r[k] >> 32)], 1u);
-            atomicAdd(&sLevel[((uint32_t)r[k] >> 28) & 15u], 1u);
+        for (uint32_t k = 0; k < 4; k++) {
+            if (!surf_has_slot(rec.y, k) || ((rec.w >> (16 + 4 * k)) & 15u) != (p & 15u)) continue;
+            own |= 1u << k;
+            rank[k] = atomicAdd(&sCount[mat], 1u);
         }
+        if (own) atomicAdd(&sLevel[rec.z >> 28], (uint32_t)__popc(own));
     }
     __syncthreads();
     for (uint32_t m = threadIdx.x; m < numMaterials; m += kScatterThreads)
@@ -845,11 +845,8 @@ __global__ void __launch_bounds__(kScatterThreads) k_neural_scatter(const unsign
     if (threadIdx.x < kNeuralMaxDecoded && sLevel[threadIdx.x]) atomicAdd(&levelCount[threadIdx.x], sLevel[threadIdx.x]);
     __syncthreads();
 #pragma unroll
-    for (uint32_t k = 0; k < kScatterPerThread; k++) {
-        if (r[k] == ~0ull) continue;
-        const uint32_t i = first + k * kScatterThreads;
-        sorted[sBase[(uint32_t)(r[k] >> 32)] + rank[k]] = ((unsigned long long)i << 32) | (uint32_t)r[k];
-    }
+    for (uint32_t k = 0; k < 4; k++)
+        if ((own >> k) & 1) sorted[sBase[mat] + rank[k]] = ((unsigned long long)(p * 4 + k) << 32) | surf_slot_texel(rec.z, k);
 }
 
 }  // namespace
@@ -938,10 +935,10 @@ void launch_neural_offsets(const uint32_t* counts, uint32_t* reqOffset, uint32_t
                            cudaStream_t st) {
     k_neural_offsets<<<1, 1024, 0, st>>>(counts, reqOffset, tileOffset, numMaterials);
 }
-void launch_neural_scatter(const unsigned long long* pixelReq, uint32_t slots, const uint32_t* reqOffset, uint32_t* cursor,
+void launch_neural_scatter(const uint4* records, uint32_t pixels, const uint32_t* reqOffset, uint32_t* cursor,
                            unsigned long long* sorted, uint32_t* levelCount, uint32_t numMaterials, cudaStream_t st) {
-    k_neural_scatter<<<(slots + kScatterSlots - 1) / kScatterSlots, kScatterThreads, 2 * numMaterials * sizeof(uint32_t), st>>>(
-        pixelReq, slots, reqOffset, cursor, sorted, levelCount, numMaterials);
+    k_neural_scatter<<<(pixels + kScatterThreads - 1) / kScatterThreads, kScatterThreads, 2 * numMaterials * sizeof(uint32_t), st>>>(
+        records, pixels, reqOffset, cursor, sorted, levelCount, numMaterials);
 }
 
 }  // namespace swr

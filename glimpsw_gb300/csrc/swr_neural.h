@@ -108,9 +108,21 @@ void launch_neural_export(const float* latent, uint16_t* half, size_t count, cud
 void launch_wait_selftest(uint32_t* status, uint64_t limitNs, cudaStream_t st);
 void launch_neural_offsets(const uint32_t* counts, uint32_t* reqOffset, uint32_t* tileOffset, uint32_t numMaterials,
                            cudaStream_t st);
-void launch_neural_scatter(const unsigned long long* pixelReq, uint32_t slots, const uint32_t* reqOffset,
-                           uint32_t* cursor, unsigned long long* sorted, uint32_t* levelCount, uint32_t numMaterials,
-                           cudaStream_t st);
+// Flags of the neural resolve's pixel records (swr_shade.cu); the filter weights are in bits 8 to 23.
+enum : uint32_t {
+    kSurfFast = 1u,        // sampled from decoded texels, or untextured (albedo and NMR 0)
+    kSurfDecoded = 2u,     // a decoded material sample: fetch it
+    kSurfNearest = 4u, kSurfInX = 8u, kSurfInY = 16u, kSurfTwoLayers = 32u,
+    kSurfHand = 1u << 31,  // the bitangent's sign bit
+};
+// Whether a decoded sample needs the texel of slot k (00 10 01 11), and which it is.
+__host__ __device__ inline bool surf_has_slot(uint32_t flags, uint32_t k) {
+    return k == 0 || (!(flags & kSurfNearest) && (!(k & 1) || (flags & kSurfInX)) && (!(k & 2) || (flags & kSurfInY)));
+}
+__host__ __device__ inline uint32_t surf_slot_texel(uint32_t first, uint32_t k) { return first + (k & 1) + ((k >> 1) << 14); }
+// records: the second plane of the pixels' records.
+void launch_neural_scatter(const uint4* records, uint32_t pixels, const uint32_t* reqOffset, uint32_t* cursor,
+                           unsigned long long* sorted, uint32_t* levelCount, uint32_t numMaterials, cudaStream_t st);
 
 }  // namespace swr
 
@@ -138,10 +150,9 @@ struct swr_neural_t {
     uint32_t trainCalls;
     bool halfStale;                          // latentHalf behind the master copy
     // neural resolve scratch (grow-only)
-    unsigned long long* pixelReq;
     unsigned long long* sorted;
     uint2* decoded;
-    uint4* surf;                             // two words per pixel: the emit pass's surface records
+    uint4* surf;                             // two planes of a word per pixel: the emit pass's surface records
     size_t scratchSlots;
     uint32_t* counters;                      // counts | cursors | reqOffset | tileOffset, numMaterials+1 each,
                                              // then 4 per-level request counts

@@ -258,31 +258,28 @@ struct ResolveArgs {
     uint32_t debugLayer;    // SWR_DEBUG_* of the debug mode
 };
 
-// Neural resolve: the emit pass records, per pixel, the texels of the levels the model decodes
-// (4 slots: the nearest texel, or the bilinear quad's 00 10 01 11 texels; ~0 = none) and counts
-// them per material; the shade pass reads the decoded texels from the same slots. Within a 4x4
-// tile, a slot whose texel a lower lane's slot of the same quad position already requests holds
-// kReqRedirect | that slot instead and is not decoded: a magnified texture gives most of a tile's
-// pixels the same quad.
+// Neural resolve: the emit pass records, per pixel, what the texels of the levels the model decodes
+// are (4 slots: the nearest texel, or the bilinear quad's 00 10 01 11 texels) and counts them per material; the
+// second pass reads the decoded texels from the same slots. Within a 4x4 tile a slot's texel is
+// decoded by the lowest lane that needs it at the same quad position (its leader): a magnified texture
+// gives most of a tile's pixels the same quad.
 enum { kResolvePlain = 0, kResolveEmit = 1, kResolveNeural = 2, kResolveDebug = 3 };
-constexpr unsigned long long kReqRedirect = 1ull << 63;  // | slot; ~0 (none) has the bit too
 struct NeuralResolve {
     const DevTexture* tex;             // model textures (data == nullptr: not decoded)
     uint32_t numMaterials, decodedLevels;  // texture levels below decodedLevels are decoded
-    unsigned long long* pixelReq;      // [pixel * 4 + k] material<<32 | level<<28 | ty<<14 | tx
     uint32_t* counts;                  // [material]
     const uint2* decoded;              // [pixel * 4 + k] layer-0 RGBA8, layer-1 RGBA8
-    uint4* surf;                       // [pixel * 2 + 0..1] the emit pass's surface record (kSurf*)
+    uint4* surf;                       // [pixel], then [pixels + pixel]: the emit pass's record
+    uint32_t pixels;
 };
-// The emit pass's per-pixel surface record, which spares the second pass the reconstruction of a
-// tile whose pixels all have it (kSurfFast): word 0-1 barycentrics b1, b2; 2-4 the vertices'
-// normal/tangent words; 5-6 the decoded quad's filter fractions; 7 flags.
-enum : uint32_t {
-    kSurfFast = 1u,        // sampled from decoded texels, or untextured (albedo and NMR 0)
-    kSurfDecoded = 2u,     // a decoded material sample: fetch it
-    kSurfNearest = 4u, kSurfInX = 8u, kSurfInY = 16u, kSurfTwoLayers = 32u,
-    kSurfHand = 1u << 31,  // the bitangent's sign bit
-};
+// The emit pass's record of a pixel, which spares the second pass the reconstruction of a tile whose pixels all have
+// it (kSurfFast). First plane: barycentrics b1, b2 and two vertices' normal/tangent words. Second plane, which
+// k_neural_scatter reads too: the third vertex's word, the flags (kSurf*, swr_neural.h) with the quad's
+// filter weights, the texel (level << 28 | ty << 14 | tx, the quad's first) and the material with the slots' leaders
+// (4 bits each from bit 16). 32 bytes a pixel instead of 64 with a word per slot, at
+// 2560x1440: emit pass 171 -> 162 us, scatter 59 -> 27, second pass 134 -> 118.
+__device__ __forceinline__ uint32_t surf_weight(uint32_t f) { return (f >> 7) & 255u; }             // of a packed 1.15 weight
+__device__ __forceinline__ uint32_t packed_weight(uint32_t w) { return (w << 7) | (w << 23); }      // and back
 
 __device__ __forceinline__ uint32_t sat_u8(int32_t v) { return (uint32_t)min(max(min(max(v, -32768), 32767), 0), 255); }
 __device__ __forceinline__ float unpack_f11(uint32_t x) { x <<= 17; return __uint_as_float((x & 0x0FFE0000u) + 0x38000000u); }
@@ -394,7 +391,6 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
     const unsigned skyBits = (__ballot_sync(hm, isSky) >> (16 * half)) & 0xFFFF;
 
     F3 color = { 0.f, 0.f, 0.f };
-    unsigned long long req[4] = { ~0ull, ~0ull, ~0ull, ~0ull };
     // ResolveDebug: sky pixels get a checkerboard of 4x4 tiles; layers other than the surface
     // ones need no surface
     const uint32_t background = ((x0 ^ y0) & 4) ? 0xFFA0A0A0u : 0xFFFFFFFFu;
@@ -406,8 +402,7 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
     }
     if constexpr (kMode == kResolveEmit) {
         if (skyBits == 0xFFFF) {
-            uint4* dst = (uint4*)(nr.pixelReq + (size_t)off * 4);
-            dst[0] = dst[1] = make_uint4(~0u, ~0u, ~0u, ~0u);
+            nr.surf[nr.pixels + off] = make_uint4(0u, 0u, 0u, 0u);  // nothing to decode
             return;
         }
     }
@@ -417,33 +412,29 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
         bool fast = false;  // the neural pass found the emit pass's records for the whole tile
         if constexpr (kMode == kResolveNeural) {
             uint4 s0 = make_uint4(0u, 0u, 0u, 0u), s1 = make_uint4(0u, 0u, 0u, 0u);
-            if (!isSky) s0 = nr.surf[(size_t)off * 2], s1 = nr.surf[(size_t)off * 2 + 1];
-            fast = (__ballot_sync(hm, isSky || (s1.w & kSurfFast)) & hm) == hm;
+            if (!isSky) s0 = nr.surf[off], s1 = nr.surf[nr.pixels + off];
+            fast = (__ballot_sync(hm, isSky || (s1.y & kSurfFast)) & hm) == hm;
             if (fast) {
                 const float nan = __int_as_float(0x7FFFFFFF);  // what the full path gives sky pixels
                 b[1] = isSky ? nan : __uint_as_float(s0.x);
                 b[2] = isSky ? nan : __uint_as_float(s0.y);
                 b[0] = 1 - b[1] - b[2];
                 ntg[0] = s0.z, ntg[1] = s0.w, ntg[2] = s1.x;
-                hand = s1.w & kSurfHand;
-                if (!isSky && (s1.w & kSurfDecoded)) {
-                    const ulonglong2* rq = (const ulonglong2*)(nr.pixelReq + (size_t)off * 4);
-                    const ulonglong2 r01 = rq[0], r23 = rq[1];
-                    auto at = [&](unsigned long long r, uint32_t k) {
-                        const size_t slot = (r != ~0ull && (r & kReqRedirect)) ? (size_t)(uint32_t)r : (size_t)off * 4 + k;
-                        return nr.decoded[slot];
-                    };
-                    const bool inX = s1.w & kSurfInX, inY = s1.w & kSurfInY;
-                    const uint2 d00 = at(r01.x, 0);
+                hand = s1.y & kSurfHand;
+                if (!isSky && (s1.y & kSurfDecoded)) {
+                    auto at = [&](uint32_t k) { return nr.decoded[(size_t)((off & ~15u) + ((s1.w >> (16 + 4 * k)) & 15u)) * 4 + k]; };
+                    const bool inX = s1.y & kSurfInX, inY = s1.y & kSurfInY;
+                    const uint2 d00 = at(0);
                     uint2 r0 = d00;
-                    if (!(s1.w & kSurfNearest)) {
-                        const uint2 d10 = inX ? at(r01.y, 1) : d00, d01 = inY ? at(r23.x, 2) : d00;
-                        const uint2 d11 = inY ? (inX ? at(r23.y, 3) : d01) : d10;
-                        r0.x = filter_rgba8(d00.x, d10.x, d01.x, d11.x, s1.y, s1.z);
-                        r0.y = filter_rgba8(d00.y, d10.y, d01.y, d11.y, s1.y, s1.z);
+                    if (!(s1.y & kSurfNearest)) {
+                        const uint2 d10 = inX ? at(1) : d00, d01 = inY ? at(2) : d00;
+                        const uint2 d11 = inY ? (inX ? at(3) : d01) : d10;
+                        const uint32_t fx = packed_weight((s1.y >> 8) & 255u), fy = packed_weight((s1.y >> 16) & 255u);
+                        r0.x = filter_rgba8(d00.x, d10.x, d01.x, d11.x, fx, fy);
+                        r0.y = filter_rgba8(d00.y, d10.y, d01.y, d11.y, fx, fy);
                     }
                     albedo = r0.x;
-                    if (s1.w & kSurfTwoLayers) nmr = r0.y;
+                    if (s1.y & kSurfTwoLayers) nmr = r0.y;
                 }
             }
         }
@@ -454,7 +445,7 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
         // round of dependent loads per id.
         F3 pos[3] = {};
         uint32_t tc[3] = {}, matId = 0;
-        uint32_t sflags = kSurfFast, sfx = 0, sfy = 0;  // the emit pass's record of this pixel
+        uint32_t sflags = kSurfFast, stexel = 0, slead = 0;  // the emit pass's record of this pixel
         const unsigned covered = ((~skyBits) & 0xFFFF) << (16 * half);
         const bool holds = skyBits == 0 || (__match_any_sync(hm, id) & covered) != 0;
         const uint32_t mId = id / 128, tri = id % 128;
@@ -546,30 +537,23 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
                       nr.tex[mid].width == tex.width && nr.tex[mid].height == tex.height;
             if constexpr (kMode == kResolveEmit) {
                 uint32_t nq = 0;
-                if (sampled) {
+                if (sampled)
                     sflags = dec ? kSurfFast | kSurfDecoded | (nearest ? kSurfNearest : 0u) | (q.inX ? kSurfInX : 0u) |
-                                       (q.inY ? kSurfInY : 0u) | (tex.num_layers >= 2 ? kSurfTwoLayers : 0u)
+                                       (q.inY ? kSurfInY : 0u) | (tex.num_layers >= 2 ? kSurfTwoLayers : 0u) |
+                                       (surf_weight(q.fx) << 8) | (surf_weight(q.fy) << 16)
                                  : 0u;  // sampled from the plain texture: the second pass reconstructs
-                    sfx = q.fx, sfy = q.fy;
-                }
-                if (dec) {
-                    const unsigned long long b = ((unsigned long long)mid << 32) | ((uint32_t)q.m << 28);
-                    const uint32_t x0 = (uint32_t)q.tx, y0 = (uint32_t)q.ty;
-                    req[0] = b | (y0 << 14) | x0;
-                    if (!nearest) {
-                        if (q.inX) req[1] = b | (y0 << 14) | (x0 + 1);
-                        if (q.inY) req[2] = b | ((y0 + 1) << 14) | x0;
-                        if (q.inX && q.inY) req[3] = b | ((y0 + 1) << 14) | (x0 + 1);
-                    }
-                }
+                if (dec) stexel = ((uint32_t)q.m << 28) | ((uint32_t)q.ty << 14) | (uint32_t)q.tx;
+                slead = dec ? mid : 0u;
+                // a slot's leader: the lowest lane with its texel in the slot, of the same material
+                const unsigned sameMaterial = __match_any_sync(hm, dec ? mid : ~0u);
 #pragma unroll
-                for (int k = 0; k < 4; k++) {  // requests equal to a lower lane's at the same position
-                    const unsigned peers = __match_any_sync(hm, req[k]);
-                    const int lead = __ffs(peers) - 1;
-                    const uint32_t leadOff = __shfl_sync(hm, off, lead);
-                    if (req[k] == ~0ull) continue;
-                    if (lead != (int)lane) req[k] = kReqRedirect | ((unsigned long long)leadOff * 4 + k);
-                    else nq++;
+                for (uint32_t k = 0; k < 4; k++) {
+                    const bool has = dec && surf_has_slot(sflags, k);
+                    const uint32_t texel = has ? surf_slot_texel(stexel, k) : ~0u;
+                    const int lead = __ffs(__match_any_sync(hm, texel) & sameMaterial) - 1;
+                    if (!has) continue;
+                    slead |= ((uint32_t)lead & 15u) << (16 + 4 * k);
+                    if (lead == (int)lane) nq++;
                 }
                 unsigned pm = __ballot_sync(hm, nq != 0) & hm;
                 while (pm) {  // the requests of each of the tile's materials
@@ -582,18 +566,13 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
                     }
                 }
             } else if (dec) {
-                // a slot's decoded texel, or the one of the slot it redirects to
-                const ulonglong2* rq = (const ulonglong2*)(nr.pixelReq + (size_t)off * 4);
-                const ulonglong2 r01 = rq[0], r23 = rq[1];
-                auto at = [&](unsigned long long r, uint32_t k) {
-                    const size_t slot = (r != ~0ull && (r & kReqRedirect)) ? (size_t)(uint32_t)r : (size_t)off * 4 + k;
-                    return nr.decoded[slot];
-                };
-                const uint2 d00 = at(r01.x, 0);
+                const uint32_t leads = nr.surf[nr.pixels + off].w >> 16;
+                auto at = [&](uint32_t k) { return nr.decoded[(size_t)((off & ~15u) + ((leads >> (4 * k)) & 15u)) * 4 + k]; };
+                const uint2 d00 = at(0);
                 uint2 r0 = d00;
                 if (!nearest) {
-                    const uint2 d10 = q.inX ? at(r01.y, 1) : d00, d01 = q.inY ? at(r23.x, 2) : d00;
-                    const uint2 d11 = q.inY ? (q.inX ? at(r23.y, 3) : d01) : d10;
+                    const uint2 d10 = q.inX ? at(1) : d00, d01 = q.inY ? at(2) : d00;
+                    const uint2 d11 = q.inY ? (q.inX ? at(3) : d01) : d10;
                     r0.x = filter_rgba8(d00.x, d10.x, d01.x, d11.x, q.fx, q.fy);
                     r0.y = filter_rgba8(d00.y, d10.y, d01.y, d11.y, q.fx, q.fy);
                 }
@@ -605,11 +584,8 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
             }
         }
         if constexpr (kMode == kResolveEmit) {
-            uint4* dst = (uint4*)(nr.pixelReq + (size_t)off * 4);
-            dst[0] = make_uint4((uint32_t)req[0], (uint32_t)(req[0] >> 32), (uint32_t)req[1], (uint32_t)(req[1] >> 32));
-            dst[1] = make_uint4((uint32_t)req[2], (uint32_t)(req[2] >> 32), (uint32_t)req[3], (uint32_t)(req[3] >> 32));
-            nr.surf[(size_t)off * 2] = make_uint4(__float_as_uint(b[1]), __float_as_uint(b[2]), ntg[0], ntg[1]);
-            nr.surf[(size_t)off * 2 + 1] = make_uint4(ntg[2], sfx, sfy, sflags | hand);
+            nr.surf[off] = make_uint4(__float_as_uint(b[1]), __float_as_uint(b[2]), ntg[0], ntg[1]);
+            nr.surf[nr.pixels + off] = make_uint4(ntg[2], sflags | hand, stexel, slead);
             return;
         }
         }  // !fast
@@ -953,13 +929,11 @@ swr_status swr_resolve_neural(swr_rasterizer r, swr_framebuffer fb, const swr_sh
     const size_t slots = (size_t)fb->width * fb->height * 4;
     cudaError_t e = cudaSuccess;
     if (n->scratchSlots < slots) {
-        if (n->pixelReq) cudaFree(n->pixelReq);
         if (n->sorted) cudaFree(n->sorted);
         if (n->decoded) cudaFree(n->decoded);
         if (n->surf) cudaFree(n->surf);
-        n->pixelReq = n->sorted = nullptr, n->decoded = nullptr, n->surf = nullptr, n->scratchSlots = 0;
-        e = cudaMalloc(&n->pixelReq, slots * sizeof(unsigned long long));
-        if (e == cudaSuccess) e = cudaMalloc(&n->sorted, slots * sizeof(unsigned long long));
+        n->sorted = nullptr, n->decoded = nullptr, n->surf = nullptr, n->scratchSlots = 0;
+        e = cudaMalloc(&n->sorted, slots * sizeof(unsigned long long));
         if (e == cudaSuccess) e = cudaMalloc(&n->decoded, slots * sizeof(uint2));
         if (e == cudaSuccess) e = cudaMalloc(&n->surf, slots / 4 * 2 * sizeof(uint4));
         if (e != cudaSuccess) {
@@ -976,7 +950,7 @@ swr_status swr_resolve_neural(swr_rasterizer r, swr_framebuffer fb, const swr_sh
     uint32_t* levelCount = tileOffset + (M + 1);
     NeuralResolve nr = {};
     nr.tex = n->d.tex, nr.numMaterials = M, nr.decodedLevels = n->d.levels + 2;
-    nr.pixelReq = n->pixelReq, nr.counts = counts, nr.decoded = n->decoded, nr.surf = n->surf;
+    nr.counts = counts, nr.decoded = n->decoded, nr.surf = n->surf, nr.pixels = (uint32_t)(slots / 4);
     const uint32_t tiles = (fb->width / 4) * (fb->height / 4), blocks = (tiles * 16 + 255) / 256;
     e = cudaMemsetAsync(counts, 0, 2 * (M + 1) * sizeof(uint32_t), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(levelCount, 0, kNeuralMaxDecoded * sizeof(uint32_t), st);
@@ -993,7 +967,7 @@ swr_status swr_resolve_neural(swr_rasterizer r, swr_framebuffer fb, const swr_sh
     }
     if (e == cudaSuccess) {
         LaunchScope ls("k_neural_scatter", st);
-        launch_neural_scatter(n->pixelReq, (uint32_t)slots, reqOffset, cursor, n->sorted, levelCount, M, st);
+        launch_neural_scatter(n->surf + slots / 4, (uint32_t)(slots / 4), reqOffset, cursor, n->sorted, levelCount, M, st);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
