@@ -797,7 +797,9 @@ __global__ void __launch_bounds__(1024) k_neural_offsets(const uint32_t* counts,
                                                          uint32_t n) {
     __shared__ uint32_t sr[1024], st[1024];
     const uint32_t t = threadIdx.x;
-    const uint32_t c = t < n ? counts[t] : 0u;
+    uint32_t c = 0;
+    if (t < n)
+        for (uint32_t k = 0; k < kCountCopies; k++) c += counts[k * count_stride(n) + t];
     sr[t] = c, st[t] = (c + 127) / 128;
     __syncthreads();
     for (uint32_t o = 1; o < 1024; o <<= 1) {

@@ -108,6 +108,10 @@ void launch_neural_export(const float* latent, uint16_t* half, size_t count, cud
 void launch_wait_selftest(uint32_t* status, uint64_t limitNs, cudaStream_t st);
 void launch_neural_offsets(const uint32_t* counts, uint32_t* reqOffset, uint32_t* tileOffset, uint32_t numMaterials,
                            cudaStream_t st);
+// The emit pass counts requests per material in kCountCopies copies on lines of their own, a block in copy block %
+// kCountCopies (one word per material, all on a line, took 230,000 atomics a frame: emit pass 162 -> 94 us).
+constexpr uint32_t kCountCopies = 16;
+__host__ __device__ inline uint32_t count_stride(uint32_t numMaterials) { return (numMaterials + 32u) & ~31u; }
 // Flags of the neural resolve's pixel records (swr_shade.cu); the filter weights are in bits 8 to 23.
 enum : uint32_t {
     kSurfFast = 1u,        // sampled from decoded texels, or untextured (albedo and NMR 0)
@@ -154,6 +158,6 @@ struct swr_neural_t {
     uint2* decoded;
     uint4* surf;                             // two planes of a word per pixel: the emit pass's surface records
     size_t scratchSlots;
-    uint32_t* counters;                      // counts | cursors | reqOffset | tileOffset, numMaterials+1 each,
+    uint32_t* counters;                      // kCountCopies counts | cursors | reqOffset | tileOffset, numMaterials+1 each,
                                              // then 4 per-level request counts
 };

@@ -233,7 +233,7 @@ swr_status swr_neural_create(const swr_texture* textures, uint32_t num_materials
     chk(dev_alloc(&n->image, (size_t)num_materials * kNeuralImage));
     chk(dev_alloc(&n->loss, kOutcomeWords));
     n->status = (uint32_t*)(n->loss + 2);
-    chk(dev_alloc(&n->counters, 4 * (size_t)(num_materials + 1) + kNeuralMaxDecoded));
+    chk(dev_alloc(&n->counters, (size_t)kCountCopies * count_stride(num_materials) + 3 * (size_t)(num_materials + 1) + kNeuralMaxDecoded));
     if (e != cudaSuccess) {
         free_model(n);
         return e == cudaErrorMemoryAllocation ? swr_internal_fail(SWR_ENOMEM, "swr_neural_create: out of device memory")

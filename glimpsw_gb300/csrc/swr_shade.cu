@@ -267,7 +267,7 @@ enum { kResolvePlain = 0, kResolveEmit = 1, kResolveNeural = 2, kResolveDebug = 
 struct NeuralResolve {
     const DevTexture* tex;             // model textures (data == nullptr: not decoded)
     uint32_t numMaterials, decodedLevels;  // texture levels below decodedLevels are decoded
-    uint32_t* counts;                  // [material]
+    uint32_t* counts;                  // [copy][material]
     const uint2* decoded;              // [pixel * 4 + k] layer-0 RGBA8, layer-1 RGBA8
     uint4* surf;                       // [pixel], then [pixels + pixel]: the emit pass's record
     uint32_t pixels;
@@ -562,7 +562,8 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
                     pm &= ~iter;
                     if ((iter >> lane) & 1) {
                         const uint32_t total = __reduce_add_sync(iter, nq);
-                        if ((int)lane == __ffs(iter) - 1) atomicAdd(&nr.counts[m], total);
+                        if ((int)lane == __ffs(iter) - 1)
+                            atomicAdd(&nr.counts[(blockIdx.x % kCountCopies) * count_stride(nr.numMaterials) + m], total);
                     }
                 }
             } else if (dec) {
@@ -944,7 +945,7 @@ swr_status swr_resolve_neural(swr_rasterizer r, swr_framebuffer fb, const swr_sh
     }
     neural_sync_half(n, st);
     uint32_t* counts = n->counters;
-    uint32_t* cursor = counts + (M + 1);
+    uint32_t* cursor = counts + kCountCopies * count_stride(M);
     uint32_t* reqOffset = cursor + (M + 1);
     uint32_t* tileOffset = reqOffset + (M + 1);
     uint32_t* levelCount = tileOffset + (M + 1);
@@ -952,7 +953,7 @@ swr_status swr_resolve_neural(swr_rasterizer r, swr_framebuffer fb, const swr_sh
     nr.tex = n->d.tex, nr.numMaterials = M, nr.decodedLevels = n->d.levels + 2;
     nr.counts = counts, nr.decoded = n->decoded, nr.surf = n->surf, nr.pixels = (uint32_t)(slots / 4);
     const uint32_t tiles = (fb->width / 4) * (fb->height / 4), blocks = (tiles * 16 + 255) / 256;
-    e = cudaMemsetAsync(counts, 0, 2 * (M + 1) * sizeof(uint32_t), st);
+    e = cudaMemsetAsync(counts, 0, (kCountCopies * count_stride(M) + M + 1) * sizeof(uint32_t), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(levelCount, 0, kNeuralMaxDecoded * sizeof(uint32_t), st);
     if (e == cudaSuccess) {
         LaunchScope ls("k_resolve_emit", st);
