@@ -77,7 +77,7 @@ swr_status size_queue(swr_rasterizer r, uint32_t count) {
         if (*r->hostStatus & kStatusBigOverflow) r->sawOverflow = true;
     }
     uint64_t want = (uint64_t)count * (r->sawOverflow ? 128u : 32u);
-    want = std::min<uint64_t>(std::max<uint64_t>(want, kDefaultBigCapacity), 1u << 26);
+    want = std::min<uint64_t>(std::max<uint64_t>(want, kDefaultBigCapacity), kQueueMaxCapacity);
     DrawScratch& s = r->scratch;
     if (r->fixedCapacity) {
         if (s.bigCapacity != r->fixedCapacity) s.bigCapacity = std::min(r->fixedCapacity, s.bigCapacity);
@@ -246,7 +246,7 @@ swr_status swr_rasterizer_set_flags(swr_rasterizer r, int enable_binning, int en
 
 swr_status swr_rasterizer_set_queue_capacity(swr_rasterizer r, uint32_t triangles) {
     if (!r) return fail(SWR_EINVAL, "swr_rasterizer_set_queue_capacity: NULL rasterizer");
-    r->fixedCapacity = triangles;
+    r->fixedCapacity = std::min(triangles, kQueueMaxCapacity);
     return SWR_OK;
 }
 

@@ -292,7 +292,7 @@ swr_status swr_batch_create(swr_rasterizer r, swr_scene s, uint32_t first, uint3
     if (e == cudaSuccess) e = cudaMalloc(&b->dGroupMasks, (size_t)num_views * words * sizeof(uint32_t) + 16);
     if (e == cudaSuccess) e = cudaMemcpy(b->dViewStart, start.data(), start.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
     // the batch's own queue: a quarter of the triangles of every view; overflow is rasterized in place
-    b->scratch.bigCapacity = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(totalTris, 1u << 18), 1u << 26);
+    b->scratch.bigCapacity = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(totalTris, 1u << 18), kQueueMaxCapacity);
     if (e == cudaSuccess) e = cudaMalloc(&b->scratch.control, 16 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemset(b->scratch.control, 0, 16 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMalloc(&b->scratch.big, (size_t)b->scratch.bigCapacity * sizeof(TriRec));

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "../../include/swr_gb300.h"
+#include "swr_queue.h"
 
 namespace swr {
 
@@ -123,7 +124,7 @@ static_assert(sizeof(AlphaExt) == sizeof(TriRec) && offsetof(AlphaExt, zero0) ==
 
 // Per-rasterizer device scratch, reused by every draw.
 struct DrawScratch {
-    unsigned long long* control;   // [0] meshlet work counter, [1] big-triangle queue (slots<<40 | chunks),
+    unsigned long long* control;   // [0] meshlet work counter, [1] big-triangle queue's tail (swr_queue.h),
                                    // [2] status flags, [3..6] perf counters, [7] the second pass's work
                                    // counter of a single-view draw, [8] chunk-stage cursor,
                                    // [9] alpha list length, [10] alpha-pass cursor,

@@ -212,22 +212,32 @@ __device__ __noinline__ void raster_serial(const TriRec& r, unsigned long long* 
         for (uint32_t x = minX; x < maxX; x++) shade_fragment(r, x, y, keys, width);
 }
 
+// Takes back a claim of the chunk queue that has no room (swr_queue.h).
+__device__ __forceinline__ void queue_release(const DrawArgs& a, unsigned long long claim) {
+    atomicAdd(&a.s.control[1], 0ull - claim);
+    atomicOr(&a.s.control[2], kStatusBigOverflow);
+}
+
+// The chunks (chunk_shape) of a triangle's render box.
+__device__ __forceinline__ uint32_t triangle_chunks(const TriRec& r, uint32_t chunk) {
+    const uint32_t tilesX = ((r.bbMax & 0xFFFF) - (r.bbMin & 0xFFFF)) >> 2, tilesY = ((r.bbMax >> 16) - (r.bbMin >> 16)) >> 2;
+    const uint32_t cw = chunk & 0xFF, ch = chunk >> 8;
+    return ((tilesX + cw - 1) / cw) * ((tilesY + ch - 1) / ch);
+}
+
 // Appends a triangle (its view index in r.pad) to the chunk queue; false when the queue is full
 // (the caller rasterizes it).
 __device__ __forceinline__ bool enqueue_big(const TriRec& r, const DrawArgs& a, uint32_t chunk) {
-    int tilesX = ((r.bbMax & 0xFFFF) - (r.bbMin & 0xFFFF)) >> 2;
-    int tilesY = ((r.bbMax >> 16) - (r.bbMin >> 16)) >> 2;
-    const uint32_t cw = chunk & 0xFF, ch = chunk >> 8;
-    unsigned long long chunks = (unsigned long long)((tilesX + cw - 1) / cw) * (unsigned long long)((tilesY + ch - 1) / ch);
-    unsigned long long old = atomicAdd(&a.s.control[1], (1ull << 40) | chunks);
-    unsigned long long slot = old >> 40;
-    if (slot < a.s.bigCapacity) {
-        a.s.big[slot] = r;
-        a.s.bigBase[slot] = old & ((1ull << 40) - 1);
-        return true;
+    const unsigned long long claim = queue_claim(1, triangle_chunks(r, chunk));
+    const unsigned long long old = atomicAdd(&a.s.control[1], claim);
+    const uint32_t slot = queue_slots(old);
+    if (!queue_fits(slot, queue_chunks(old), 1, a.s.bigCapacity)) {
+        queue_release(a, claim);
+        return false;
     }
-    atomicOr(&a.s.control[2], kStatusBigOverflow);
-    return false;
+    a.s.big[slot] = r;
+    a.s.bigBase[slot] = queue_chunks(old);
+    return true;
 }
 
 // ------------------------------------------------------------------ alpha test
@@ -357,29 +367,22 @@ __device__ __noinline__ void raster_serial_alpha(const TriRec& r, const AlphaExt
 }
 
 // Appends an alpha-tested triangle and its AlphaExt (in the next slot, which owns no chunks) to
-// the chunk queue; false when the queue is full (the caller rasterizes it). A pair that finds
-// one slot left leaves an empty record there, so every slot below the capacity is written.
+// the chunk queue; false when the queue is full (the caller rasterizes it).
 __device__ __forceinline__ bool enqueue_alpha(const TriRec& r, const AlphaExt& x, const DrawArgs& a, uint32_t chunk) {
-    const int tilesX = ((r.bbMax & 0xFFFF) - (r.bbMin & 0xFFFF)) >> 2;
-    const int tilesY = ((r.bbMax >> 16) - (r.bbMin >> 16)) >> 2;
-    const uint32_t cw = chunk & 0xFF, ch = chunk >> 8;
-    const unsigned long long chunks = (unsigned long long)((tilesX + cw - 1) / cw) * (unsigned long long)((tilesY + ch - 1) / ch);
-    const unsigned long long old = atomicAdd(&a.s.control[1], (2ull << 40) | chunks);
-    const unsigned long long slot = old >> 40, base = old & ((1ull << 40) - 1);
-    if (slot + 1 < a.s.bigCapacity) {
-        a.s.big[slot] = r;
-        a.s.big[slot + 1] = *(const TriRec*)&x;
-        a.s.bigBase[slot] = base;
-        a.s.bigBase[slot + 1] = base + chunks;
-        return true;
+    const uint32_t chunks = triangle_chunks(r, chunk);
+    const unsigned long long claim = queue_claim(2, chunks);
+    const unsigned long long old = atomicAdd(&a.s.control[1], claim);
+    const uint32_t slot = queue_slots(old);
+    const unsigned long long base = queue_chunks(old);
+    if (!queue_fits(slot, base, 2, a.s.bigCapacity)) {
+        queue_release(a, claim);
+        return false;
     }
-    if (slot < a.s.bigCapacity) {
-        TriRec e = {};
-        a.s.big[slot] = e;
-        a.s.bigBase[slot] = base;
-    }
-    atomicOr(&a.s.control[2], kStatusBigOverflow);
-    return false;
+    a.s.big[slot] = r;
+    a.s.big[slot + 1] = *(const TriRec*)&x;
+    a.s.bigBase[slot] = base;
+    a.s.bigBase[slot + 1] = base + chunks;
+    return true;
 }
 
 // Appends the records of the lanes with `want` (rec, its view index in pad; alpha-tested ones with their
@@ -394,12 +397,7 @@ __device__ __forceinline__ bool enqueue_warp(bool want, const TriRec& rec, const
     const unsigned m = __ballot_sync(0xFFFFFFFFu, want);
     if (m == 0) return true;
     constexpr uint32_t kSlots = kAlpha ? 2 : 1;
-    uint32_t chunks = 0;
-    if (want) {
-        const uint32_t tilesX = ((rec.bbMax & 0xFFFF) - (rec.bbMin & 0xFFFF)) >> 2, tilesY = ((rec.bbMax >> 16) - (rec.bbMin >> 16)) >> 2;
-        const uint32_t cw = chunk & 0xFF, ch = chunk >> 8;
-        chunks = ((tilesX + cw - 1) / cw) * ((tilesY + ch - 1) / ch);
-    }
+    const uint32_t chunks = want ? triangle_chunks(rec, chunk) : 0u;
     uint32_t incl = chunks;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -407,27 +405,25 @@ __device__ __forceinline__ bool enqueue_warp(bool want, const TriRec& rec, const
         if (lane >= o) incl += v;
     }
     unsigned long long old = 0;
-    if (lane == 31) old = atomicAdd(&a.s.control[1], ((unsigned long long)(__popc(m) * kSlots) << 40) | incl);
+    if (lane == 31) old = atomicAdd(&a.s.control[1], queue_claim(__popc(m) * kSlots, incl));
     old = __shfl_sync(0xFFFFFFFFu, old, 31);
-    if (!want) return true;
-    const unsigned long long slot = (old >> 40) + __popc(m & ((1u << lane) - 1u)) * kSlots;
-    const unsigned long long base = (old & ((1ull << 40) - 1)) + (incl - chunks);
-    if (slot + (kSlots - 1) < a.s.bigCapacity) {
+    const uint32_t slot = queue_slots(old) + __popc(m & ((1u << lane) - 1u)) * kSlots;
+    const unsigned long long base = queue_chunks(old) + (incl - chunks);
+    const bool fits = queue_fits(slot, base, kSlots, a.s.bigCapacity);
+    if (want && fits) {
         a.s.big[slot] = rec;
         a.s.bigBase[slot] = base;
         if constexpr (kAlpha) {
             a.s.big[slot + 1] = *(const TriRec*)x;
             a.s.bigBase[slot + 1] = base + chunks;
         }
-        return true;
     }
-    if (kAlpha && slot < a.s.bigCapacity) {  // one slot left: an empty record
-        const TriRec e = {};
-        a.s.big[slot] = e;
-        a.s.bigBase[slot] = base;
+    const unsigned full = __ballot_sync(0xFFFFFFFFu, want && !fits);
+    if (full) {  // the last lanes' claims: one addition for all
+        const uint32_t all = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        if (lane == __ffs(full) - 1) queue_release(a, queue_claim(__popc(full) * kSlots, all - (incl - chunks)));
     }
-    atomicOr(&a.s.control[2], kStatusBigOverflow);
-    return false;
+    return !want || fits;
 }
 
 // A small triangle's record (the mesh stage's tile walk): pad = tilesX | row_magic << 8 | kPadReadKey.
@@ -1490,7 +1486,7 @@ __global__ void __launch_bounds__(256, kAlpha || kOver ? 4 : 5) k_raster_big(con
     const unsigned long long q = control[1];
     if (lastStage && blockIdx.x == 0 && threadIdx.x == 0)  // the next draw's second cursor, alpha list and idle-warp counts
         control[7] = control[9] = control[10] = control[11] = control[12] = 0;
-    const uint32_t n = (uint32_t)min((unsigned long long)capacity, q >> 40);
+    const uint32_t n = min(capacity, queue_slots(q));
     if (n == 0) return;
     const int lane = threadIdx.x & 31;
     const TriRec& last = big[n - 1];
