@@ -137,10 +137,9 @@ __device__ __forceinline__ float min4_lanes(float v, uint32_t down, uint32_t rig
 // Bound by latency (a load, three shuffles, a barrier, two shuffles): all of 2560x1440
 // 22.1 -> 9.1 us (a thread per texel of levels 0-3 through shared memory, and one block for the levels above),
 // 1280x720 14.4 -> 6.4 us.
-// ordered: the texture lacks some of the levels, which all land at its start, the highest last.
 __global__ void __launch_bounds__(1024) k_hiz_local(const float* __restrict__ depth, uint32_t fbW, uint32_t fbH,
                                                     uint32_t* __restrict__ tex, HizOffsets offs, int32_t rowShift,
-                                                    uint32_t nLocal, uint32_t ordered) {
+                                                    uint32_t nLocal) {
     __shared__ float s3[8][8];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t X = blockIdx.x * 32 + (warp & 3) * 8 + (lane >> 2), Y = blockIdx.y * 32 + (warp >> 2) * 4 + (lane & 3);
@@ -162,13 +161,10 @@ __global__ void __launch_bounds__(1024) k_hiz_local(const float* __restrict__ de
         *(float2*)&tex[offs.off[0] + texel_offset(2 * X, 2 * Y, rowShift)] = make_float2(v00, v01);
         *(float2*)&tex[offs.off[0] + texel_offset(2 * X + 1, 2 * Y, rowShift)] = make_float2(v10, v11);
     }
-    if (ordered) __syncthreads();
     const float v1 = min4(v00, v01, v10, v11);
     write(X, Y, 1, v1);
-    if (ordered) __syncthreads();
     const float v2 = min4_lanes(v1, 1, 4);
     if ((lane & 5) == 0) write(X >> 1, Y >> 1, 2, v2);
-    if (ordered) __syncthreads();
     const float v3 = min4_lanes(v2, 2, 8);
     if ((lane & 15) == 0) {
         write(X >> 2, Y >> 2, 3, v3);
@@ -181,10 +177,8 @@ __global__ void __launch_bounds__(1024) k_hiz_local(const float* __restrict__ de
     const float v4 = min4(s3[2 * y][2 * x], s3[2 * y + 1][2 * x], s3[2 * y][2 * x + 1], s3[2 * y + 1][2 * x + 1]);
     if (lane < 16) write(blockIdx.x * 4 + x, blockIdx.y * 4 + y, 4, v4);
     const float v5 = min4_lanes(v4, 1, 4);
-    if (ordered) __syncwarp();
     if (lane < 16 && (lane & 5) == 0) write(blockIdx.x * 2 + (x >> 1), blockIdx.y * 2 + (y >> 1), 5, v5);
     const float v6 = min4_lanes(v5, 2, 8);
-    if (ordered) __syncwarp();
     if (lane == 0) write(blockIdx.x, blockIdx.y, 6, v6);
 }
 
@@ -228,6 +222,15 @@ __global__ void __launch_bounds__(1024) k_hiz_tail(uint32_t fbW, uint32_t fbH, u
         }
         __syncthreads();
         src = dst;
+    }
+}
+
+// One level's texels (w x h, as written) from a scratch pyramid to the texture.
+__global__ void __launch_bounds__(256) k_hiz_place(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t w, uint32_t h,
+                                                   int32_t stride) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < w * h; i += gridDim.x * blockDim.x) {
+        const uint32_t o = texel_offset((int32_t)(i % w), (int32_t)(i / w), stride);
+        dst[o] = src[o];
     }
 }
 
@@ -852,16 +855,36 @@ swr_status swr_downsample_depth(swr_framebuffer fb, swr_texture dest) {
         if (stride < 0 || mipOff(m) + 7 + (maxX << 3) + (maxY << stride) >= dest->words)
             return swr_internal_fail(SWR_EINVAL, "swr_downsample_depth: destination too small for this framebuffer");
     }
+    // The tail's levels that the texture lacks land at its start level by level, after the local kernel's, which it has.
+    // A texture with fewer of those (below 4 levels: the tail cannot hold more) gets its levels from a scratch
+    // pyramid that has them all, one launch a level: blocks writing them at once would leave the words they
+    // share to whichever came last.
+    const uint32_t levels = dest->d.mip_levels;
+    const bool place = levels < std::min(root - 3, 4u);
     HizOffsets offs = {};
-    for (uint32_t m = 0; m + 3 <= root && m < 16; m++) offs.off[m] = mipOff(m);
-    // levels with 8x8-texel blocks; above level 3 those the texture has (the others are the tail's, after these)
-    const uint32_t levels = dest->d.mip_levels, nLocal = std::min(root - 3, std::max(4u, std::min(7u, levels)));
+    uint32_t* pyramid = tex;
+    cudaError_t e = cudaSuccess;
+    if (place) {
+        size_t words = 0;
+        for (uint32_t m = 0; m + 3 <= root; m++) {
+            uint32_t rx, ry, bt;
+            blocks(m, rx, ry, bt);
+            const uint32_t side = bt == 64 ? 8 : 4;
+            offs.off[m] = (uint32_t)words;
+            words += (((((size_t)rx * side - 1) << 3) + (((size_t)ry * side - 1) << (dest->d.row_shift - m)) + 7) | 63) + 1;
+        }
+        e = cudaMallocAsync(&pyramid, words * sizeof(uint32_t), st);
+        if (e != cudaSuccess) return swr_internal_cuda_fail(e, "swr_downsample_depth: scratch");
+    } else {
+        for (uint32_t m = 0; m + 3 <= root && m < 16; m++) offs.off[m] = mipOff(m);
+    }
+    const uint32_t nLocal = std::min(root - 3, place ? 7u : std::min(7u, levels));  // levels with 8x8-texel blocks
     {
         LaunchScope ls("k_hiz_local", st);
         // whole blocks of the highest level
         const uint32_t side = std::max(kHizRegion, 8u << nLocal), per = side / kHizRegion;
         const dim3 grid((fb->width + side - 1) / side * per, (fb->height + side - 1) / side * per);
-        k_hiz_local<<<grid, 1024, 0, st>>>(depth, fb->width, fb->height, tex, offs, (int32_t)dest->d.row_shift, nLocal, nLocal > levels);
+        k_hiz_local<<<grid, 1024, 0, st>>>(depth, fb->width, fb->height, pyramid, offs, (int32_t)dest->d.row_shift, nLocal);
     }
     if (root - 3 >= nLocal) {
         size_t smem = 0;  // levels nLocal-1 .. root-3, texels whose origin lies in the frame
@@ -869,10 +892,22 @@ swr_status swr_downsample_depth(swr_framebuffer fb, swr_texture dest) {
             smem += (size_t)hiz_extent(fb->width, m) * hiz_extent(fb->height, m) * sizeof(float);
         if (smem > 48 * 1024) cudaFuncSetAttribute(k_hiz_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         LaunchScope ls("k_hiz_tail", st);
-        k_hiz_tail<<<1, 1024, smem, st>>>(fb->width, fb->height, tex, offs, (int32_t)dest->d.row_shift, nLocal, root - 3,
+        k_hiz_tail<<<1, 1024, smem, st>>>(fb->width, fb->height, pyramid, offs, (int32_t)dest->d.row_shift, nLocal, root - 3,
                                            root);
     }
-    cudaError_t e = cudaGetLastError();
+    if (place) {
+        for (uint32_t m = 0; m + 3 <= root; m++) {
+            uint32_t rx, ry, bt;
+            blocks(m, rx, ry, bt);
+            const uint32_t side = bt == 64 ? 8 : 4, w = rx * side, h = ry * side;
+            LaunchScope ls("k_hiz_place", st);
+            k_hiz_place<<<std::min((w * h + 255) / 256, 1216u), 256, 0, st>>>(pyramid + offs.off[m], tex + mipOff(m), w, h,
+                                                                             (int32_t)(dest->d.row_shift - m));
+        }
+        e = cudaGetLastError();
+        cudaFreeAsync(pyramid, st);
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return swr_internal_cuda_fail(e, "swr_downsample_depth");
     return SWR_OK;
 }
