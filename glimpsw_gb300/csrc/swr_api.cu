@@ -7,6 +7,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -104,6 +106,37 @@ swr_status size_alpha_list(swr_rasterizer r, uint32_t count) {
     SWR_CUDA(cudaMallocAsync(&s.alphaList, (size_t)want * sizeof(uint32_t), t_stream));
     s.alphaCapacity = want;
     return SWR_OK;
+}
+
+// The unit vectors' table of the current device: one for all of its scenes, given back with the last. It is complete
+// before any caller has it, whatever streams draw and resolve later. Empty where there is no room for it.
+std::shared_ptr<float4> oct_table() {
+    struct Entry {
+        std::weak_ptr<float4> table;
+        unsigned long long context;  // a cudaDeviceReset ends the one the table lives in
+    };
+    static std::mutex mu;
+    static Entry entries[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return {};
+    std::lock_guard<std::mutex> lock(mu);
+    Entry& e = entries[dev];
+    const unsigned long long context = swr_internal_context_id();
+    std::shared_ptr<float4> t = context != 0 && context == e.context ? e.table.lock() : nullptr;
+    if (t) return t;
+    float4* p = nullptr;
+    cudaError_t err = cudaMalloc(&p, kOctTable * sizeof(float4));
+    if (err == cudaSuccess) {
+        t = std::shared_ptr<float4>(p, [](float4* q) { cudaFree(q); });
+        err = fill_oct_table(p);
+    }
+    if (err != cudaSuccess) {
+        cudaGetLastError();
+        return {};
+    }
+    e.table = t;
+    e.context = swr_internal_context_id();  // the allocation made the context current if none was
+    return t;
 }
 
 }  // namespace
@@ -424,7 +457,6 @@ swr_status swr_scene_destroy(swr_scene s) {
     cudaFree(s->meshlets);
     cudaFree(s->materials);
     cudaFree(s->fsIds);
-    cudaFree(s->octTable);
     delete s;
     return SWR_OK;
 }
@@ -437,16 +469,7 @@ swr_status swr_scene_upload_meshlets(swr_scene s, const void* meshlets, uint32_t
                     SWR_MAX_MESHLETS);
     // Records are not inspected on the host (that would cost a cache miss per meshlet); kernels
     // clamp NumVertices to 64 and NumTriangles to 128, the sizes of the record's arrays.
-    // Room is not needed for it (the shading kernels compute what it holds without it).
-    if (!s->octTable && end) {
-        if (cudaMalloc(&s->octTable, kOctTable * sizeof(float4)) == cudaSuccess) {
-            launch_oct_table(s->octTable, t_stream);
-            SWR_CHECK_LAUNCH("swr_scene_upload_meshlets");
-        } else {
-            cudaGetLastError();
-            s->octTable = nullptr;
-        }
-    }
+    if (!s->octTable && end) s->octTable = oct_table();
     if (end > s->capacity) {
         uint32_t cap = (uint32_t)std::max<uint64_t>(end, (uint64_t)s->capacity * 3 / 2);
         cap = std::min(cap, SWR_MAX_MESHLETS);

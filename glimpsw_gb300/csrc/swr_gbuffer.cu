@@ -111,7 +111,7 @@ swr_status swr_internal_draw_deferred(swr_rasterizer r, swr_framebuffer fb, uint
     g.meshlets = ctx->scene->meshlets;
     g.materials = ctx->scene->materials;
     g.numMaterials = ctx->scene->num_materials;
-    g.octTable = ctx->scene->octTable;
+    g.octTable = ctx->scene->octTable.get();
     memcpy(g.objectToWorld, ctx->object_to_world, sizeof(g.objectToWorld));
     cudaStream_t st = swr_internal_stream();
     {

@@ -4,6 +4,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -230,7 +231,8 @@ void launch_finalize(const unsigned long long* keys, uint32_t* layer0, uint32_t*
 void launch_finalize_overdraw(const unsigned long long* keys, const unsigned long long* counts, uint32_t* layer0,
                               uint32_t* layer1, uint32_t n, cudaStream_t st);
 constexpr uint32_t kOctTable = 65536;
-void launch_oct_table(float4* table, cudaStream_t st);  // swr_shade.cu
+// The table on a stream of its own, waited for (swr_shade.cu).
+cudaError_t fill_oct_table(float4* table);
 void launch_detile(const uint32_t* src, const unsigned long long* keys, uint32_t* dst, uint32_t width, uint32_t height,
                    uint32_t stride, uint32_t layer, cudaStream_t st);
 
@@ -245,6 +247,7 @@ cudaStream_t swr_internal_stream();
 swr_status swr_internal_device(int* dev, int* sms);
 // SM count of the current device, 148 if the query fails (launch sizing only).
 int swr_internal_sm_count();
+unsigned long long swr_internal_context_id();  // of the current context, 0 if unknown (swr_noalloc.cu)
 // Profiling on/off for this thread (returns the previous state) and extra launches to count
 // (kernels replayed inside a CUDA graph).
 bool swr_internal_set_profiling(bool on);
@@ -285,7 +288,9 @@ struct swr_scene_t {
     bool hasAlpha;                 // some material selects FS_EncodeSurfaceId<true> (swr::material_alpha_tested)
     bool hasAlphaAll;              // some material is alpha-tested under FS_EncodeGBuffer (material_alpha_tested_all)
     uint8_t* fsIds;                // device: FragmentShaderId of each material under ShadeMeshlet
-    float4* octTable;              // device: unmap_oct of every 16-bit normal (with the first meshlets; nullptr: none)
+    // device: unmap_oct of every 16-bit normal, shared by the scenes of a device (with the first meshlets; none:
+    // the kernels compute what they read from it)
+    std::shared_ptr<float4> octTable;
     uint64_t version;              // bumped when meshlets or materials move (recorded draw graphs re-capture)
 };
 

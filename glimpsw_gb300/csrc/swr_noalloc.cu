@@ -15,6 +15,32 @@
 #include "swr_device.cuh"
 #include "swr_internal.h"
 
+using CtxGetCurrentFn = CUresult (*)(CUcontext*);
+using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long*);
+
+// Identity of the calling thread's current context (0 if none is current or the driver does not
+// tell: what was kept for a context is then made anew).
+unsigned long long swr_internal_context_id() {
+    static CtxGetCurrentFn getCurrent = nullptr;
+    static CtxGetIdFn getId = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            getCurrent = (CtxGetCurrentFn)f;
+        f = nullptr;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            getId = (CtxGetIdFn)f;
+    });
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    if (!getCurrent || !getId || getCurrent(&c) != CUDA_SUCCESS || !c || getId(c, &id) != CUDA_SUCCESS) return 0;
+    return id + 1;
+}
+
 namespace swr {
 namespace {
 
@@ -39,32 +65,6 @@ static __device__ __align__(256) unsigned char g_noallocScratch[kNoAllocBytes];
 // is looked up with the device current and cached per device, together with the identity of the
 // context it was looked up in. A cudaDeviceReset ends that context; the next call sees a new
 // context and looks the address up again.
-using CtxGetCurrentFn = CUresult (*)(CUcontext*);
-using CtxGetIdFn = CUresult (*)(CUcontext, unsigned long long*);
-
-// Identity of the calling thread's current context (0 if none is current or the driver does not
-// tell; the address is then looked up at every call).
-unsigned long long current_context_id() {
-    static CtxGetCurrentFn getCurrent = nullptr;
-    static CtxGetIdFn getId = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            getCurrent = (CtxGetCurrentFn)f;
-        f = nullptr;
-        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            getId = (CtxGetIdFn)f;
-    });
-    CUcontext c = nullptr;
-    unsigned long long id = 0;
-    if (!getCurrent || !getId || getCurrent(&c) != CUDA_SUCCESS || !c || getId(c, &id) != CUDA_SUCCESS) return 0;
-    return id + 1;
-}
-
 struct DeviceScratch {
     unsigned char* ptr;
     unsigned long long context;
@@ -79,13 +79,13 @@ swr_status scratch_for_current_device(unsigned char** out, int* sms) {
     if (st != SWR_OK) return st;
     std::lock_guard<std::mutex> lock(g_mu);
     DeviceScratch& d = g_scratch[dev];
-    const unsigned long long ctx = current_context_id();
+    const unsigned long long ctx = swr_internal_context_id();
     if (!d.ptr || ctx == 0 || ctx != d.context) {
         void* p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_noallocScratch);
         if (e != cudaSuccess) return swr_internal_cuda_fail(e, "swr_draw_meshlets_noalloc: cudaGetSymbolAddress");
         d.ptr = (unsigned char*)p;
-        d.context = current_context_id();  // the lookup made the context current if none was
+        d.context = swr_internal_context_id();  // the lookup made the context current if none was
     }
     *out = d.ptr;
     return SWR_OK;

@@ -696,9 +696,19 @@ __global__ void __launch_bounds__(256) k_resolve(const __grid_constant__ Resolve
 
 }  // namespace
 
-void launch_oct_table(float4* table, cudaStream_t st) {
-    LaunchScope ls("k_oct_table", st);
-    k_oct_table<<<kOctTable / 256, 256, 0, st>>>(table);
+cudaError_t fill_oct_table(float4* table) {
+    cudaStream_t st = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return e;
+    {
+        LaunchScope ls("k_oct_table", st);
+        k_oct_table<<<kOctTable / 256, 256, 0, st>>>(table);
+        e = cudaGetLastError();
+    }
+    const cudaError_t w = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = w;
+    cudaStreamDestroy(st);
+    return e;
 }
 }  // namespace swr
 
@@ -724,7 +734,7 @@ swr_status build_resolve_args(swr_framebuffer fb, const swr_shading_context* ctx
     a.numMeshlets = ctx->scene->count;
     a.materials = ctx->scene->materials;
     a.numMaterials = ctx->scene->num_materials;
-    a.octTable = ctx->scene->octTable;
+    a.octTable = ctx->scene->octTable.get();
     a.color = fb->layers;
     a.depth = (float*)(fb->layers + fb->layer_stride);
     a.width = fb->width, a.height = fb->height;
