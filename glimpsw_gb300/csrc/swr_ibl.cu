@@ -545,11 +545,13 @@ swr_status swr_ibl_irradiance_map(swr_texture env, swr_texture out) {
     static const IrradianceTables tb = irradiance_tables();
     cudaStream_t st = swr_internal_stream();
     const uint32_t n = out->d.width * out->d.height, blocks = (n + kIrrTexels - 1) / kIrrTexels;
-    // Every sample reads one level. Up to kSkyScratchTexels texels (4 MB unpacked, which the caches hold) it is
-    // unpacked first; a larger one is read as it is.
+    // Every sample reads one level. Up to kSkyScratchTexels texels (4 MB unpacked, which the caches hold) level 2 is
+    // unpacked first; a larger one, and the last level of a map without a level 2, is read as it is. Calls on several
+    // streams may unpack one map at once: each writes the same words, made of texels that no caller may change
+    // before all of them have read them.
     if (env->skyScratch) {
         uint4* texels = (uint4*)env->skyScratch;
-        const uint32_t level = std::min(2u, env->d.mip_levels - 1), count = ((env->d.width >> level) + 1) * (env->d.height >> level);
+        const uint32_t count = ((env->d.width >> 2) + 1) * (env->d.height >> 2);
         {
             LaunchScope ls("k_unpack_env", st);
             k_unpack_env<<<(count + 255) / 256, 256, 0, st>>>(env->d, texels);

@@ -299,8 +299,10 @@ struct swr_texture_t {
     uint32_t format;
     swr::DevTexture d;             // d.data is the device storage
     size_t words;
-    void* skyScratch;              // R11G11B10: room for its level 2 (or last) unpacked and padded, 16 bytes a texel, up
-                                   // to kSkyScratchTexels texels of a map of at most kSkyScratchSide a side (else nullptr)
+    void* skyScratch;              // R11G11B10: room for its level 2 unpacked and padded, 16 bytes a texel (a fifth more
+                                   // than the texture), where it has one, of up to kSkyScratchTexels texels in a map
+                                   // of at most kSkyScratchSide a side (else nullptr). A map of one or two levels, which
+                                   // the irradiance map's output is and a sky seldom, would take four times its own size.
 };
 
 struct swr_rasterizer_t {

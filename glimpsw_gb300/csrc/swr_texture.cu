@@ -170,8 +170,8 @@ swr_status swr_texture_create(uint32_t format, uint32_t width, uint32_t height, 
     const bool keep = format == SWR_FORMAT_RGBA8U && !shared;
     uint32_t* p = nullptr;
     const size_t alphaAt = (t->words + 3) & ~(size_t)3;
-    const uint32_t skyLevel = std::min(2u, mip - 1), skyW = width >> skyLevel, skyH = height >> skyLevel;
-    const bool sky = format == SWR_FORMAT_R11G11B10F && skyW * skyH <= kSkyScratchTexels && std::max(width, height) <= kSkyScratchSide;
+    const uint32_t skyW = width >> 2, skyH = height >> 2;
+    const bool sky = format == SWR_FORMAT_R11G11B10F && mip >= 3 && skyW * skyH <= kSkyScratchTexels && std::max(width, height) <= kSkyScratchSide;
     cudaError_t e = cudaMalloc(&p, (alphaAt + 16 + (sky ? 4 * (size_t)(skyW + 1) * skyH : 0)) * 4);
     if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, t->words * 4, swr_internal_stream());
     if (e == cudaSuccess) e = cudaMemsetAsync(p + alphaAt, 0, mip * 4, swr_internal_stream());  // texels start as 0
