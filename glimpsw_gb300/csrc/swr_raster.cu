@@ -896,7 +896,9 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
         curView = 0;
         __syncwarp();
     }
-    uint32_t nProcessed = 0, nRaster = 0, nClipped = 0;  // per warp, within 32 bits (< 2^21 meshlets x 128)
+    // per warp, within 32 bits: less than 2^21 meshlets x 128 in a view; thousands of warps share the less than 2^32
+    // positions x 128 of a batch, whose blocks add theirs in 64 bits
+    uint32_t nProcessed = 0, nRaster = 0, nClipped = 0;
     if (blockIdx.x == 0 && threadIdx.x == 0) a.s.control[8] = 0;  // the cursor of the chunk stage after this pass
 
     // Work items are fetched a group at a time: one contended atomic per group. A group's cull
@@ -955,7 +957,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
     };
     constexpr bool kPool = !kAlpha && !kSmall && !kOver;  // (the overdraw shader's pass loses by it, 159 -> 169 us)
     __shared__ uint32_t pool[kPool ? kPoolSlots : 1];
-    __shared__ uint32_t blockSums[kPool ? 4 : 1];  // the warps' counters, and how many have added theirs
+    __shared__ unsigned long long blockSums[kPool ? 4 : 1];  // the warps' counters, and how many have added theirs
     if constexpr (kPool) {
         if (threadIdx.x < 4) blockSums[threadIdx.x] = 0;
         for (uint32_t k = threadIdx.x; k < kPoolSlots; k += blockDim.x) pool[k] = kPoolFree;
@@ -1363,15 +1365,15 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
         } else {
             // one addition a block, by its last warp: the words share a line, which takes one at a time (1080p mesh
             // stage 340 -> 333 us)
-            if (nProcessed) atomicAdd(&blockSums[0], nProcessed);
-            if (nRaster) atomicAdd(&blockSums[1], nRaster);
-            if (nClipped) atomicAdd(&blockSums[2], nClipped);
+            if (nProcessed) atomicAdd(&blockSums[0], (unsigned long long)nProcessed);
+            if (nRaster) atomicAdd(&blockSums[1], (unsigned long long)nRaster);
+            if (nClipped) atomicAdd(&blockSums[2], (unsigned long long)nClipped);
             __threadfence_block();
-            if (atomicAdd(&blockSums[3], 1u) == (blockDim.x >> 5) - 1) {
+            if (atomicAdd(&blockSums[3], 1ull) == (blockDim.x >> 5) - 1) {
                 __threadfence_block();
-                const volatile uint32_t* sums = blockSums;
+                const volatile unsigned long long* sums = blockSums;
                 for (int k = 0; k < 3; k++)
-                    if (const uint32_t n = sums[k]) atomicAdd(&a.s.control[3 + k], (unsigned long long)n);
+                    if (const unsigned long long n = sums[k]) atomicAdd(&a.s.control[3 + k], n);
             }
         }
     }
