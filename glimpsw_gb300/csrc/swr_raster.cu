@@ -911,18 +911,26 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
     // Single view: positions per fetch. A draw of fewer meshlets than groups for every warp starts with
     // smaller groups, so that no warp draws several meshlets in a row while others have none.
     const uint32_t leastGroup = totalItems < 2 * numWarps ? 1u : 2u;
-    // Sparse: of 1024 positions sampled from the cull bitmap fewer than 32 are visible. Groups start at 32 then,
-    // which with the warps' own first groups takes 150,000 positions without a cursor (its contended atomics kept
-    // the warps from their first meshlet for 25,000 cycles and more), and every triangle above kSpreadTiles tiles is
-    // queued, as no other meshlets hide the few visible ones' serial steps: 213 of 150,000 visible, 67.6 -> 42.7 us
-    // (own first groups alone 62, with groups of 32 49); 100,000 mostly visible: no change.
+    // Sparse: of 1024 positions sampled from the cull bitmap few are visible. Groups start at 32 then, so that the
+    // warps' own first groups take 150,000 positions without a cursor (its contended atomics kept the warps from their
+    // first meshlet for 25,000 cycles and more), and every triangle above kSpreadTiles tiles is queued, as no other
+    // meshlets hide the few visible ones' serial steps: 213 of 150,000 visible, mesh stage 67.6 -> 42.7 us.
+    // "Few" depends on the positions a warp has: where the first groups take them all, nothing balances the visible
+    // ones between the blocks, and what is saved is soon lost; where most groups come from the cursor, it pays longer.
+    // Whole draws at 1280x720 and 2560x1440, mean us, sparse / not, by meshlets and visible share:
+    //             0.05 %      0.3 %       0.5 %       1 %         2 %         3 %
+    //    20,000   66 /  71    86 /  85    91 /  89   112 /  98   137 / 112   139 / 122
+    //   150,000   89 / 103   119 / 126   139 / 133   160 / 154   186 / 164   196 / 170
+    //   220,000   90 / 107   121 / 134   134 / 144   155 / 159   191 / 174   198 / 191
+    //   400,000  107 / 123   144 / 156   160 / 172   178 / 189   207 / 219   229 / 233
     uint32_t firstGroup = min(kDrawGroup, max(totalItems / numWarps, leastGroup));
     bool sparse = false;
     if (!kSmall && !kAlpha && !multi && a.cullBitmap && totalItems >= 1024) {
         const unsigned long long words = totalItems >> 4;
         unsigned seen = 0;
         for (uint32_t k = 2 * lane; k < 2u * lane + 2; k++) seen += __popc(a.cullBitmap[(uint32_t)((words * k) >> 6)]);
-        sparse = __reduce_add_sync(0xFFFFFFFFu, seen) < 32;
+        const unsigned few = totalItems > 64 * numWarps ? 32u : totalItems > 40 * numWarps ? 12u : 4u;
+        sparse = __reduce_add_sync(0xFFFFFFFFu, seen) < few;
         if (sparse) firstGroup = 32;
     }
     uint32_t fetchGroup = firstGroup;
