@@ -782,7 +782,15 @@ __device__ __noinline__ bool takes_alpha_pass(const DevMaterial* materials, uint
 // the view) lie in a box of tiles whose depth bounds are all above the nearest vertex (triangle_depth_bound of
 // the meshlet). The alpha pass finds 41 to 46 % of its meshlets hidden by the opaque pass and by each other: 94 ->
 // 77 us of a 1916x1036 frame from inside, 175 -> 144 us of a 1600x900 G-buffer.
-constexpr uint32_t kHiddenTiles = 512;  // larger boxes are not tested (16 loads a lane)
+// Larger boxes are not tested (256 loads a lane). Alpha pass + the chunk stage after it, us, by the limit in tiles:
+//                                               512          2048          8192          none
+//   50,000 meshlets, inside, 1916x1036       70 + 231      56 + 211      54 + 192      71 + 191
+//   30,000, G-buffer, 1600x900              125 + 171     109 + 163     109 + 133     109 + 131
+//   18,960, outside, 836x688                 89 + 110      85 +  87      85 +  86      85 +  87
+//   61,025, outside, 1188x1104               34 +  92      34 +  92      35 +  90      53 +  99
+//    1,960, inside, 2516x1168                27 + 170      28 + 169      29 + 166      47 + 137
+//   53,291, inside, 1160x1104                20 + 105      23 + 105      23 + 105      23 + 105
+constexpr uint32_t kHiddenTiles = 8192;
 __device__ __forceinline__ bool meshlet_hidden(const uint2* pz, uint32_t slots, const ViewParams& vp, int lane) {
     uint32_t lo = 0x7FFF7FFFu, hi = 0x80008000u, z = 0;
 #pragma unroll
