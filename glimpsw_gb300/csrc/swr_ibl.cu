@@ -60,7 +60,7 @@ __device__ __forceinline__ uint32_t pack_r11g11b10(F3 c) {
     return f11(c.x) << 21 | f11(c.y) << 10 | f10(c.z);
 }
 
-// Two values at a time with the packed FP32 instructions (sm_100): the same IEEE operations on each.
+// Two values at a time (__ffma2_rn, __fadd2_rn, __fmul2_rn): the same IEEE operations on each.
 // a + (b - a) f, rounded after each operation (b - a as the exact product's fma).
 __device__ __forceinline__ float2 lerp2(float2 a, float2 b, float f) {
     const float2 d = __ffma2_rn(a, make_float2(-1.0f, -1.0f), b);

@@ -98,8 +98,7 @@ __device__ __forceinline__ float gelu_and_grad(float x, float& d) {
 // inference kernel keeps its activations doubled and its next layer's weights halved (exact for
 // BF16 weights of normal magnitude), so the products, hence z2 and y, are those of gelu.
 constexpr float kGeluAB = kGeluA * kGeluB;
-// Two values at a time with the packed FP32 instructions (FMUL2 / FFMA2, sm_100): the same IEEE operations on
-// each value, in half the instructions.
+// Two values at a time (__fmul2_rn, __ffma2_rn): the same IEEE operations on each value.
 __device__ __forceinline__ float2 gelu_x2_pair(float2 x) {
     const float2 p = __ffma2_rn(make_float2(kGeluAB, kGeluAB), __fmul2_rn(x, x), make_float2(kGeluA, kGeluA));
     const float2 u = __fmul2_rn(x, p);

@@ -25,6 +25,14 @@
 // tile is shaded, an upper bound of the triangle's depth over the tile is compared with it; a tile
 // the triangle cannot win anywhere is skipped. The vis-buffer is unchanged (only fragments that
 // would fail the depth test are skipped), while the dense scenes' overdraw mostly disappears.
+//
+// Figures of the form a -> b beside a choice are of that choice alone, on the kernels as they were then: later
+// choices moved both. The kernels as they are (us, SM at 2070 MHz):
+//   1080p frame of 100k meshlets: mesh stage 333, chunk stage 151; 24 views of 100k meshlets in a batch: 1231, 221
+//   inside a 50k-meshlet scene, half of the materials alpha-tested, 1916x1036: mesh stage 126, opaque chunks 125,
+//   alpha pass 54, its chunks 199; G-buffer draw of 30k, 1600x900: 140, 80, 112, 127
+//   overdraw draw of 20k, 1280x720: 160, 148; 150k meshlets culled against the Hi-Z, 2560x1440: 43, 81
+//   1024 meshlets at 1280x720: 30, 15; 60 at 252x140: 9.2, 7.5
 #include <algorithm>
 #include <cfloat>
 #include <mutex>
@@ -151,10 +159,9 @@ __device__ __forceinline__ uint32_t row_magic(int n) {
 }
 
 // The terms of a triangle's tile tests that do not depend on the tile, computed once per triangle (in
-// the mesh stage by the lane that sets it up, in the chunk stage when a run enters the triangle): with
-// them a tile costs six multiply-adds, one sign test, two conversions and two fmas (opaque chunk stage within
-// noise, the compiler had moved most of the rest to the uniform path; alpha-tested chunks 629 -> 608 us of a
-// 1916x1036 frame, 24-view batched mesh stage 1.47 -> 1.45 ms).
+// the mesh stage by the lane that sets it up, in the chunk stage before a chunk's tiles): with them a tile costs six
+// multiply-adds, one sign test, two conversions and two fmas (alpha-tested chunks 629 -> 608 us of a
+// 1916x1036 frame, 24-view batched mesh stage 1.47 -> 1.45 ms; opaque chunk stage no change).
 //
 // F is the edge value at pixel (0, 0) plus the edge's largest increase over a 4x4 tile, so the tile at
 // (px, py) holds a sample inside the edge only if F + A px + B py >= 0 (wrapping as the shading's).
@@ -462,9 +469,6 @@ __device__ __forceinline__ bool tile_live(const TriRec& r, const TileTest& t, ui
     return ((uint32_t)max(__float_as_int(fminf(b, zmax)), 0) | 0x80000000u) >= *known;
 }
 
-// Shades the live tiles of the warp-wide candidate set (the lanes in `mask` hold a tile origin
-// tpx/tpy, its depth bound tmin and a triangle selector rsel for rec()), two tiles per step, and
-// raises the tiles' depth bounds.
 // The key DrawTriangle + FS_EncodeSurfaceId<false> (Rasterizer.h:287-323, Shading.cpp:309-331)
 // offers for pixel (tx + l % 4, ty + l / 4) of the 4x4 tile at the 4-aligned (tx, ty), 0 if the
 // sample is outside the triangle or its depth is NaN. The tiled key offset is the tile's base
@@ -591,7 +595,7 @@ __device__ __forceinline__ bool raster_region_with(const TriRec& r, const TileTe
     return any;
 }
 
-// raster_region_with for an opaque triangle, two tiles per step.
+// raster_region_with for an opaque triangle, four tiles per step.
 __device__ __forceinline__ bool raster_region(const TriRec& r, const TileTest& tt, uint32_t x0, uint32_t y0, int tilesX, int tilesY,
                                               unsigned long long* keys, uint32_t* tileMin, uint32_t width, int lane, uint32_t readTiles,
                                               uint4* list, uint32_t divMagic = 0) {
@@ -603,7 +607,7 @@ __device__ __forceinline__ bool raster_region(const TriRec& r, const TileTest& t
                        }, divMagic);
 }
 
-// The same for the alpha-tested triangle *rp with alpha terms *xp (material texture tex, cutoff << 24).
+// The same for the alpha-tested triangle *rp with alpha terms *xp (material texture tex, alpha cutoff).
 __device__ __forceinline__ bool raster_region_alpha(const TriRec* rp, const TileTest& tt, const AlphaExt* xp, const DevTexture& tex,
                                                     uint32_t cutoff, uint32_t x0, uint32_t y0, int tilesX, int tilesY,
                                                     unsigned long long* keys, uint32_t* tileMin, uint32_t width, int lane,
@@ -770,8 +774,8 @@ struct WarpSmemAlpha : WarpSmem {
 };
 
 // True if a meshlet of material mat goes to the alpha pass. Out of line: it is run once per 32 positions of
-// scenes with alpha-tested materials, and inline it moved the mesh stage's loop across the instruction
-// cache's reach (24 batched views without such materials: 1281 -> 1492 us).
+// scenes with alpha-tested materials, and inline it slowed draws without any (24 batched views: mesh stage
+// 1281 us out of line, 1492 inline).
 __device__ __noinline__ bool takes_alpha_pass(const DevMaterial* materials, uint32_t numMaterials, uint32_t mat, bool all) {
     if (mat == 0xFFFFFFFFu || mat >= numMaterials) return false;
     const DevMaterial& m = materials[mat];
@@ -954,8 +958,8 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
     bool ownTaken = false;  // a pass's first group is the warp's own, later ones come from the cursor
     // Opaque pass of a scene with alpha-tested materials: a fetched group's alpha-tested meshlets go to the
     // alpha pass's list with one atomic, before their records are read (a draw of alpha-tested meshlets alone:
-    // 45 -> 27 us;a shaded meshlet's FragmentShaderId is only known from its
-    // record, and is looked at later). Returns the lanes left to draw.
+    // 45 -> 27 us). A shaded meshlet's FragmentShaderId is only known from its record, and is looked at
+    // later. Returns the lanes left to draw.
     constexpr bool kSplitAlpha = kPass == kPassOpaque && !kShaded;
     auto split_alpha = [&](unsigned mask, uint32_t meshlet, uint32_t item) -> unsigned {
         bool alpha = false;
@@ -1147,7 +1151,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
         // ShadeMeshlet vertex loop (Shading.cpp:295-298): 16-vertex chunks up to NumVertices; the
         // slots past them are zero. What the triangles need of a vertex alone is computed here, once
         // instead of in about six triangles: the projection, the snapped position and the clip codes.
-        // The stage is bound by instruction issue (64-69 % of the slots, 270 M instructions in the 1080p frame
+        // The stage is bound by instruction issue (68 % of the slots, 263 M instructions in the 1080p frame
         // of 100k meshlets): with the positions snapped per vertex, packed index bytes, the clip codes
         // skipped for a meshlet inside the view and the tile owners found by ballots, 379 -> 355 us there,
         // 24 batched views 1.44 -> 1.31 ms.
@@ -1303,8 +1307,8 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
             const AlphaExt* ext = nullptr;
             if constexpr (kAlpha) ext = &S.exts[lane].v;
             if (!enqueue_warp<kAlpha>(queue, tris[lane].v, ext, a, chunk, lane)) {
-                // The full queue turned it away: its tiles join the warp's list, however many they are. (A second
-                // copy of the tile loop for it cost the loop's place in the instruction cache.)
+                // The full queue turned it away: its tiles join the warp's list, however many they are. (With a second
+                // copy of the tile loop for it the batched mesh stage took 1281 us instead of 1276.)
                 TriRec& r = tris[lane].v;
                 myTiles = (int)triangle_tiles(r);
                 r.pad = kPadWide | kPadReadKey;
@@ -1312,8 +1316,8 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                 S.zmax[lane] = __int_as_float(0x7F800000);
             }
 
-            // Small triangles: the warp walks the concatenated tile lists of all of them, two
-            // tiles (32 pixels) per step, so tiny triangles share steps.
+            // Small triangles: the warp walks the concatenated tile lists of all of them, four
+            // tiles (64 pixels) per step, so tiny triangles share steps.
             int incl = myTiles;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -1326,7 +1330,7 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
             if (myTiles > 0) S.order[__popc(owners & ((1u << lane) - 1u))] = (uint8_t)lane;
             __syncwarp();
             // 32 tiles at a time: lane j tests tile b + j of the list (empty or hidden tiles are
-            // dropped), then the live ones are shaded two per step.
+            // dropped), then the live ones are shaded four per step.
             const uint32_t tw = vp.width >> 2;
             for (int b = 0; b < total; b += 32) {
                 const int t = b + lane;
@@ -1419,7 +1423,7 @@ constexpr uint32_t kChunkRun = 8, kChunkRunAlpha = 4;
 constexpr uint32_t kRunsPerWarp = 8;
 
 // Per 32x32-pixel block, a lower bound of the tile depth bounds inside it, in the words after the tile
-// bounds (tile_bounds_words): one load tells a chunk's lane that the whole block is nearer. The bounds are
+// bounds (tile_blocks): one load tells a chunk's lane that the whole block is nearer. The bounds are
 // only refreshed where they proved too loose: a chunk that passed them and then had no live tile raises
 // the blocks it touches to the minimum of their 64 tiles (tile bounds only grow, so a stale block
 // bound stays a bound).
