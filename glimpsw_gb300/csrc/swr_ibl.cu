@@ -36,10 +36,12 @@ struct IrradianceTables {
     float cosTheta[kMaxTheta], sinTheta[kMaxTheta];  // cosf(theta), sinf(theta) of each theta step
     uint32_t numPhi, numTheta;
     float scale;                                     // simd::pi * 1.0f / sampleCount
+    float one;                                       // 1 (round_sum)
 };
 template <uint32_t N>
 struct HammersleyTable {
     float t[3 * N];  // Hammersley(i, N): Xi.y, cos(phi), sin(phi) with phi = 2 pi Xi.x
+    float one;       // 1 (round_sum)
 };
 
 __device__ __forceinline__ float unpack_f11_(uint32_t x) { x <<= 17; return __uint_as_float((x & 0x0FFE0000u) + 0x38000000u); }
@@ -60,11 +62,15 @@ __device__ __forceinline__ uint32_t pack_r11g11b10(F3 c) {
     return f11(c.x) << 21 | f11(c.y) << 10 | f10(c.z);
 }
 
-// Two values at a time (__ffma2_rn, __fadd2_rn, __fmul2_rn): the same IEEE operations on each.
+// Two values at a time (__ffma2_rn, __fmul2_rn): the same IEEE operations on each.
+// a + p for a product p, each rounded. A packed product that feeds a packed addition comes out as one fma, whatever
+// -fmad says (measured: __fadd2_rn(a, __fmul2_rn(b, c)) equals fma(b, c, a) on 1.6 million random operands, and
+// add.rn.f32x2 of mul.rn.f32x2 does, too): the sum is a fma with a one that only the launch knows.
+__device__ __forceinline__ float2 round_sum(float2 a, float2 p, float one) { return __ffma2_rn(p, make_float2(one, one), a); }
 // a + (b - a) f, rounded after each operation (b - a as the exact product's fma).
-__device__ __forceinline__ float2 lerp2(float2 a, float2 b, float f) {
+__device__ __forceinline__ float2 lerp2(float2 a, float2 b, float f, float one) {
     const float2 d = __ffma2_rn(a, make_float2(-1.0f, -1.0f), b);
-    return __fadd2_rn(a, __fmul2_rn(d, make_float2(f, f)));
+    return round_sum(a, __fmul2_rn(d, make_float2(f, f)), one);
 }
 
 // One level of an environment map as the sampler reads it.
@@ -83,7 +89,7 @@ __device__ __forceinline__ EnvLevel env_level(const DevTexture& t, int32_t mipIn
 
 // SampleLevel<EnvSampler> (Texture.h:412-459: ClampToEdge, linear in both directions) of an
 // R11G11B10 texture at (u, v) on one level, with SampleLinear's float path (Texture.h:506-575).
-__device__ __forceinline__ F3 sample_env_level(const DevTexture& t, const EnvLevel& e, float u, float v) {
+__device__ __forceinline__ F3 sample_env_level(const DevTexture& t, const EnvLevel& e, float u, float v, float one) {
     // round2i without its range checks: a NaN gives 0 here instead of INT_MIN and clamps to the same 0, and u and
     // v lie in [0, 1] otherwise
     const int32_t ix = min(max(__float2int_rn(u * t.scale_lerp_u), 0), t.mask_lerp_u) >> e.m;
@@ -96,10 +102,10 @@ __device__ __forceinline__ F3 sample_env_level(const DevTexture& t, const EnvLev
     const F3 c01 = unpack_r11g11b10(e.base[i01]), c11 = unpack_r11g11b10(e.base[i01 + 8]);
     const float fs = 1.0f / 256;
     const float fx = inX ? (float)(xf & 255) * fs : 0.0f, fy = (float)(yf & 255) * fs;
-    const float2 ra = lerp2(make_float2(c00.x, c00.y), make_float2(c10.x, c10.y), fx);
-    const float2 rb = lerp2(make_float2(c01.x, c01.y), make_float2(c11.x, c11.y), fx);
-    const float2 rz = lerp2(make_float2(c00.z, c01.z), make_float2(c10.z, c11.z), fx);
-    const float2 r = lerp2(ra, rb, fy);
+    const float2 ra = lerp2(make_float2(c00.x, c00.y), make_float2(c10.x, c10.y), fx, one);
+    const float2 rb = lerp2(make_float2(c01.x, c01.y), make_float2(c11.x, c11.y), fx, one);
+    const float2 rz = lerp2(make_float2(c00.z, c01.z), make_float2(c10.z, c11.z), fx, one);
+    const float2 r = lerp2(ra, rb, fy, one);
     return { r.x, r.y, rz.x + (rz.y - rz.x) * fy };
 }
 
@@ -130,14 +136,14 @@ __device__ __forceinline__ int32_t env_coordinate(float s, int32_t mask, int32_t
 }
 // sample_env_level from them.
 __device__ __forceinline__ void sample_env_unpacked(const DevTexture& t, const EnvLevel& e, const uint4* __restrict__ texels, float u, float v,
-                                                    float2& xy, float& z) {
+                                                    float one, float2& xy, float& z) {
     float fx, fy;
     const int32_t tx = env_coordinate(u * t.scale_lerp_u, t.mask_lerp_u, e.m, fx);
     const int32_t ty = env_coordinate(v * t.scale_lerp_v, t.mask_lerp_v, e.m, fy);
     const uint4* p = texels + (uint32_t)(ty * (e.width + 1) + tx);
     const uint4 l = p[0], r = p[1];
-    xy = lerp2(lerp2(unpacked_xy(l.x), unpacked_xy(r.x), fx), lerp2(unpacked_xy(l.y), unpacked_xy(r.y), fx), fy);
-    const float2 rz = lerp2(unpacked_z(l), unpacked_z(r), fx);
+    xy = lerp2(lerp2(unpacked_xy(l.x), unpacked_xy(r.x), fx, one), lerp2(unpacked_xy(l.y), unpacked_xy(r.y), fx, one), fy, one);
+    const float2 rz = lerp2(unpacked_z(l), unpacked_z(r), fx, one);
     z = rz.x + (rz.y - rz.x) * fy;
 }
 
@@ -158,14 +164,14 @@ __device__ __forceinline__ void map_oct_unit(F3 n, float& u, float& v, const uin
 }
 
 // SampleOctLevel<EnvSampler> (Texture.h:467-480): between mips trunc(level) and trunc(level) + 1.
-__device__ __forceinline__ F3 sample_oct_level(const DevTexture& t, F3 dir, float level) {
+__device__ __forceinline__ F3 sample_oct_level(const DevTexture& t, F3 dir, float level, float one) {
     float u, v;
     map_oct(dir, u, v);
     const int32_t baseMip = trunc2i(level);
-    const F3 b = sample_env_level(t, env_level(t, baseMip), u, v);
+    const F3 b = sample_env_level(t, env_level(t, baseMip), u, v, one);
     const float frac = level - (float)baseMip;
     if (frac > 0.0f && baseMip < (int32_t)t.mip_levels - 1) {
-        const F3 l = sample_env_level(t, env_level(t, baseMip + 1), u, v);
+        const F3 l = sample_env_level(t, env_level(t, baseMip + 1), u, v, one);
         return { b.x + (l.x - b.x) * frac, b.y + (l.y - b.y) * frac, b.z + (l.z - b.z) * frac };
     }
     return b;
@@ -284,7 +290,7 @@ __device__ __forceinline__ void gather_sums(float acc, uint32_t t, float (&sum)[
 // SMs, each with a barrier every two samples of a warp): 1.47 -> 1.01 ms for 133 M samples. Bound by instruction
 // issue (67 % of the slots, about 160 operations a sample) and by the texel loads' lines (75 % of the load
 // unit): the texels with both rows in 16 bytes, the phi steps' rows made by one warp, four sums a read
-// and reciprocals without their special cases, 1.01 -> 0.83 ms. 6 compute warps 0.94 ms, 10 0.84; a warp over two phi steps at once
+// and reciprocals without their special cases, 1.01 -> 0.84 ms. 6 compute warps 0.94 ms, 10 0.84; a warp over two phi steps at once
 // 0.85; 8 texels a block was slower (1.07 against 1.01); with the level read as it is packed (a larger map) 0.94.
 constexpr int kIrrWarps = 8, kIrrTexels = 4;
 constexpr int kIrrRows = 2;  // phi steps a chunk
@@ -340,16 +346,16 @@ __global__ void __launch_bounds__((kIrrWarps + 1) * 32) k_ibl_irradiance(const _
             const float4 a = row[second ? 1 : 0][threadIdx.x % kIrrTexels];
             const float2 cs = theta[second ? k - tb.numTheta : k];
             const float ct = cs.x, st = cs.y;
-            const float2 d = __fadd2_rn(__fmul2_rn(make_float2(ct, ct), make_float2(N.x, N.y)),
-                                        __fmul2_rn(make_float2(st, st), make_float2(a.x, a.y)));
+            const float2 d = round_sum(__fmul2_rn(make_float2(ct, ct), make_float2(N.x, N.y)),
+                                       __fmul2_rn(make_float2(st, st), make_float2(a.x, a.y)), tb.one);
             const F3 dir = { d.x, d.y, ct * N.z + st * a.z };
             float su, sv, z;
             float2 xy;
             map_oct_unit(dir, su, sv, segments);
             if constexpr (kUnpacked) {
-                sample_env_unpacked(env, level, texels, su, sv, xy, z);
+                sample_env_unpacked(env, level, texels, su, sv, tb.one, xy, z);
             } else {
-                const F3 s = sample_env_level(env, level, su, sv);
+                const F3 s = sample_env_level(env, level, su, sv, tb.one);
                 xy = make_float2(s.x, s.y), z = s.z;
             }
             // tonemap_sample, then times cos(theta) sin(theta)
@@ -404,7 +410,7 @@ __global__ void __launch_bounds__((kRadWarps + 1) * 32) k_ibl_radiance(const __g
                 const float pdf = d_ggx(NoH, roughness) / 4.0f + 0.001f;
                 const float omegaS = 1.0f / ((float)numSamples * pdf);
                 const float mip = vmax(0.5f * approx_log2(omegaS / omegaP), 0.0f);
-                const F3 c = tonemap_sample(sample_oct_level(env, L, mip), 1.0f);
+                const F3 c = tonemap_sample(sample_oct_level(env, L, mip, ham.one), 1.0f);
                 t[0] = c.x * NoL, t[1] = c.y * NoL, t[2] = c.z * NoL, t[3] = NoL;
             }
         });
@@ -493,6 +499,7 @@ void sincos_2pi(float x, float& s, float& c) {
 template <uint32_t n>
 HammersleyTable<n> hammersley_table() {
     HammersleyTable<n> h;
+    h.one = 1.0f;
     for (uint32_t i = 0; i < n; i++) {
         uint32_t bits = i;
         bits = (bits << 16) | (bits >> 16);
@@ -520,6 +527,7 @@ IrradianceTables irradiance_tables() {
     for (float theta = 0.0f; theta < halfPi && t.numTheta < kMaxTheta; theta += deltaTheta, t.numTheta++)
         t.cosTheta[t.numTheta] = cosf(theta), t.sinTheta[t.numTheta] = sinf(theta);
     t.scale = kPi * 1.0f / (float)(t.numPhi * t.numTheta);
+    t.one = 1.0f;
     return t;
 }
 
