@@ -163,17 +163,21 @@ swr_status swr_texture_create(uint32_t format, uint32_t width, uint32_t height, 
     d.scale_lerp_u = (float)(d.mask_lerp_u + 1), d.scale_lerp_v = (float)(d.mask_lerp_v + 1);
     t->format = format;
     t->words = (size_t)stride * num_layers + 64;
-    // The least-alpha words follow the storage. A level 4 texels high and more than 8 wide spreads its texels
-    // past its storage (TiledY8 columns hold 8 rows): what its words hold is not kept.
-    bool shared = false;
-    for (uint32_t l = 0; l < mip; l++) shared = shared || ((height >> l) < 8 && (width >> l) > 8);
+    // A level 4 texels high (the last, if any) has columns of 8 rows all the same, and wider than 8 its texels reach past
+    // its words: into the next layer's, as in the reference, and past the last layer's end, where there is room for
+    // them (and for a right neighbour) before anything else.
+    const uint32_t last = mip - 1;
+    const bool shared = (height >> last) < 8 && (width >> last) > 8;
+    const size_t reach = (size_t)stride * (num_layers - 1) + d.mip_offsets[last] + 8 * (size_t)(width >> last) + 64;
+    const size_t held = shared ? std::max(t->words, reach) : t->words;
+    // The least-alpha words follow; where levels share words, what those hold is not kept.
     const bool keep = format == SWR_FORMAT_RGBA8U && !shared;
     uint32_t* p = nullptr;
-    const size_t alphaAt = (t->words + 3) & ~(size_t)3;
+    const size_t alphaAt = (held + 3) & ~(size_t)3;
     const uint32_t skyW = width >> 2, skyH = height >> 2;
     const bool sky = format == SWR_FORMAT_R11G11B10F && mip >= 3 && skyW * skyH <= kSkyScratchTexels && std::max(width, height) <= kSkyScratchSide;
     cudaError_t e = cudaMalloc(&p, (alphaAt + 16 + (sky ? 4 * (size_t)(skyW + 1) * skyH : 0)) * 4);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, t->words * 4, swr_internal_stream());
+    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, held * 4, swr_internal_stream());
     if (e == cudaSuccess) e = cudaMemsetAsync(p + alphaAt, 0, mip * 4, swr_internal_stream());  // texels start as 0
     if (e == cudaSuccess && mip < 16) e = cudaMemsetAsync(p + alphaAt + mip, 0xFF, (16 - mip) * 4, swr_internal_stream());
     if (e != cudaSuccess) {
