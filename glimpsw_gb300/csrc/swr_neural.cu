@@ -149,7 +149,8 @@ __device__ __forceinline__ Taps latent_taps(const NeuralDev& n, Sample s) {
     return q;
 }
 // v = (c00 (1-fx) + c10 fx)(1-fy) + (c01 (1-fx) + c11 fx) fy, per channel, in this order.
-// Two channels at a time with the packed FP32 instructions: the same operations per channel.
+// Two channels at a time. A packed product that feeds a packed sum is not rounded on its own (swr_ibl.cu, round_sum):
+// each sum of two products here is an fma of the first with the second's product. Training and decoding share it.
 __device__ __forceinline__ void interpolate(const float (&c)[4][8], float fx, float fy, float* x0) {
     const float gx = 1.0f - fx, gy = 1.0f - fy;
     const float2 GX = make_float2(gx, gx), FX = make_float2(fx, fx), GY = make_float2(gy, gy), FY = make_float2(fy, fy);
