@@ -225,12 +225,21 @@ __global__ void __launch_bounds__(1024) k_hiz_tail(uint32_t fbW, uint32_t fbH, u
     }
 }
 
-// One level's texels (w x h, as written) from a scratch pyramid to the texture.
-__global__ void __launch_bounds__(256) k_hiz_place(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t w, uint32_t h,
-                                                   int32_t stride) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < w * h; i += gridDim.x * blockDim.x) {
-        const uint32_t o = texel_offset((int32_t)(i % w), (int32_t)(i / w), stride);
-        dst[o] = src[o];
+// One level's texels (cols x rows, as written) from a scratch pyramid to a texture whose words several of them may share:
+// a texel's word is (y & 7) | x << 3 | (y & ~7) << stride, and in a texture narrower than what is written
+// x and the bands of 8 rows overlap. The reference writes bands in order and texels from left to right: of
+// the texels of a word the one of the last band, and there of the last column, stays.
+__global__ void __launch_bounds__(256) k_hiz_place(const uint32_t* __restrict__ src, int32_t srcStride, uint32_t* __restrict__ dst,
+                                                   int32_t stride, uint32_t cols, uint32_t rows) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < cols * rows; i += gridDim.x * blockDim.x) {
+        const uint32_t x = i % cols, y = i / cols, band = y >> 3, low = x & ((1u << stride) - 1u);
+        const uint32_t word = (x >> stride) | band;  // the bits that columns and bands share
+        uint32_t last = (rows + 7) / 8 - 1;
+        while (last > band && ((last & ~word) || ((word & ~last) << stride | low) >= cols)) last--;
+        uint32_t column = (cols - 1) >> stride;
+        while (((column << stride | low) >= cols) || (column & ~word) || ((column | last) != word)) column--;
+        if (last == band && column == x >> stride)
+            dst[texel_offset((int32_t)x, (int32_t)y, stride)] = src[texel_offset((int32_t)x, (int32_t)y, srcStride)];
     }
 }
 
@@ -865,23 +874,35 @@ swr_status swr_downsample_depth(swr_framebuffer fb, swr_texture dest) {
         if (stride < 0 || mipOff(m) + 7 + (maxX << 3) + (maxY << stride) >= dest->words)
             return swr_internal_fail(SWR_EINVAL, "swr_downsample_depth: destination too small for this framebuffer");
     }
-    // The tail's levels that the texture lacks land at its start level by level, after the local kernel's, which it has.
-    // A texture with fewer of those (below 4 levels: the tail cannot hold more) gets its levels from a scratch
-    // pyramid that has them all, one launch a level: blocks writing them at once would leave the words they
-    // share to whichever came last.
+    // The levels above k_hiz_local's that the texture lacks land at its start one after the other (k_hiz_tail). Where more
+    // words are shared, blocks writing them at once would leave them to whichever came last: by the lower levels of
+    // a texture of fewer than 4, by the texels of a level wider than the texture's, or by a level that reaches into
+    // the next. Such a texture gets its levels from a scratch pyramid in which nothing is shared, one launch a level.
     const uint32_t levels = dest->d.mip_levels;
-    const bool place = levels < std::min(root - 3, 4u);
+    bool place = levels < std::min(root - 3, 4u);
+    uint32_t columns = 8;
+    for (uint32_t m = 0; m + 3 <= root; m++) {
+        uint32_t rx, ry, bt;
+        blocks(m, rx, ry, bt);
+        const uint32_t side = bt == 64 ? 8 : 4, cols = rx * side, rows = ry * side, stride = dest->d.row_shift - m;
+        columns = std::max(columns, cols << m);
+        place = place || (cols > 1u << stride && rows > 8);
+        const uint64_t end = 8 * (uint64_t)cols + ((uint64_t)((rows - 1) & ~7u) << stride);
+        place = place || (m + 1 < levels && m + 4 <= root && end > dest->d.mip_offsets[m + 1] - dest->d.mip_offsets[m]);
+    }
     HizOffsets offs = {};
     uint32_t* pyramid = tex;
+    int32_t rowShift = (int32_t)dest->d.row_shift;
     cudaError_t e = cudaSuccess;
     if (place) {
+        rowShift = 32 - __builtin_clz(columns - 1);  // as wide as the widest level
         size_t words = 0;
         for (uint32_t m = 0; m + 3 <= root; m++) {
             uint32_t rx, ry, bt;
             blocks(m, rx, ry, bt);
             const uint32_t side = bt == 64 ? 8 : 4;
             offs.off[m] = (uint32_t)words;
-            words += (((((size_t)rx * side - 1) << 3) + (((size_t)ry * side - 1) << (dest->d.row_shift - m)) + 7) | 63) + 1;
+            words += (size_t)((ry * side + 7) / 8) << (rowShift - (int32_t)m + 3);
         }
         e = cudaMallocAsync(&pyramid, words * sizeof(uint32_t), st);
         if (e != cudaSuccess) return swr_internal_cuda_fail(e, "swr_downsample_depth: scratch");
@@ -894,7 +915,7 @@ swr_status swr_downsample_depth(swr_framebuffer fb, swr_texture dest) {
         // whole blocks of the highest level
         const uint32_t side = std::max(kHizRegion, 8u << nLocal), per = side / kHizRegion;
         const dim3 grid((fb->width + side - 1) / side * per, (fb->height + side - 1) / side * per);
-        k_hiz_local<<<grid, 1024, 0, st>>>(depth, fb->width, fb->height, pyramid, offs, (int32_t)dest->d.row_shift, nLocal);
+        k_hiz_local<<<grid, 1024, 0, st>>>(depth, fb->width, fb->height, pyramid, offs, rowShift, nLocal);
     }
     if (root - 3 >= nLocal) {
         size_t smem = 0;  // levels nLocal-1 .. root-3, texels whose origin lies in the frame
@@ -902,17 +923,17 @@ swr_status swr_downsample_depth(swr_framebuffer fb, swr_texture dest) {
             smem += (size_t)hiz_extent(fb->width, m) * hiz_extent(fb->height, m) * sizeof(float);
         if (smem > 48 * 1024) cudaFuncSetAttribute(k_hiz_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         LaunchScope ls("k_hiz_tail", st);
-        k_hiz_tail<<<1, 1024, smem, st>>>(fb->width, fb->height, pyramid, offs, (int32_t)dest->d.row_shift, nLocal, root - 3,
+        k_hiz_tail<<<1, 1024, smem, st>>>(fb->width, fb->height, pyramid, offs, rowShift, nLocal, root - 3,
                                            root);
     }
     if (place) {
         for (uint32_t m = 0; m + 3 <= root; m++) {
             uint32_t rx, ry, bt;
             blocks(m, rx, ry, bt);
-            const uint32_t side = bt == 64 ? 8 : 4, w = rx * side, h = ry * side;
+            const uint32_t side = bt == 64 ? 8 : 4, cols = rx * side, rows = ry * side;
             LaunchScope ls("k_hiz_place", st);
-            k_hiz_place<<<std::min((w * h + 255) / 256, 1216u), 256, 0, st>>>(pyramid + offs.off[m], tex + mipOff(m), w, h,
-                                                                             (int32_t)(dest->d.row_shift - m));
+            k_hiz_place<<<std::min((cols * rows + 255) / 256, 1216u), 256, 0, st>>>(
+                pyramid + offs.off[m], rowShift - (int32_t)m, tex + mipOff(m), (int32_t)(dest->d.row_shift - m), cols, rows);
         }
         e = cudaGetLastError();
         cudaFreeAsync(pyramid, st);
