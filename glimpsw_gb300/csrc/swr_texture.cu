@@ -177,9 +177,9 @@ swr_status swr_texture_create(uint32_t format, uint32_t width, uint32_t height, 
     const uint32_t skyW = width >> 2, skyH = height >> 2;
     const bool sky = format == SWR_FORMAT_R11G11B10F && mip >= 3 && skyW * skyH <= kSkyScratchTexels && std::max(width, height) <= kSkyScratchSide;
     cudaError_t e = cudaMalloc(&p, (alphaAt + 16 + (sky ? 4 * (size_t)(skyW + 1) * skyH : 0)) * 4);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, held * 4, swr_internal_stream());
-    if (e == cudaSuccess) e = cudaMemsetAsync(p + alphaAt, 0, mip * 4, swr_internal_stream());  // texels start as 0
-    if (e == cudaSuccess && mip < 16) e = cudaMemsetAsync(p + alphaAt + mip, 0xFF, (16 - mip) * 4, swr_internal_stream());
+    // texels start as 0, and so do their levels' least alphas
+    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, (keep ? alphaAt + mip : held) * 4, swr_internal_stream());
+    if (e == cudaSuccess && keep && mip < 16) e = cudaMemsetAsync(p + alphaAt + mip, 0xFF, (16 - mip) * 4, swr_internal_stream());
     if (e != cudaSuccess) {
         cudaFree(p);
         delete t;
