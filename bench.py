@@ -356,9 +356,9 @@ def peaks():
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of the frame's kernels, from
 # one ncu capture of the default workload drawn in one call (100k meshlets, 1920x1080; the capture
-# used 256^2 textures, which changes only the resolve's texel addresses): k_draw_meshlets 108.83 MB
-# read + 22.18 MB written, k_raster_big 52.39 + 0.42 MB, k_resolve 27.26 MB.
-NCU_DRAM_BYTES_PER_LAUNCH = {"k_draw_meshlets": 131.01e6, "k_raster_big": 52.81e6, "k_resolve": 27.26e6}
+# used 256^2 textures, which changes only the resolve's texel addresses): k_draw_meshlets 113.79 MB
+# read + 25.88 MB written, k_raster_big 51.82 + 0.45 MB, k_resolve 27.42 + 0.02 MB.
+NCU_DRAM_BYTES_PER_LAUNCH = {"k_draw_meshlets": 139.66e6, "k_raster_big": 52.27e6, "k_resolve": 27.44e6}
 NCU_WORKLOAD = (100_000, 1920, 1080)
 
 
