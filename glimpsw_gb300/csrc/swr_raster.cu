@@ -955,7 +955,13 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
     // 10,000 by two: 143 -> 128 us; by four 128, and 7,200 of another 84 instead of 72 us).
     constexpr bool kParts = kSmall || kAlpha;
     const uint32_t partShift = kSmall ? a.partShift : kAlpha ? (totalItems < numWarps ? 2u : totalItems < 4 * numWarps ? 1u : 0u) : 0u;
-    bool ownTaken = false;  // a pass's first group is the warp's own, later ones come from the cursor
+    // A pass's first group is the warp's own, later ones come from the cursor, where those first groups take at most a
+    // quarter of the positions (or the draw is sparse; the overdraw shader's pass gains by it at any size). In smaller
+    // draws all come from the cursor: own groups of 4 hand out 20,000 positions at once, and the warps with costly
+    // ones end last (20,000 meshlets at 64x36 84 us with own groups, 68 without, 16x8 80 and 62, 320x180 125 and 113;
+    // 50,000 at 64x36 116 and 106; 60,000 at 2560x1440 860 and 837 of a frame; 100,000 at 1920x1080 618 and 623).
+    const bool ownFirst = kAlpha || kOver || sparse || totalItems >= 4 * numWarps * firstGroup;
+    bool ownTaken = !ownFirst;
     // Opaque pass of a scene with alpha-tested materials: a fetched group's alpha-tested meshlets go to the
     // alpha pass's list with one atomic, before their records are read (a draw of alpha-tested meshlets alone:
     // 45 -> 27 us). A shaded meshlet's FragmentShaderId is only known from its record, and is looked at
@@ -1068,13 +1074,13 @@ __global__ void __launch_bounds__(512, 2) k_draw_meshlets(DrawArgs a) {
                         b = (warp * gridDim.x + blockIdx.x) * firstGroup;
                         ownTaken = true;
                     } else if (lane == 0) {
-                        b = numWarps * firstGroup + (uint32_t)atomicAdd(twoPass && pass == 1 ? &a.s.control[7] : cursor,
-                                                                        (unsigned long long)fetchGroup);
+                        b = (ownFirst ? numWarps * firstGroup : 0u) +
+                            (uint32_t)atomicAdd(twoPass && pass == 1 ? &a.s.control[7] : cursor, (unsigned long long)fetchGroup);
                     }
                     const uint32_t base = __shfl_sync(0xFFFFFFFFu, b, 0);
                     if (base >= totalItems) {
                         if (pass == 0) {  // the large meshlets are all taken: the rest from position 0
-                            pass = 1, fetchGroup = firstGroup, ownTaken = false;
+                            pass = 1, fetchGroup = firstGroup, ownTaken = !ownFirst;
                             continue;
                         }
                         break;
