@@ -785,15 +785,16 @@ __device__ __noinline__ bool takes_alpha_pass(const DevMaterial* materials, uint
 // True if no triangle of a meshlet can change a pixel: its vertices (slots below `slots` of pz, all of them inside
 // the view) lie in a box of tiles whose depth bounds are all above the nearest vertex (triangle_depth_bound of
 // the meshlet). The alpha pass finds 41 to 46 % of its meshlets hidden by the opaque pass and by each other: 94 ->
-// 77 us of a 1916x1036 frame from inside, 175 -> 144 us of a 1600x900 G-buffer.
-// Larger boxes are not tested (256 loads a lane). Alpha pass + the chunk stage after it, us, by the limit in tiles:
+// 77 us of a 1916x1036 frame from inside, 175 -> 144 us of a 1600x900 G-buffer. The box is read four rows of tiles
+// at a time and left at the first rows that are not nearer, mostly the first ones: five meshlets that fill 1280x720
+// 112.7 -> 100 us. Larger boxes are not tested. Alpha pass + the chunk stage after it, us, by the limit in tiles:
 //                                               512          2048          8192          none
-//   50,000 meshlets, inside, 1916x1036       70 + 231      56 + 211      54 + 192      71 + 191
-//   30,000, G-buffer, 1600x900              125 + 171     109 + 163     109 + 133     109 + 131
-//   18,960, outside, 836x688                 89 + 110      85 +  87      85 +  86      85 +  87
-//   61,025, outside, 1188x1104               34 +  92      34 +  92      35 +  90      53 +  99
-//    1,960, inside, 2516x1168                27 + 170      28 + 169      29 + 166      47 + 137
-//   53,291, inside, 1160x1104                20 + 105      23 + 105      23 + 105      23 + 105
+//   50,000 meshlets, inside, 1916x1036       71 + 229      57 + 211      54 + 197      55 + 191
+//   30,000, G-buffer, 1600x900              127 + 171     112 + 157     111 + 132     111 + 131
+//   18,960, outside, 836x688                 90 + 111      83 +  90      85 +  90      84 +  89
+//   61,025, outside, 1188x1104               34 +  94      34 +  93      34 +  92      34 +  99
+//    1,960, inside, 2516x1168                27 + 173      27 + 170      28 + 167      56 + 140
+//   53,291, inside, 1160x1104                20 + 105      20 + 105      20 + 105      20 + 105
 constexpr uint32_t kHiddenTiles = 8192;
 __device__ __forceinline__ bool meshlet_hidden(const uint2* pz, uint32_t slots, const ViewParams& vp, int lane) {
     uint32_t lo = 0x7FFF7FFFu, hi = 0x80008000u, z = 0;
@@ -812,11 +813,15 @@ __device__ __forceinline__ bool meshlet_hidden(const uint2* pz, uint32_t slots, 
     const int32_t tx1 = (min(((x1 + 7) >> 4) + vp.halfW, 2 * vp.halfW) + 3) >> 2, ty1 = (min(((y1 + 8) >> 4) + vp.halfH, 2 * vp.halfH) + 3) >> 2;
     if (tx1 <= tx0 || ty1 <= ty0 || (uint32_t)((tx1 - tx0) * (ty1 - ty0)) > kHiddenTiles) return false;
     const int32_t tw = vp.width >> 2;
-    uint32_t known = 0xFFFFFFFFu;
-    for (int32_t y = ty0 + (lane >> 3); y < ty1; y += 4)
-        for (int32_t x = tx0 + (lane & 7); x < tx1; x += 8) known = min(known, vp.tileMin[y * tw + x]);
     const float zf = __uint_as_float(z), bound = fadd(zf, fmul(zf, 0x1p-16f));
-    return (int32_t)z >= 0 && __all_sync(0xFFFFFFFFu, (__float_as_uint(bound) | 0x80000000u) < known);
+    if ((int32_t)z < 0) return false;
+    for (int32_t top = ty0; top < ty1; top += 4) {  // the first rows mostly tell that a meshlet is not hidden
+        const int32_t y = top + (lane >> 3);
+        uint32_t known = 0xFFFFFFFFu;
+        for (int32_t x = tx0 + (lane & 7); x < tx1 && y < ty1; x += 8) known = min(known, vp.tileMin[y * tw + x]);
+        if (!__all_sync(0xFFFFFFFFu, (__float_as_uint(bound) | 0x80000000u) < known)) return false;
+    }
+    return true;
 }
 
 // Mesh stage. A work item is one meshlet of one view: a single-view draw numbers its meshlets
