@@ -29,9 +29,9 @@
 // Figures of the form a -> b beside a choice are of that choice alone, on the kernels as they were then: later
 // choices moved both. The kernels as they are (us, SM at 2070 MHz):
 //   1080p frame of 100k meshlets: mesh stage 333, chunk stage 151; 24 views of 100k meshlets in a batch: 1231, 221
-//   inside a 50k-meshlet scene, half of the materials alpha-tested, 1916x1036: mesh stage 126, opaque chunks 125,
-//   alpha pass 54, its chunks 199; G-buffer draw of 30k, 1600x900: 140, 80, 112, 127
-//   overdraw draw of 20k, 1280x720: 160, 148; 150k meshlets culled against the Hi-Z, 2560x1440: 43, 81
+//   inside a 50k-meshlet scene, half of the materials alpha-tested, 1916x1036: mesh stage 103, opaque chunks 122,
+//   alpha pass 53, its chunks 193; G-buffer draw of 30k, 1600x900: 113, 81, 110, 133
+//   overdraw draw of 20k, 1280x720: 160, 148; 150k meshlets culled against the Hi-Z, 2560x1440: 40, 81
 //   1024 meshlets at 1280x720: 30, 15; 60 at 252x140: 9.2, 7.5
 #include <algorithm>
 #include <cfloat>
