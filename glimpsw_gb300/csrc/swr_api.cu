@@ -109,8 +109,9 @@ swr_status size_alpha_list(swr_rasterizer r, uint32_t count) {
 }
 
 // The unit vectors' table of the current device: one for all of its scenes, given back with the last. It is complete
-// before any caller has it, whatever streams draw and resolve later. Empty where there is no room for it.
-std::shared_ptr<float4> oct_table() {
+// before any caller has it, whatever streams draw and resolve later. Empty where there is no room for it, on the
+// device or (for the pointer's count) on the host.
+std::shared_ptr<float4> oct_table() try {
     struct Entry {
         std::weak_ptr<float4> table;
         unsigned long long context;  // a cudaDeviceReset ends the one the table lives in
@@ -137,6 +138,8 @@ std::shared_ptr<float4> oct_table() {
     e.table = t;
     e.context = swr_internal_context_id();  // the allocation made the context current if none was
     return t;
+} catch (const std::bad_alloc&) {
+    return {};
 }
 
 }  // namespace
